@@ -125,21 +125,29 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
     // the work plan's scratch, grown on demand (like the reference's device
     // arrays, held until exit)
     static SRWork w{};
-    if (w.seg_cap < numCells || w.heavy_cap < shortrange_heavy_cap(numParticles)) {
-        cudaFree(w.heavy);
-        cudaFree(w.seg_nt);
+    static uint32_t *off = nullptr;  // cell offsets, then the conversion's scratch
+    static size_t off_cap = 0;
+    const size_t off_need = (size_t)numCells + 1 + offsets_scratch(numCells);
+    const uint32_t cap = shortrange_unit_cap(numParticles, numCells);
+    if (w.cap < cap) {
+        cudaFree(w.units);
         cudaFree(w.ctl);
         w = SRWork{};
-        const uint32_t hc = shortrange_heavy_cap(numParticles);
-        capi_check(cudaMalloc(&w.heavy, sizeof(uint2) * hc), "cudaForceEvaluateShortrange");
-        capi_check(cudaMalloc(&w.seg_nt, sizeof(uint32_t) * numCells), "cudaForceEvaluateShortrange");
+        capi_check(cudaMalloc(&w.units, sizeof(uint2) * cap), "cudaForceEvaluateShortrange");
         capi_check(cudaMalloc(&w.ctl, kSRCtlWords * sizeof(uint32_t)), "cudaForceEvaluateShortrange");
         capi_check(cudaMemset(w.ctl, 0, kSRCtlWords * sizeof(uint32_t)), "cudaForceEvaluateShortrange");
-        w.heavy_cap = hc;
-        w.seg_cap = numCells;
+        w.cap = cap;
     }
-    capi_status(launch_shortrange(p, (const float4 *)sortedPos, gridParticleIndex, cellStart, cellEnd,
-                                  kCellStartEnd, s.table, (float4 *)gravAccel, k, w, 0),
+    if (off_cap < off_need) {
+        cudaFree(off);
+        off_cap = 0;
+        capi_check(cudaMalloc(&off, sizeof(uint32_t) * off_need), "cudaForceEvaluateShortrange");
+        off_cap = off_need;
+    }
+    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, off + numCells + 1, 0),
+                "cudaForceEvaluateShortrange");
+    capi_status(launch_shortrange(p, (const float4 *)sortedPos, gridParticleIndex, off, s.table, (float4 *)gravAccel,
+                                  k, w, 0),
                 "cudaForceEvaluateShortrange");
     capi_status(shortrange_check(w.ctl, 0), "cudaForceEvaluateShortrange");
 }

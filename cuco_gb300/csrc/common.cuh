@@ -104,6 +104,13 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, float4 *sorted_pos,
                                      const float4 *pos, uint32_t n, uint32_t ncells,
                                      cudaStream_t stream);
 
+// The reference's cell bounds (cell_end is read where cell_start is not
+// empty) -> the engine's offsets (ncells + 1).  scratch: offsets_scratch(ncells)
+// words.
+size_t offsets_scratch(uint32_t ncells);
+cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
+                                       uint32_t ncells, uint32_t *scratch, cudaStream_t stream);
+
 // A box's cell grid within a concatenated cell numbering (cells
 // cell_base .. cell_base + G^3 - 1).
 struct CellBox {
@@ -146,17 +153,14 @@ struct ShortRangeParams {
     // pair-law bounds, filled in by the short-range launch from the above:
     // fast-path cut and flag cut (plain: a band around rcut^2 decided in
     // double), the softening bound below which the spline applies, the bin
-    // factor scaled down and up by the bin-edge band, rcut^2 in double
-    float rc2_lo, rc2_hi, hmin2, alo, ahi;
+    // factor scaled down and up by the bin-edge band, a radius just above the
+    // flag cut, rcut^2 in double
+    float rc2_lo, rc2_hi, hmin2, alo, ahi, r_hi;
     double rcut2_d;
     // the z-slice counts of the cells (launch_cell_subsort), indexed by cell
-    // id; null when the sources are not in slice order or the per-segment
-    // table would not fit in shared memory
+    // id; null when the sources are not in slice order
     const uint4 *slices;
 };
-
-// Which cell-bound format the kernel reads.
-enum CellFormat { kCellOffsets = 0, kCellStartEnd = 1 };
 
 // Kick applied in the short-range epilogue (null vel: no kick).
 struct KickArgs {
@@ -167,36 +171,34 @@ struct KickArgs {
     const float4 *acc_pm_o;   // PM acceleration in original order (used when acc_pm_s is null)
 };
 
-// Device scratch of a launch's work plan: each segment's target count, the
-// slices of segments denser than one unit, and two counters.  seg_cap must
-// cover the launch's segments (G^3 is always enough), heavy_cap
-// shortrange_heavy_cap(n).
+// Device scratch of a launch's work plan: the units (first target, segment)
+// and the control words.  cap must be at least shortrange_unit_cap(n, segments)
+// of the launch (G^3 bounds a box's segments).
 struct SRWork {
-    uint2 *heavy;
-    uint32_t heavy_cap;
-    uint32_t *seg_nt;
-    uint32_t seg_cap;
-    uint32_t *ctl;  // kSRCtlWords: [0] dense slices listed, [1] next unit (both reset per
-                    // launch), [2] nonzero once a staging wait gave up (kept until read)
+    uint2 *units;
+    uint32_t cap;
+    uint32_t *ctl;  // kSRCtlWords: [0] dense slices listed, [1] next unit, [2] other units listed
+                    // (reset per launch), [3] timeout word (kept until read), [4] spare
 };
-uint32_t shortrange_heavy_cap(uint32_t n);
-constexpr int kSRCtlWords = 4;
-// Reads and clears the short range's timeout word (ctl[2]) after the work on
-// `stream` is done: CUCO_ERR_TIMEOUT when a staging wait gave up.
+uint32_t shortrange_unit_cap(uint32_t n, uint64_t segments);
+constexpr int kSRCtlWords = 8;
+// Reads and clears the short range's timeout word (ctl[3]) after the work on
+// `stream` is done: CUCO_ERR_TIMEOUT when a bounded wait gave up.
 cuco_status_t shortrange_check(uint32_t *ctl, cudaStream_t stream);
-// Runs the staging wait's timeout path with a barrier that never completes
-// and a limit of `limit_cycles`: returns what shortrange_check then reports.
+// Runs a bounded wait on a barrier that never completes, with a limit of
+// `limit_cycles`: returns what shortrange_check then reports.
 cuco_status_t shortrange_timeout_probe(uint32_t *ctl, long long limit_cycles, cudaStream_t stream);
 
 // pair_counter: when non-null, the launch adds its in-range pair count to it.
 // late_stream (with plan_done, an event of the caller's): the persistent grid
 // is split, one CTA per SM fewer on `stream` and the rest queued on
-// late_stream behind whatever that stream runs first (the PM); both parts
-// take units from the same counter, so work left when the late part starts
+// late_stream behind whatever that stream runs first (the PM).  The first
+// part's warps start on units given by their number (every warp asking the
+// counter at once cost 10 us of a small box's launch); the rest, for both
+// parts, come from one counter, so work left when the late part starts
 // spreads over both.  The launch is complete when both streams have run it.
 cuco_status_t launch_shortrange(const ShortRangeParams &p, const float4 *sorted_pos,
-                                const uint32_t *perm, const uint32_t *cell_a,
-                                const uint32_t *cell_b, CellFormat fmt, const float *table,
+                                const uint32_t *perm, const uint32_t *cell_off, const float *table,
                                 float4 *acc_out, const KickArgs &kick, const SRWork &work, cudaStream_t stream,
                                 unsigned long long *pair_counter = nullptr, cudaStream_t late_stream = nullptr,
                                 cudaEvent_t plan_done = nullptr);
@@ -204,15 +206,15 @@ cuco_status_t launch_shortrange(const ShortRangeParams &p, const float4 *sorted_
 // Many boxes in one launch (the batched form).  A box's descriptor holds its
 // parameters and neighbour-column set; shortrange_desc_fill writes one (in
 // host memory, shortrange_desc_bytes() long) and returns the box's segment
-// count and shared memory.  kicks[b] = (kick_pp, kick_pm) of box b.
+// count.  kicks[b] = (kick_pp, kick_pm) of box b.
 size_t shortrange_desc_bytes();
-cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32_t *segments, size_t *smem);
+cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32_t *segments);
 // uniform_law_desc (host memory, or null): a descriptor whose pair law every
 // box shares (shortrange_descs_uniform_law said so); the launch then reads
 // the law from its parameters instead of each box's descriptor.
 bool shortrange_descs_uniform_law(const void *host_descs, int nbox);
 cuco_status_t launch_shortrange_multi(const void *descs, const double2 *kicks, const uint32_t *seg_base,
-                                      int nbox, uint32_t segments, size_t smem, bool fixed,
+                                      int nbox, uint32_t segments, uint32_t n, bool fixed,
                                       const float4 *sorted_pos, const uint32_t *perm, const uint32_t *cell_off,
                                       const float *table, float4 *acc_out, const KickArgs &kick,
                                       const SRWork &work, cudaStream_t stream, unsigned long long *pair_counter,

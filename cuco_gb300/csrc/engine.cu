@@ -464,8 +464,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
         k.acc_pm_s = nullptr;
         k.acc_pm_out = nullptr;
         k.acc_pm_o = pm && !split ? b->acc_pm : nullptr;
-        CUCO_TRY(launch_shortrange(make_sr_params(b), b->spos, perm_s, b->cell_off,
-                                   nullptr, kCellOffsets, b->table, b->acc_pp, k, b->work, b->stream,
+        CUCO_TRY(launch_shortrange(make_sr_params(b), b->spos, perm_s, b->cell_off, b->table, b->acc_pp, k, b->work, b->stream,
                                    b->count_pairs ? b->pair_counter : nullptr, split ? b->pm_stream : nullptr,
                                    b->sr_plan));
         b->launches += split ? 3 : 2;  // work plan + persistent short range (in two parts beside the PM)
@@ -589,12 +588,11 @@ cuco_status_t cuco_box_create(const cuco_config_t *cfg, cuco_box_t **out) {
         (s = alloc(&b->cell_off, (size_t)b->ncells + 1)) || (s = alloc(&b->cell_sl, (size_t)b->ncells)) ||
         (s = alloc(&b->table, kNTab)) ||
         (s = alloc(&b->stage3, 3 * n)) || (s = alloc(&b->pair_counter, 1)) ||
-        (s = alloc(&b->work.heavy, shortrange_heavy_cap(b->n))) || (s = alloc(&b->work.seg_nt, b->ncells)) ||
+        (s = alloc(&b->work.units, shortrange_unit_cap(b->n, b->ncells))) ||
         (s = alloc(&b->work.ctl, kSRCtlWords)))
         return fail(s);
     cudaMemset(b->work.ctl, 0, sizeof(uint32_t) * kSRCtlWords);
-    b->work.heavy_cap = shortrange_heavy_cap(b->n);
-    b->work.seg_cap = b->ncells;  // G^3 covers every segment length
+    b->work.cap = shortrange_unit_cap(b->n, b->ncells);  // G^3 covers every segment length
     cudaMemset(b->pair_counter, 0, sizeof(unsigned long long));
     std::vector<float> t(kNTab);
     shortrange_table(t.data());
@@ -636,8 +634,7 @@ cuco_status_t cuco_box_destroy(cuco_box_t *b) {
     cudaFree(b->table);
     cudaFree(b->stage3);
     cudaFree(b->pair_counter);
-    cudaFree(b->work.heavy);
-    cudaFree(b->work.seg_nt);
+    cudaFree(b->work.units);
     cudaFree(b->work.ctl);
     if (b->tstart) cudaEventDestroy(b->tstart);
     if (b->tstop) cudaEventDestroy(b->tstop);
@@ -668,7 +665,7 @@ __global__ void k_count_nonfinite(const float *__restrict__ v, size_t n, uint32_
 // The staged triplets (b->stage3) must all be finite: a state with a NaN or
 // an infinity is refused before it reaches the box (CUCO_ERR_INVALID).
 cuco_status_t check_finite(cuco_box_t *b, const char *what) {
-    uint32_t *count = b->work.ctl + 3;  // the plan's spare control word
+    uint32_t *count = b->work.ctl + 4;  // the plan's spare control word
     CUCO_TRY_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), b->stream));
     const size_t n = 3 * (size_t)b->n;
     if (n) {

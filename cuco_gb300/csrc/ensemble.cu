@@ -315,7 +315,6 @@ struct cuco_ensemble {
     int slot = 0;
     PMMulti pm{};
     uint32_t segments = 0;
-    size_t sr_smem = 0;
     // box 0's short-range descriptor (host copy) when every box has its pair
     // law, so the launch reads the law from its parameters
     std::vector<char> sr_law;
@@ -335,10 +334,10 @@ struct cuco_ensemble {
            cap_green = 0, cap_tw = 0, cap_table = 0, cap_pbeg = 0, cap_segbase = 0, cap_drift = 0, cap_pm = 0,
            cap_kicks = 0, cap_factors = 0, cap_counter = 0, cap_sr = 0, cap_hfactors[2] = {0, 0},
            cap_hkicks[2] = {0, 0},
-           cap_mapz = 0, cap_mapa = 0, cap_heavy = 0, cap_segnt = 0, cap_ctl = 0, cap_cellsl = 0;
+           cap_mapz = 0, cap_mapa = 0, cap_units = 0, cap_ctl = 0, cap_cellsl = 0;
     // the short range's work-plan scratch
-    uint2 *sr_heavy = nullptr;
-    uint32_t *sr_segnt = nullptr, *sr_ctl = nullptr;
+    uint2 *sr_units = nullptr;
+    uint32_t *sr_ctl = nullptr;
 };
 
 namespace {
@@ -376,8 +375,8 @@ cuco_status_t ensemble_pass(cuco_ensemble *e, int do_drift, bool kick) {
     KickArgs k{};
     k.vel = kick ? e->vel : nullptr;
     k.acc_pm_o = e->acc_pm;
-    SRWork w{e->sr_heavy, (uint32_t)e->cap_heavy, e->sr_segnt, (uint32_t)e->cap_segnt, e->sr_ctl};
-    CUCO_TRY(launch_shortrange_multi(e->d_sr, e->d_kicks, e->d_segbase, e->nbox, e->segments, e->sr_smem, e->fixed,
+    SRWork w{e->sr_units, (uint32_t)e->cap_units, e->sr_ctl};
+    CUCO_TRY(launch_shortrange_multi(e->d_sr, e->d_kicks, e->d_segbase, e->nbox, e->segments, e->n, e->fixed,
                                      e->spos, perm_s, e->cell_off, e->table, e->acc_pp, k, w, e->stream,
                                      e->count_pairs ? e->pair_counter : nullptr,
                                      e->sr_law.empty() ? nullptr : e->sr_law.data()));
@@ -599,7 +598,7 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     std::vector<uint2> mapz, mapa;
     std::vector<float> green(gbase[nbox]);
     std::vector<float2> tw(tbase[nbox]);
-    size_t smz = 0, sma = 0, sr_smem = 0;
+    size_t smz = 0, sma = 0;
     for (int b = 0; b < nbox; ++b) {
         const cuco_config_t &c = cfg[b];
         const int M = c.pm_grid, Mh = M / 2 + 1;
@@ -615,16 +614,14 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
         smz = std::max(smz, pm_smem_z(M, P[b]));
         sma = std::max(sma, pm_smem_axis(M, B[b]));
         uint32_t nseg = 0;
-        size_t sm = 0;
         if ((s = shortrange_desc_fill(sr_params(c, (uint32_t)c.n, (uint32_t)cbase[b], e->cell_sl),
-                                      srd.data() + b * shortrange_desc_bytes(), &nseg, &sm)))
+                                      srd.data() + b * shortrange_desc_bytes(), &nseg)))
             return s;
         segbase[b + 1] = segbase[b] + nseg;
-        sr_smem = std::max(sr_smem, sm);
     }
     if ((s = grow(e->d_mapz, e->cap_mapz, mapz.size(), st)) || (s = grow(e->d_mapa, e->cap_mapa, mapa.size(), st)) ||
-        (s = grow(e->sr_heavy, e->cap_heavy, (size_t)shortrange_heavy_cap((uint32_t)n) + 16u * nbox, st)) ||
-        (s = grow(e->sr_segnt, e->cap_segnt, (size_t)segbase[nbox], st)) || (s = grow(e->sr_ctl, e->cap_ctl, kSRCtlWords, st)))
+        (s = grow(e->sr_units, e->cap_units, (size_t)shortrange_unit_cap((uint32_t)n, segbase[nbox]), st)) ||
+        (s = grow(e->sr_ctl, e->cap_ctl, kSRCtlWords, st)))
         return s;
     if (cudaStreamSynchronize(st) != cudaSuccess ||
         cudaMemcpy(e->table, tab.data(), sizeof(float) * kNTab, cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -655,7 +652,6 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     e->ncells = ncells;
     e->key_bits = kbits;
     e->segments = segbase[nbox];
-    e->sr_smem = sr_smem;
     e->sr_law.clear();
     if (shortrange_descs_uniform_law(srd.data(), nbox))
         e->sr_law.assign(srd.begin(), srd.begin() + shortrange_desc_bytes());
@@ -744,8 +740,8 @@ cuco_status_t cuco_ensemble_destroy(cuco_ensemble_t *e) {
                     (void *)e->spec,
                     (void *)e->green, (void *)e->tw, (void *)e->table, (void *)e->d_pbeg, (void *)e->d_segbase,
                     (void *)e->d_drift, (void *)e->d_pm, (void *)e->d_mapz, (void *)e->d_mapa, (void *)e->d_sr,
-                    (void *)e->d_kicks, (void *)e->d_factors, (void *)e->pair_counter, (void *)e->sr_heavy,
-                    (void *)e->sr_segnt, (void *)e->sr_ctl})
+                    (void *)e->d_kicks, (void *)e->d_factors, (void *)e->pair_counter, (void *)e->sr_units,
+                    (void *)e->sr_ctl})
         if (p && e->stream) cudaFreeAsync(p, e->stream);
     if (e->stream) cudaStreamSynchronize(e->stream);
     for (int k = 0; k < 2; ++k) {

@@ -560,6 +560,85 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, float4 *sorted_pos,
     return CUCO_OK;
 }
 
+// ---- start/end -> offsets: off[c] is the largest end of the cells before c
+// (ends grow along the cell order), a running maximum over the cells in two
+// launches: each block's maximum, then every block its cells after the
+// maximum of the blocks before it.
+namespace {
+constexpr uint32_t kOffBlock = 4096;  // cells per block
+
+__device__ __forceinline__ uint32_t end_of(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+                                           uint32_t c, uint32_t ncells) {
+    return c < ncells && start[c] != kEmptyCell ? end[c] : 0u;
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_block_end_max(const uint32_t *__restrict__ start,
+                                                                const uint32_t *__restrict__ end, uint32_t ncells,
+                                                                uint32_t *__restrict__ block_max) {
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    uint32_t m = 0;
+#pragma unroll 4
+    for (uint32_t k = threadIdx.x; k < kOffBlock; k += kSortThreads)
+        m = max(m, end_of(start, end, blockIdx.x * kOffBlock + k, ncells));
+    m = __reduce_max_sync(kFull, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
+    __syncthreads();
+    if (threadIdx.x == 0) block_max[blockIdx.x] = s_max;
+}
+
+__global__ void __launch_bounds__(kSortThreads) k_start_end_offsets(const uint32_t *__restrict__ start,
+                                                                    const uint32_t *__restrict__ end, uint32_t ncells,
+                                                                    const uint32_t *__restrict__ block_max,
+                                                                    uint32_t *__restrict__ cell_off) {
+    __shared__ uint32_t s_carry, s_warp[kSortWarps];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_carry = 0;
+    __syncthreads();
+    uint32_t carry = 0;
+    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kSortThreads) carry = max(carry, block_max[k]);
+    carry = __reduce_max_sync(kFull, carry);
+    if (lane == 0) atomicMax(&s_carry, carry);
+    __syncthreads();
+    carry = s_carry;
+    for (uint32_t k = 0; k < kOffBlock; k += kSortThreads) {
+        const uint32_t c = blockIdx.x * kOffBlock + k + threadIdx.x;
+        uint32_t incl = end_of(start, end, c, ncells);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(kFull, incl, off);
+            if (lane >= off) incl = max(incl, v);
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        uint32_t before = carry, all = carry;
+        for (uint32_t w = 0; w < (uint32_t)kSortWarps; ++w) {
+            if (w < warp) before = max(before, s_warp[w]);
+            all = max(all, s_warp[w]);
+        }
+        incl = max(incl, before);
+        // cell c ends, and the next begins, at the largest end so far
+        if (c < ncells) cell_off[c + 1] = incl;
+        if (c == 0) cell_off[0] = 0;
+        carry = all;
+        __syncthreads();  // s_warp is rewritten by the next round
+    }
+}
+}  // namespace
+
+size_t offsets_scratch(uint32_t ncells) { return (ncells + kOffBlock - 1) / kOffBlock; }
+
+cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
+                                       uint32_t ncells, uint32_t *scratch, cudaStream_t stream) {
+    const unsigned blocks = (unsigned)offsets_scratch(ncells);
+    if (!blocks) return CUCO_OK;
+    k_block_end_max<<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch);
+    k_start_end_offsets<<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, cell_off);
+    CUCO_TRY_CUDA(cudaGetLastError());
+    return CUCO_OK;
+}
+
 uint32_t bounds_violations_sort() { return bounds_violations_take(); }
 
 }  // namespace cuco
