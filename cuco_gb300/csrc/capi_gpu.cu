@@ -152,6 +152,9 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
     capi_status(shortrange_check(w.ctl, 0), "cudaForceEvaluateShortrange");
 }
 
+// what a caller's `counters` holds at least (the reference RadixSort's allocation)
+static size_t counter_words(uint n) { return 32 * (((size_t)n + 1023) / 1024); }
+
 void radixSort(uint *keys, uint *values, uint *tempKeys, uint *tempValues, uint *counters,
                uint *countersSum, uint *blockOffsets, CUDPPHandle scanPlan, uint numElements,
                uint keyBits, bool flipBits) {
@@ -161,8 +164,8 @@ void radixSort(uint *keys, uint *values, uint *tempKeys, uint *tempValues, uint 
     if (flipBits) capi_fail("radixSort", "flipBits is not supported");
     bool in_alt = false;
     int launches = 0;
-    capi_status(sort_pairs(keys, values, values, tempKeys, tempValues, counters, numElements,
-                           (int)keyBits, 6, 0, &in_alt, &launches),
+    capi_status(sort_pairs(keys, values, values, tempKeys, tempValues, counters, counter_words(numElements),
+                           numElements, (int)keyBits, 6, 0, &in_alt, &launches),
                 "radixSort");
     if (in_alt) {
         capi_check(cudaMemcpyAsync(keys, tempKeys, sizeof(uint) * numElements, cudaMemcpyDeviceToDevice, 0),
@@ -182,8 +185,8 @@ void radixSortKeysOnly(uint *keys, uint *tempKeys, uint *counters, uint *counter
     if (flipBits) capi_fail("radixSortKeysOnly", "flipBits is not supported");
     bool in_alt = false;
     int launches = 0;
-    capi_status(sort_pairs(keys, nullptr, nullptr, tempKeys, nullptr, counters, numElements,
-                           (int)keyBits, 6, 0, &in_alt, &launches),
+    capi_status(sort_pairs(keys, nullptr, nullptr, tempKeys, nullptr, counters, counter_words(numElements),
+                           numElements, (int)keyBits, 6, 0, &in_alt, &launches),
                 "radixSortKeysOnly");
     if (in_alt)
         capi_check(cudaMemcpyAsync(keys, tempKeys, sizeof(uint) * numElements, cudaMemcpyDeviceToDevice, 0),

@@ -318,7 +318,8 @@ struct cuco_box {
     float4 *pos = nullptr, *vel = nullptr, *acc_pp = nullptr, *acc_pm = nullptr;
     float4 *spos = nullptr;
     uint32_t *keys = nullptr, *perm = nullptr, *keys_alt = nullptr, *perm_alt = nullptr;
-    uint32_t *hist = nullptr, *hist2 = nullptr, *cell_off = nullptr;
+    uint32_t *hist = nullptr, *cell_off = nullptr;
+    size_t hist_words = 0;
     uint4 *cell_sl = nullptr;  // per cell: z-slice counts
     uint32_t *sorted_keys = nullptr, *sorted_perm = nullptr;  // where the last sort ended
     uint32_t *perm_s = nullptr;  // the z-slice order's map to original indices (the sort's spare buffer)
@@ -430,8 +431,8 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
         record(b, 6);
     }
     bool in_alt = false;
-    CUCO_TRY(sort_pairs(b->keys, b->perm, nullptr, b->keys_alt, b->perm_alt, b->hist, b->n,
-                        b->key_bits, 8, b->stream, &in_alt, &b->launches, b->hist2));
+    CUCO_TRY(sort_pairs(b->keys, b->perm, nullptr, b->keys_alt, b->perm_alt, b->hist, b->hist_words,
+                        b->n, b->key_bits, 8, b->stream, &in_alt, &b->launches));
     b->sorted_keys = in_alt ? b->keys_alt : b->keys;
     b->sorted_perm = in_alt ? b->perm_alt : b->perm;
     record(b, 2);
@@ -579,12 +580,12 @@ cuco_status_t cuco_box_create(const cuco_config_t *cfg, cuco_box_t **out) {
         return fail(CUCO_ERR_CUDA);
     }
     const size_t n = b->n;
+    b->hist_words = sort_hist_entries(b->n, b->key_bits, 8);
     if ((s = alloc(&b->pos, n)) || (s = alloc(&b->vel, n)) || (s = alloc(&b->acc_pp, n)) ||
         (s = alloc(&b->acc_pm, n)) || (s = alloc(&b->spos, n)) ||
         (s = alloc(&b->keys, n)) || (s = alloc(&b->perm, n)) || (s = alloc(&b->keys_alt, n)) ||
         (s = alloc(&b->perm_alt, n)) ||
-        (s = alloc(&b->hist, sort_hist_entries(b->n, b->key_bits, 8))) ||
-        (s = alloc(&b->hist2, sort_hist_entries(b->n, b->key_bits, 8))) ||
+        (s = alloc(&b->hist, b->hist_words)) ||
         (s = alloc(&b->cell_off, (size_t)b->ncells + 1)) || (s = alloc(&b->cell_sl, (size_t)b->ncells)) ||
         (s = alloc(&b->table, kNTab)) ||
         (s = alloc(&b->stage3, 3 * n)) || (s = alloc(&b->pair_counter, 1)) ||
@@ -628,7 +629,6 @@ cuco_status_t cuco_box_destroy(cuco_box_t *b) {
     cudaFree(b->keys_alt);
     cudaFree(b->perm_alt);
     cudaFree(b->hist);
-    cudaFree(b->hist2);
     cudaFree(b->cell_off);
     cudaFree(b->cell_sl);
     cudaFree(b->table);

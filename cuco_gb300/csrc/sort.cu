@@ -5,8 +5,8 @@
 // reorderDataAndFindCellStartD (gravlist_kernel.cu:121-160).
 //
 // The sort is a three-kernel-per-pass LSD radix sort designed for sm_103a:
-//   1. k_sort_hist:   per 4096-key tile, a digit histogram (warp match_any
-//                     aggregation into shared-memory counters);
+//   1. k_sort_hist:   per tile, a digit histogram (one shared-memory counter
+//                     row per warp);
 //   2. k_sort_scan:   one CTA per digit turns its tile counts into inclusive
 //                     prefixes over the tiles (the digit's total is the last);
 //   3. k_sort_scatter: each tile ranks its keys stably with warp ballots
@@ -17,6 +17,15 @@
 //                     and writes out digit runs with coalesced stores.
 // Digits are 4..8 bits; a pass count of ceil(bits/8) with equal digit widths
 // is used (18-bit keys: three 6-bit passes).
+//
+// What bounds it: memory traffic at millions of keys, latency below.  Every
+// kernel issues all of a thread's loads before it uses the first: the ranking
+// loop used to load a key per round, behind the round's warp barriers, and
+// the scatter counted the next pass's digits with global atomics, which cost
+// more than reading the keys again.  A tile is 4096 keys, or 2048 or 1024
+// where that would leave SMs without four tiles (sort_items).  Measured alone,
+// before and after, a pass over 4M pairs: histogram 27 -> 6, scan 5 -> 4,
+// scatter 33 -> 26 us; three passes over 32K pairs 93 -> 36 us.
 #include "common.cuh"
 
 namespace cuco {
@@ -24,8 +33,6 @@ namespace cuco {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr unsigned kFull = 0xffffffffu;
 
@@ -47,101 +54,126 @@ __global__ void k_cell_keys(const float4 *__restrict__ pos, uint32_t *__restrict
     }
 }
 
-template <int RB>
+// Digit counts of each tile of kSortThreads * ITEMS keys.
+template <int RB, int ITEMS>
 __global__ void __launch_bounds__(kSortThreads)
-    k_sort_hist(const uint32_t *__restrict__ keys, uint32_t n, int shift,
-                uint32_t *__restrict__ hist, uint32_t tiles) {
+    k_sort_hist(const uint32_t *__restrict__ keys, uint32_t n, int shift, uint32_t *__restrict__ hist,
+                uint32_t tiles) {
     constexpr int RADIX = 1 << RB;
-    __shared__ uint32_t h[RADIX];
-    for (int d = threadIdx.x; d < RADIX; d += kSortThreads) h[d] = 0;
-    __syncthreads();
-    const uint32_t tile = blockIdx.x;
-    const uint32_t base = tile * kSortTile;
-    const int lane = threadIdx.x & 31;
-#pragma unroll 4
-    for (int k = 0; k < kSortItems; ++k) {
-        uint32_t i = base + k * kSortThreads + threadIdx.x;
-        bool valid = i < n;
-        uint32_t d = valid ? (keys[i] >> shift) & (RADIX - 1) : (uint32_t)RADIX;
-        uint32_t peers = __match_any_sync(kFull, d);
-        if (valid && lane == __ffs(peers) - 1) atomicAdd(&h[d], (uint32_t)__popc(peers));
+    __shared__ uint32_t h[kSortWarps][RADIX];
+    const int warp = threadIdx.x >> 5;
+    const uint32_t tile = blockIdx.x, base = tile * (kSortThreads * ITEMS) + threadIdx.x;
+    uint32_t key[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const uint32_t i = base + k * kSortThreads;
+        key[k] = i < n ? keys[i] : 0u;
     }
+    for (int e = threadIdx.x; e < kSortWarps * RADIX; e += kSortThreads) (&h[0][0])[e] = 0;
     __syncthreads();
-    for (int d = threadIdx.x; d < RADIX; d += kSortThreads) hist[d * tiles + tile] = h[d];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k)
+        if (base + k * kSortThreads < n) atomicAdd(&h[warp][(key[k] >> shift) & (RADIX - 1)], 1u);
+    __syncthreads();
+    for (int d = threadIdx.x; d < RADIX; d += kSortThreads) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int w = 0; w < kSortWarps; ++w) c += h[w][d];
+        hist[(size_t)d * tiles + tile] = c;
+    }
 }
 
 // hist[d*tiles + t] (count of digit d in tile t) -> the inclusive prefix of
 // those counts over the tiles, one CTA per digit.  A digit's total is then its
 // last entry, and the scatter derives every run's global offset from these
-// (no second pass over the table, no scratch beyond it).
-// zero_next (or null): the next pass's histogram, whose row of this digit is
-// cleared here for the scatter to count into.
-__global__ void __launch_bounds__(kSortThreads) k_sort_scan(uint32_t *__restrict__ hist, uint32_t tiles,
-                                                            uint32_t *__restrict__ zero_next) {
-    __shared__ uint32_t wsum[kSortWarps];
+// (no second pass over the table, no scratch beyond it).  Four counts a
+// thread and round are in flight together.
+constexpr int kScanThreads = 512, kScanWarps = kScanThreads / 32, kScanItems = 4;
+__global__ void __launch_bounds__(kScanThreads) k_sort_scan(uint32_t *__restrict__ hist, uint32_t tiles) {
+    __shared__ uint32_t wsum[kScanItems][kScanWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t *h = hist + (size_t)blockIdx.x * tiles;
-    if (zero_next)
-        for (uint32_t t = threadIdx.x; t < tiles; t += kSortThreads) zero_next[(size_t)blockIdx.x * tiles + t] = 0u;
     uint32_t carry = 0;
-    for (uint32_t t0 = 0; t0 < tiles; t0 += kSortThreads) {
-        const uint32_t t = t0 + threadIdx.x;
-        const uint32_t v = t < tiles ? h[t] : 0u;
-        uint32_t incl = v;
+    for (uint32_t t0 = 0; t0 < tiles; t0 += kScanThreads * kScanItems) {
+        uint32_t incl[kScanItems];
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, off);
-            if (lane >= off) incl += y;
+        for (int j = 0; j < kScanItems; ++j) {
+            const uint32_t t = t0 + j * kScanThreads + threadIdx.x;
+            incl[j] = t < tiles ? h[t] : 0u;
         }
-        if (lane == 31) wsum[warp] = incl;
+#pragma unroll
+        for (int j = 0; j < kScanItems; ++j) {
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, incl[j], off);
+                if (lane >= off) incl[j] += y;
+            }
+            if (lane == 31) wsum[j][warp] = incl[j];
+        }
         __syncthreads();
-        uint32_t before = 0, all = 0;
 #pragma unroll
-        for (int w = 0; w < kSortWarps; ++w) {
-            const uint32_t x = wsum[w];
-            before += w < warp ? x : 0u;
-            all += x;
+        for (int j = 0; j < kScanItems; ++j) {
+            uint32_t before = carry;
+#pragma unroll
+            for (int w = 0; w < kScanWarps; ++w) {
+                const uint32_t x = wsum[j][w];
+                before += w < warp ? x : 0u;
+                carry += x;
+            }
+            const uint32_t t = t0 + j * kScanThreads + threadIdx.x;
+            if (t < tiles) h[t] = before + incl[j];
         }
-        if (t < tiles) h[t] = carry + before + incl;
-        carry += all;
         __syncthreads();  // wsum is rewritten by the next round
     }
 }
 
-// NEXT: also count the next pass's digit (at next_shift) of every key placed,
-// per destination tile, into next_hist (cleared by this pass's scan): the
-// histogram the next pass would build from this pass's output.
-template <int RB, bool WITH_VALS, bool SINGLE_TILE, bool NEXT>
-__global__ void __launch_bounds__(kSortThreads, 4)
-    k_sort_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
-                   uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint32_t n,
-                   int shift, const uint32_t *__restrict__ hist, uint32_t tiles,
-                   uint32_t *__restrict__ next_hist, int next_shift) {
+// SINGLE: one tile, whose own digit starts are the global ones.
+// The values are read when the ranks are known: held through the ranking they
+// took 88 registers, two CTAs an SM.  (At 16 keys a thread three CTAs without
+// spills beat four: 4 passes over 4M pairs 132 against 140 us.)
+template <int RB, int ITEMS, bool WITH_VALS, bool SINGLE>
+__global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 3 : 4)
+    k_sort_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint32_t *__restrict__ kout,
+                   uint32_t *__restrict__ vout, uint32_t n, int shift, const uint32_t *__restrict__ hist,
+                   uint32_t tiles) {
     constexpr int RADIX = 1 << RB;
+    constexpr uint32_t TILE = kSortThreads * ITEMS;
+    static_assert(RADIX <= kSortThreads, "a thread per digit");
     __shared__ uint32_t wcnt[kSortWarps][RADIX];
-    __shared__ uint32_t dstart[RADIX];
-    __shared__ uint32_t gbase[RADIX];
-    __shared__ uint32_t skeys[kSortTile];
-    __shared__ uint32_t svals[WITH_VALS ? kSortTile : 1];
+    __shared__ uint32_t dstart[RADIX];  // digit's start in the staged tile
+    __shared__ uint32_t gofs[RADIX];    // staged position -> global position
+    __shared__ uint32_t wsum[2][kSortWarps];
+    __shared__ uint32_t skeys[TILE];
+    __shared__ uint32_t svals[WITH_VALS ? TILE : 1];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t tile = blockIdx.x;
-    const uint32_t base = tile * kSortTile;
+    const uint32_t base = tile * TILE;
     const uint32_t lt = (1u << lane) - 1u;
-    for (int e = threadIdx.x; e < kSortWarps * RADIX; e += kSortThreads) (&wcnt[0][0])[e] = 0;
-    __syncthreads();
-
-    // Warp w owns tile elements [w*512, w*512+512); item k covers 32 of them in
-    // lane order, so (k, lane) order is input order and the ranks are stable.
-    // The ranks (below 4096) are kept two to a register; keys and values are
-    // read again when they are placed, so few registers stay live.
-    uint32_t rank2[kSortItems / 2];
+    // Warp w owns tile elements [w * 32 * ITEMS, ...); item k covers 32 of
+    // them in lane order, so (k, lane) order is input order and the ranks are
+    // stable.
+    const uint32_t first = base + warp * (32 * ITEMS) + lane;
+    uint32_t key[ITEMS];
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t i = base + warp * (32 * kSortItems) + k * 32 + lane;
-        const bool valid = i < n;
-        const uint32_t key = valid ? kin[i] : 0xffffffffu;
-        const uint32_t d = (key >> shift) & (RADIX - 1);
+    for (int k = 0; k < ITEMS; ++k) {
+        const uint32_t i = first + k * 32;
+        key[k] = i < n ? kin[i] : 0xffffffffu;
+    }
+    // this thread's digit: the prefix over the tiles up to this one, the total
+    uint32_t gp = 0, gt = 0;
+    if (!SINGLE && tid < RADIX) {
+        gp = hist[(size_t)tid * tiles + tile];
+        gt = hist[(size_t)tid * tiles + tiles - 1];
+    }
+    for (int d = lane; d < RADIX; d += 32) wcnt[warp][d] = 0;
+    __syncwarp();
+    // the ranks (below 4096) two to a register
+    uint32_t rank2[(ITEMS + 1) / 2];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const bool valid = first + k * 32 < n;
+        const uint32_t d = (key[k] >> shift) & (RADIX - 1);
         uint32_t peers = __ballot_sync(kFull, valid);
 #pragma unroll
         for (int b = 0; b < RB; ++b) {
@@ -149,140 +181,140 @@ __global__ void __launch_bounds__(kSortThreads, 4)
             const uint32_t m = __ballot_sync(kFull, bit);
             peers &= bit ? m : ~m;
         }
-        const uint32_t cnt = wcnt[warp][d];
-        const uint32_t r = cnt + __popc(peers & lt);
+        if (!valid) peers = 1u << lane;
+        // the lowest lane of a digit's group keeps the warp's counter
+        const int lead = __ffs(peers) - 1;
+        uint32_t c = 0;
+        if (valid && lane == lead) {
+            c = wcnt[warp][d];
+            wcnt[warp][d] = c + __popc(peers);
+        }
+        const uint32_t r = __shfl_sync(kFull, c, lead) + __popc(peers & lt);
         if (k & 1)
             rank2[k >> 1] |= r << 16;
         else
             rank2[k >> 1] = r;
         __syncwarp();
-        if (valid && lane == __ffs(peers) - 1) wcnt[warp][d] = cnt + __popc(peers);
-        __syncwarp();
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < RADIX; d += kSortThreads) {
-        uint32_t run = 0;
+    uint32_t val[WITH_VALS ? ITEMS : 1];
+    if (WITH_VALS) {
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint32_t i = first + k * 32;
+            val[k] = vin && i < n ? vin[i] : i;
+        }
+    }
+    // thread d: the digit's counts over the warps, then two exclusive scans
+    // over the digits (this tile's counts, the global totals)
+    uint32_t v = 0;
+    if (tid < RADIX) {
 #pragma unroll
         for (int w = 0; w < kSortWarps; ++w) {
-            uint32_t c = wcnt[w][d];
-            wcnt[w][d] = run;
-            run += c;
+            const uint32_t c = wcnt[w][tid];
+            wcnt[w][tid] = v;
+            v += c;
         }
-        dstart[d] = run;
     }
-    __syncthreads();
-    if (warp == 0) {
-        // exclusive scan of this tile's digit counts; and, over the digits,
-        // of the digit totals (the last tile's inclusive prefixes)
-        constexpr int PER = (RADIX + 31) / 32;
-        uint32_t v[PER], tv[PER], s = 0, ts = 0;
+    uint32_t incl = v, tincl = gt;
 #pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int d = lane * PER + j;
-            v[j] = d < RADIX ? dstart[d] : 0;
-            tv[j] = (!SINGLE_TILE && d < RADIX) ? hist[(size_t)d * tiles + tiles - 1] : 0;
-            s += v[j];
-            ts += tv[j];
-        }
-        uint32_t incl = s, tincl = ts;
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, incl, off), ty = __shfl_up_sync(kFull, tincl, off);
+        if (lane >= off) incl += y, tincl += ty;
+    }
+    if (RADIX > 32) {
+        if (lane == 31) wsum[0][warp] = incl, wsum[1][warp] = tincl;
+        __syncthreads();
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, off), ty = __shfl_up_sync(kFull, tincl, off);
-            if (lane >= off) incl += y, tincl += ty;
+        for (int w = 0; w < kSortWarps; ++w) {
+            incl += w < warp ? wsum[0][w] : 0u;
+            tincl += w < warp ? wsum[1][w] : 0u;
         }
-        uint32_t run = incl - s, trun = tincl - ts;
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int d = lane * PER + j;
-            if (d < RADIX) {
-                dstart[d] = run;
-                // the run of digit d from this tile starts after the lower
-                // digits' totals and this digit's runs from earlier tiles
-                gbase[d] = SINGLE_TILE ? run : trun + hist[(size_t)d * tiles + tile] - v[j];
-                run += v[j];
-                trun += tv[j];
-            }
-        }
+    }
+    if (tid < RADIX) {
+        dstart[tid] = incl - v;
+        // the digit's run from this tile starts after the lower digits'
+        // totals and this digit's runs from earlier tiles
+        gofs[tid] = SINGLE ? 0u : (tincl - gt) + (gp - v) - (incl - v);
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t i = base + warp * (32 * kSortItems) + k * 32 + lane;
-        if (i < n) {
-            const uint32_t key = kin[i];
-            const uint32_t d = (key >> shift) & (RADIX - 1);
+    for (int k = 0; k < ITEMS; ++k) {
+        if (first + k * 32 < n) {
+            const uint32_t d = (key[k] >> shift) & (RADIX - 1);
             const uint32_t lp = dstart[d] + wcnt[warp][d] + ((rank2[k >> 1] >> (16 * (k & 1))) & 0xffffu);
-            skeys[lp] = key;
-            if (WITH_VALS) svals[lp] = vin ? vin[i] : i;
+            skeys[CUCO_IDX(lp, TILE)] = key[k];
+            if (WITH_VALS) svals[CUCO_IDX(lp, TILE)] = val[k];
         }
     }
     __syncthreads();
-    const uint32_t tile_n = min((uint32_t)kSortTile, n - base);
-    // (the loop's trip count is the same for every lane of a warp: tile_n
-    // only cuts the last warp's lanes, which still vote)
-    for (uint32_t j0 = 0; j0 < (uint32_t)kSortTile; j0 += kSortThreads) {
-        const uint32_t j = j0 + threadIdx.x;
-        const bool in = j < tile_n;
-        uint32_t kk = 0, o = 0;
-        if (in) {
-            kk = skeys[j];
-            const uint32_t d = (kk >> shift) & (RADIX - 1);
-            o = gbase[d] + j - dstart[d];
+    const uint32_t tile_n = min(TILE, n - base);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const uint32_t j = k * kSortThreads + tid;
+        if (j < tile_n) {
+            const uint32_t kk = skeys[j];
+            const uint32_t o = gofs[(kk >> shift) & (RADIX - 1)] + j;
             kout[CUCO_IDX(o, n)] = kk;
             if (WITH_VALS) vout[CUCO_IDX(o, n)] = svals[j];
-        }
-        if (NEXT) {
-            // one atomic per (digit, destination tile) group of the warp
-            const uint32_t slot = in ? ((kk >> next_shift) & (RADIX - 1)) * tiles + o / kSortTile : 0xffffffffu;
-            const uint32_t peers = __match_any_sync(kFull, slot);
-            if (in && (threadIdx.x & 31) == __ffs(peers) - 1)
-                atomicAdd(&next_hist[CUCO_IDX(slot, (uint32_t)RADIX * tiles)], (uint32_t)__popc(peers));
         }
     }
 }
 
-// One pass.  hist_ready: `hist` already holds this pass's histogram (counted
-// by the previous pass's scatter); next_hist (or null): count the next pass's
-// digits at next_shift into it.
-template <int RB>
-cuco_status_t sort_pass(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout,
-                        bool with_vals, uint32_t *hist, uint32_t n, int shift,
-                        cudaStream_t stream, int *launches, bool hist_ready = false,
-                        uint32_t *next_hist = nullptr, int next_shift = 0) {
-    const uint32_t tiles = (n + kSortTile - 1) / kSortTile;
-    if (tiles == 1) {
-        if (with_vals)
-            k_sort_scatter<RB, true, true, false><<<1, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift,
-                                                                                 hist, tiles, nullptr, 0);
-        else
-            k_sort_scatter<RB, false, true, false><<<1, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift,
-                                                                                  hist, tiles, nullptr, 0);
+// Keys per thread of a tile: the most that leave four tiles for each of ~150
+// SMs (2M pairs, three passes: 8 keys 70 us, 16 keys 83 us; at 4M they are
+// level), in a table of at most hist_words counts (16 always fits); up to
+// 4096 keys are one tile, which needs no histogram.
+int sort_items(uint32_t n, int rb, size_t hist_words) {
+    if (n <= 16u * kSortThreads) return 16;
+    for (int items : {4, 8}) {
+        const uint32_t next = kSortThreads * items * 2;
+        const size_t tiles = (n + kSortThreads * items - 1) / (kSortThreads * items);
+        if (n / next < 608u && (tiles << rb) <= hist_words) return items;
+    }
+    return 16;
+}
+
+// One pass.
+template <int RB, int ITEMS>
+cuco_status_t sort_pass_items(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout,
+                              bool with_vals, uint32_t *hist, uint32_t n, int shift, cudaStream_t stream,
+                              int *launches) {
+    const uint32_t tiles = (n + kSortThreads * ITEMS - 1) / (kSortThreads * ITEMS);
+    auto scatter = [&](auto kernel) {
+        kernel<<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, hist, tiles);
         *launches += 1;
+    };
+    bool single = false;
+    if constexpr (ITEMS == 16) single = tiles == 1;
+    if (single) {
+        if constexpr (ITEMS == 16) {
+            if (with_vals)
+                scatter(k_sort_scatter<RB, ITEMS, true, true>);
+            else
+                scatter(k_sort_scatter<RB, ITEMS, false, true>);
+        }
     } else {
-        if (!hist_ready) {
-            k_sort_hist<RB><<<tiles, kSortThreads, 0, stream>>>(kin, n, shift, hist, tiles);
-            *launches += 1;
-        }
-        k_sort_scan<<<1u << RB, kSortThreads, 0, stream>>>(hist, tiles, next_hist);
-        if (next_hist) {
-            if (with_vals)
-                k_sort_scatter<RB, true, false, true><<<tiles, kSortThreads, 0, stream>>>(
-                    kin, vin, kout, vout, n, shift, hist, tiles, next_hist, next_shift);
-            else
-                k_sort_scatter<RB, false, false, true><<<tiles, kSortThreads, 0, stream>>>(
-                    kin, vin, kout, vout, n, shift, hist, tiles, next_hist, next_shift);
-        } else {
-            if (with_vals)
-                k_sort_scatter<RB, true, false, false><<<tiles, kSortThreads, 0, stream>>>(
-                    kin, vin, kout, vout, n, shift, hist, tiles, nullptr, 0);
-            else
-                k_sort_scatter<RB, false, false, false><<<tiles, kSortThreads, 0, stream>>>(
-                    kin, vin, kout, vout, n, shift, hist, tiles, nullptr, 0);
-        }
+        k_sort_hist<RB, ITEMS><<<tiles, kSortThreads, 0, stream>>>(kin, n, shift, hist, tiles);
+        k_sort_scan<<<1u << RB, kScanThreads, 0, stream>>>(hist, tiles);
         *launches += 2;
+        if (with_vals)
+            scatter(k_sort_scatter<RB, ITEMS, true, false>);
+        else
+            scatter(k_sort_scatter<RB, ITEMS, false, false>);
     }
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
+}
+
+template <int RB>
+cuco_status_t sort_pass(int items, const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout,
+                        bool with_vals, uint32_t *hist, uint32_t n, int shift, cudaStream_t stream, int *launches) {
+    switch (items) {
+        case 4: return sort_pass_items<RB, 4>(kin, vin, kout, vout, with_vals, hist, n, shift, stream, launches);
+        case 8: return sort_pass_items<RB, 8>(kin, vin, kout, vout, with_vals, hist, n, shift, stream, launches);
+        default: return sort_pass_items<RB, 16>(kin, vin, kout, vout, with_vals, hist, n, shift, stream, launches);
+    }
 }
 
 void split_bits(int key_bits, int max_radix_bits, int *passes, int *rb) {
@@ -484,14 +516,15 @@ cuco_status_t launch_cell_subsort(const uint32_t *cell_off, const uint32_t *perm
 size_t sort_hist_entries(uint32_t n, int key_bits, int max_radix_bits) {
     int passes, rb;
     split_bits(key_bits, max_radix_bits, &passes, &rb);
-    size_t tiles = (n + kSortTile - 1) / kSortTile;
+    const uint32_t tile = (uint32_t)kSortThreads * sort_items(n, rb, ~(size_t)0);
+    const size_t tiles = (n + tile - 1) / tile;
     return (size_t)(1u << rb) * (tiles ? tiles : 1);
 }
 
 cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in,
-                         uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *hist, uint32_t n,
+                         uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *hist, size_t hist_words, uint32_t n,
                          int key_bits, int max_radix_bits, cudaStream_t stream,
-                         bool *result_in_alt, int *launches, uint32_t *hist2) {
+                         bool *result_in_alt, int *launches) {
     int passes, rb;
     split_bits(key_bits, max_radix_bits, &passes, &rb);
     bool with_vals = vals != nullptr;
@@ -499,22 +532,16 @@ cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in
     if (n == 0) return CUCO_OK;
     uint32_t *kbuf[2] = {keys, keys_alt};
     uint32_t *vbuf[2] = {vals, vals_alt};
-    uint32_t *hbuf[2] = {hist, hist2 ? hist2 : hist};
+    const int items = sort_items(n, rb, hist_words);
     int cur = 0;
     for (int p = 0; p < passes; ++p) {
         const uint32_t *vin = (p == 0) ? vals_in : vbuf[cur];
         const int shift = p * rb;
-        // with two histograms, pass p uses hbuf[p & 1] and counts pass p+1's
-        // digits into the other
-        const bool fused = hist2 != nullptr;
-        uint32_t *h = hbuf[fused ? (p & 1) : 0];
-        uint32_t *hn = fused && p + 1 < passes ? hbuf[(p + 1) & 1] : nullptr;
-        const bool ready = fused && p > 0;
         cuco_status_t s;
         switch (rb) {
-#define CUCO_SORT_PASS(R)                                                                                    \
-    s = sort_pass<R>(kbuf[cur], vin, kbuf[cur ^ 1], vbuf[cur ^ 1], with_vals, h, n, shift, stream, launches, \
-                     ready, hn, shift + rb)
+#define CUCO_SORT_PASS(R)                                                                                         \
+    s = sort_pass<R>(items, kbuf[cur], vin, kbuf[cur ^ 1], vbuf[cur ^ 1], with_vals, hist, n, shift, stream, \
+                     launches)
             case 4: CUCO_SORT_PASS(4); break;
             case 5: CUCO_SORT_PASS(5); break;
             case 6: CUCO_SORT_PASS(6); break;
@@ -565,65 +592,73 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, float4 *sorted_pos,
 // launches: each block's maximum, then every block its cells after the
 // maximum of the blocks before it.
 namespace {
-constexpr uint32_t kOffBlock = 4096;  // cells per block
+constexpr uint32_t kOffItems = 4, kOffBlock = kSortThreads * kOffItems;  // cells per block
 
-__device__ __forceinline__ uint32_t end_of(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                                           uint32_t c, uint32_t ncells) {
-    return c < ncells && start[c] != kEmptyCell ? end[c] : 0u;
+// this thread's kOffItems consecutive cells: the largest end of each
+__device__ __forceinline__ void load_ends(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+                                          uint32_t ncells, uint32_t (&v)[kOffItems]) {
+    const uint32_t c0 = blockIdx.x * kOffBlock + threadIdx.x * kOffItems;
+    uint32_t s[kOffItems], e[kOffItems];
+#pragma unroll
+    for (uint32_t k = 0; k < kOffItems; ++k) {
+        s[k] = c0 + k < ncells ? start[c0 + k] : kEmptyCell;
+        e[k] = c0 + k < ncells ? end[c0 + k] : 0u;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kOffItems; ++k) v[k] = s[k] != kEmptyCell ? e[k] : 0u;
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_block_end_max(const uint32_t *__restrict__ start,
                                                                 const uint32_t *__restrict__ end, uint32_t ncells,
                                                                 uint32_t *__restrict__ block_max) {
-    __shared__ uint32_t s_max;
-    if (threadIdx.x == 0) s_max = 0;
-    __syncthreads();
-    uint32_t m = 0;
-#pragma unroll 4
-    for (uint32_t k = threadIdx.x; k < kOffBlock; k += kSortThreads)
-        m = max(m, end_of(start, end, blockIdx.x * kOffBlock + k, ncells));
+    __shared__ uint32_t s_max[kSortWarps];
+    uint32_t v[kOffItems], m = 0;
+    load_ends(start, end, ncells, v);
+#pragma unroll
+    for (uint32_t k = 0; k < kOffItems; ++k) m = max(m, v[k]);
     m = __reduce_max_sync(kFull, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, m);
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x == 0) block_max[blockIdx.x] = s_max;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kSortWarps; ++w) m = max(m, s_max[w]);
+        block_max[blockIdx.x] = m;
+    }
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_start_end_offsets(const uint32_t *__restrict__ start,
                                                                     const uint32_t *__restrict__ end, uint32_t ncells,
                                                                     const uint32_t *__restrict__ block_max,
                                                                     uint32_t *__restrict__ cell_off) {
-    __shared__ uint32_t s_carry, s_warp[kSortWarps];
+    __shared__ uint32_t s_carry[kSortWarps], s_warp[kSortWarps];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_carry = 0;
-    __syncthreads();
+    uint32_t v[kOffItems];
+    load_ends(start, end, ncells, v);
     uint32_t carry = 0;
     for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kSortThreads) carry = max(carry, block_max[k]);
     carry = __reduce_max_sync(kFull, carry);
-    if (lane == 0) atomicMax(&s_carry, carry);
-    __syncthreads();
-    carry = s_carry;
-    for (uint32_t k = 0; k < kOffBlock; k += kSortThreads) {
-        const uint32_t c = blockIdx.x * kOffBlock + k + threadIdx.x;
-        uint32_t incl = end_of(start, end, c, ncells);
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, off);
-            if (lane >= off) incl = max(incl, v);
-        }
-        if (lane == 31) s_warp[warp] = incl;
-        __syncthreads();
-        uint32_t before = carry, all = carry;
-        for (uint32_t w = 0; w < (uint32_t)kSortWarps; ++w) {
-            if (w < warp) before = max(before, s_warp[w]);
-            all = max(all, s_warp[w]);
-        }
-        incl = max(incl, before);
-        // cell c ends, and the next begins, at the largest end so far
-        if (c < ncells) cell_off[c + 1] = incl;
-        if (c == 0) cell_off[0] = 0;
-        carry = all;
-        __syncthreads();  // s_warp is rewritten by the next round
+    for (uint32_t k = 1; k < kOffItems; ++k) v[k] = max(v[k], v[k - 1]);
+    uint32_t incl = v[kOffItems - 1];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, incl, off);
+        if (lane >= off) incl = max(incl, u);
     }
+    uint32_t before = __shfl_up_sync(kFull, incl, 1);
+    if (lane == 0) before = 0;
+    if (lane == 31) s_warp[warp] = incl;
+    if (lane == 0) s_carry[warp] = carry;
+    __syncthreads();
+    for (uint32_t w = 0; w < (uint32_t)kSortWarps; ++w) {
+        before = max(before, s_carry[w]);
+        if (w < warp) before = max(before, s_warp[w]);
+    }
+    // cell c ends, and the next begins, at the largest end so far
+    const uint32_t c0 = blockIdx.x * kOffBlock + threadIdx.x * kOffItems;
+#pragma unroll
+    for (uint32_t k = 0; k < kOffItems; ++k)
+        if (c0 + k < ncells) cell_off[c0 + k + 1] = max(before, v[k]);
+    if (c0 == 0) cell_off[0] = 0;
 }
 }  // namespace
 

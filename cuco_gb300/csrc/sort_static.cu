@@ -91,7 +91,7 @@ extern "C" cuco_status_t cuco_radix_sort_noalloc(uint32_t *keys, uint32_t *value
     bool in_alt = false;
     int launches = 0;
     // digits of at most 8 bits: the histogram holds 2^8 * ceil(n/4096) words
-    CUCO_TRY(sort_pairs(keys, values, values, tmp_keys, values ? tmp_vals : nullptr, hist, n,
+    CUCO_TRY(sort_pairs(keys, values, values, tmp_keys, values ? tmp_vals : nullptr, hist, kHistWords, n,
                         (int)key_bits, 8, s, &in_alt, &launches));
     if (in_alt) {
         CUCO_TRY_CUDA(cudaMemcpyAsync(keys, tmp_keys, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
