@@ -222,6 +222,7 @@ cuco_status_t launch_shortrange_multi(const void *descs, const double2 *kicks, c
 
 struct PMPlan {
     int M;
+    uint32_t stages;    // the Stockham transform's radices (meshes without register transforms)
     bool fixed;         // positions are 32-bit fixed point (units of L / 2^32)
     float boxsize;
     float to_slab_fac;  // M / L in float (pm_periodic.c:42)
@@ -230,7 +231,7 @@ struct PMPlan {
     float *rho;         // M^3 real grid: the potential
     unsigned long long *rho64;  // M^3 deposited mass in units of m / 2^32
     bool rho64_dirty;   // rho64 may hold sums (the z pass clears what it reads)
-    float2 *spec;       // M*M*(M/2+1) complex grid
+    float2 *spec;       // half spectrum, pm_spec_points(M)
     float *green1d;     // M/2+1: exp(-k^2 a) / sinc(pi k/M)^4
     float2 *twiddle;    // M: exp(-2 pi i t / M)
 };
@@ -248,11 +249,12 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, uint32_t n, float4 *acc
 // Many boxes' meshes in one launch per PM phase (the batched form).
 struct PMBoxDesc {
     int M, P, B;         // mesh; z-pass row pairs and axis-pass columns per CTA
+    uint32_t stages;     // pm_stage_plan(M)
     float to_slab_fac, mass, fd_fac;
     float *rho;          // this box's M^3 real grid (the potential)
     unsigned long long *rho64;  // its deposited mass, units of m / 2^32
     float mscale;        // m / 2^32
-    float2 *spec;        // its M*M*(M/2+1) half spectrum
+    float2 *spec;        // its half spectrum, pm_spec_points(M)
     const float *green1d;
     const float2 *twiddle;
 };
@@ -273,6 +275,10 @@ struct PMMulti {
 // register transforms, which run in kernels of their own.
 bool pm_big_fft(int M, int P, int B);
 bool pm_fft_batches_ok(int M, int P, int B);
+// Radices of a mesh's Stockham transform, five bits each.
+uint32_t pm_stage_plan(int M);
+// Points of a mesh's half-spectrum array.
+size_t pm_spec_points(int M);
 int pm_batch_z(int M);
 int pm_batch_axis(int M);
 size_t pm_smem_z(int M, int P);

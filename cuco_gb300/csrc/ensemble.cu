@@ -217,7 +217,7 @@ void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out
     uint32_t *pbeg = nullptr;
     uint2 *mz = nullptr, *ma = nullptr;
     bool ok = dalloc(&rho, (size_t)M * M * M) == CUCO_OK && dalloc(&rho64, (size_t)M * M * M) == CUCO_OK &&
-              dalloc(&spec, (size_t)M * M * Mh) == CUCO_OK &&
+              dalloc(&spec, pm_spec_points(M)) == CUCO_OK &&
               dalloc(&green, Mh) == CUCO_OK && dalloc(&tw, (size_t)M) == CUCO_OK && dalloc(&dd, 1) == CUCO_OK &&
               dalloc(&pbeg, 2) == CUCO_OK && dalloc(&mz, (size_t)M * M) == CUCO_OK &&
               dalloc(&ma, (size_t)M * Mh) == CUCO_OK;
@@ -238,7 +238,7 @@ void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out
             if (P > M / 2 || (M * M / 2) % P || pm_smem_z(M, P) > 200 * 1024) continue;
             for (int B : {4, 8, 16}) {
                 if (pm_smem_axis(M, B) > 200 * 1024 || !pm_fft_batches_ok(M, P, B)) continue;
-                PMBoxDesc d{M, P, B, 1.f, 0.f, 0.f, rho, rho64, 1.f, spec, green, tw};
+                PMBoxDesc d{M, P, B, pm_stage_plan(M), 1.f, 0.f, 0.f, rho, rho64, 1.f, spec, green, tw};
                 cudaMemcpy(dd, &d, sizeof d, cudaMemcpyHostToDevice);
                 const uint32_t nz = (uint32_t)(M * M / (2 * P)), nbx = (uint32_t)((Mh + B - 1) / B),
                                na = nbx * M;
@@ -499,7 +499,7 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
         pbeg[b + 1] = pbeg[b] + (uint32_t)c.n;
         cbase[b + 1] = cbase[b] + G * G * G;
         mbase[b + 1] = mbase[b] + M * M * M;
-        sbase[b + 1] = sbase[b] + M * M * (M / 2 + 1);
+        sbase[b + 1] = sbase[b] + pm_spec_points((int)M);
         gbase[b + 1] = gbase[b] + (M / 2 + 1);
         tbase[b + 1] = tbase[b] + M;
         maxn = std::max(maxn, (size_t)c.n);
@@ -602,7 +602,7 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
         const int M = c.pm_grid, Mh = M / 2 + 1;
         drift[b] = DriftBox{(uint32_t)c.cell_grid, (uint32_t)cbase[b], c.boxsize, (float)c.cell_grid / c.boxsize};
         pm_tables(M, c.boxsize, c.asmth, green.data() + gbase[b], tw.data() + tbase[b]);
-        pmd[b] = PMBoxDesc{M, P[b], B[b], (float)M / c.boxsize, c.mass, pm_fd_fac(M, c.boxsize, c.G),
+        pmd[b] = PMBoxDesc{M, P[b], B[b], pm_stage_plan(M), (float)M / c.boxsize, c.mass, pm_fd_fac(M, c.boxsize, c.G),
                            e->rho + mbase[b], e->rho64 + mbase[b], ldexpf(c.mass, -32), e->spec + sbase[b],
                            e->green + gbase[b], e->tw + tbase[b]};
         const uint32_t nz = (uint32_t)(M * M / (2 * P[b]));
@@ -924,7 +924,7 @@ cuco_status_t cuco_ensemble_footprint(const cuco_config_t *boxes, int nbox, uint
         const uint64_t G = boxes[k].cell_grid > 0 ? (uint64_t)boxes[k].cell_grid : M / 2;  // the largest tuned grid
         b += n * (6 * sizeof(float4) + 4 * sizeof(uint32_t));    // state, sorted copies, keys
         b += 4 * (G * G * G + 1) + 16 * G * G * G;               // cell offsets, z-slice counts
-        b += 12 * M * M * M + 8 * M * M * (M / 2 + 1);           // deposit + real grid + half spectrum
+        b += 12 * M * M * M + 8 * pm_spec_points((int)M);        // deposit + real grid + half spectrum
         b += 12 * (M / 2 + 1) + 8 * M + 2048 + 16 * (M * M);    // tables, descriptors, CTA maps
         maxn = std::max(maxn, n);
     }

@@ -29,7 +29,7 @@
 // meshes up to 1024 use a two-level transform with the points in registers
 // (RegFFT; the one-box axis passes with their column batch fixed at compile
 // time, fft_axis_reg_fixed); other meshes M = 2^a 3^b 5^c use a shared-memory
-// Stockham FFT over a batch of columns with radix-4/2/3/5 stages.  Twiddles
+// Stockham FFT over a batch of columns with stages of radix 2 to 16.  Twiddles
 // come from an FP64-built table.
 // The Green's function factorises: smth(k) = -g(kx) g(ky) g(kz) / k^2 with
 // g(k) = exp(-k^2 (2 pi asmth / L)^2) / sinc(pi k / M)^4, built in FP64.
@@ -46,13 +46,39 @@ namespace {
 constexpr int kFFTThreads = 256;
 constexpr int kLoadBatch = 8;  // global loads issued per thread before use
 
+// Points from one (x, y) row of the half spectrum to the next.  (Rounded up to
+// whole 32-byte sectors the axis passes gained 3 % at M = 512 and the inverse
+// z pass lost a quarter.)
+__host__ __device__ constexpr int spec_stride(int M) { return M / 2 + 1; }
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// Stage radix for the remaining length: 4, 2, 3 or 5 (M = 2^a 3^b 5^c).
-__host__ __device__ __forceinline__ int stage_radix(int rem) {
-    return (rem & 3) == 0 ? 4 : (rem & 1) == 0 ? 2 : rem % 3 == 0 ? 3 : 5;
+// The stages of a mesh's Stockham transform, largest radix first, five bits
+// each (0 ends): the fewest stages of radix at most 16, of those the smallest
+// radix sum.  Every stage is one round trip through shared memory and one CTA
+// barrier, which is what these passes spend their time on: M = 384 takes 3
+// stages (8 8 6) instead of the 5 of radices 4, 2, 3, and 5; M = 200 3 instead
+// of 4; most meshes to 240 take 2.
+constexpr int kRadices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+uint32_t stage_plan(int M) {
+    struct Best {
+        int stages = 99, sum = 0;
+        uint32_t plan = 0;
+    } best;
+    auto search = [&](auto &&self, int rem, int from, int stages, int sum, uint32_t plan) -> void {
+        if (rem == 1) {
+            if (stages < best.stages || (stages == best.stages && sum < best.sum)) best = {stages, sum, plan};
+            return;
+        }
+        if (stages == 6) return;
+        for (int i = from; i < (int)(sizeof kRadices / sizeof kRadices[0]); ++i)
+            if (rem % kRadices[i] == 0)
+                self(self, rem / kRadices[i], i, stages + 1, sum + kRadices[i], plan | (uint32_t)kRadices[i] << (5 * stages));
+    };
+    search(search, M, 0, 0, 0, 0u);
+    return best.plan;
 }
 
 // Division by a runtime d without a divide instruction: j / d is
@@ -110,12 +136,80 @@ __device__ __forceinline__ void dft_small(float2 (&v)[R], int sign) {
     }
 }
 
+// sin(2 pi j / n) in double at compile time (Taylor, the angle reduced to
+// [-pi/4, pi/4] and an octant)
+constexpr double kTau = 6.283185307179586476925286766559;
+constexpr double taylor(double x, bool cosine) {
+    double term = cosine ? 1.0 : x, sum = term;
+    for (int k = cosine ? 1 : 2; k < 24; k += 2) {
+        term *= -x * x / (k * (k + 1));
+        sum += term;
+    }
+    return sum;
+}
+constexpr double sin_turns(int j, int n) {
+    j = ((j % n) + n) % n;
+    // octant q of 8 j / n, rounded; the rest of the angle
+    const int q = (16 * j + n) / (2 * n);
+    const double x = kTau * ((double)j / n - q / 8.0);
+    const double c = taylor(x, true), s = taylor(x, false), h = 0.70710678118654752440084436210485;
+    switch (q & 7) {
+        case 0: return s;
+        case 1: return h * (c + s);
+        case 2: return c;
+        case 3: return h * (c - s);
+        case 4: return -s;
+        case 5: return -h * (c + s);
+        case 6: return -c;
+        default: return h * (s - c);
+    }
+}
+template <int N>
+struct Roots {
+    float c[N], s[N];
+    constexpr Roots() : c(), s() {
+        for (int j = 0; j < N; ++j) c[j] = (float)sin_turns(4 * j + N, 4 * N), s[j] = (float)sin_turns(j, N);
+    }
+};
+
+// In-register DFT of N points (5-smooth), X[k] = sum_n v[n] exp(S 2 pi i n k / N):
+// N = A Q by Cooley-Tukey with A in {4, 3, 2, 5}; the roots are constants.
+template <int N, int S>
+__device__ __forceinline__ void dft_any(float2 (&v)[N]) {
+    if constexpr (N <= 5) {
+        dft_small<N>(v, S);
+    } else {
+        constexpr int A = N % 4 == 0 ? 4 : N % 3 == 0 ? 3 : N % 2 == 0 ? 2 : 5, Q = N / A;
+        constexpr Roots<N> root;
+        float2 w[N];
+#pragma unroll
+        for (int n2 = 0; n2 < Q; ++n2) {
+            float2 t[A];
+#pragma unroll
+            for (int n1 = 0; n1 < A; ++n1) t[n1] = v[Q * n1 + n2];
+            dft_small<A>(t, S);
+#pragma unroll
+            for (int k1 = 0; k1 < A; ++k1)
+                w[Q * k1 + n2] = n2 * k1 ? cmul(t[k1], make_float2(root.c[n2 * k1 % N], S * root.s[n2 * k1 % N])) : t[k1];
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < A; ++k1) {
+            float2 u[Q];
+#pragma unroll
+            for (int n2 = 0; n2 < Q; ++n2) u[n2] = w[Q * k1 + n2];
+            dft_any<Q, S>(u);
+#pragma unroll
+            for (int k2 = 0; k2 < Q; ++k2) v[k1 + A * k2] = u[k2];
+        }
+    }
+}
+
 // One Stockham stage of radix R over Ns already-combined points, for B = 2^bs
 // columns: reads x[j + p M/R] (p < R), twiddles it by w^{p k M/(Ns R)} (k = j
 // mod Ns), and writes the R-point DFT to y[(j/Ns) Ns R + k + q Ns].
-template <int R>
+template <int R, int S>
 __device__ __forceinline__ void stockham_stage(const float2 *in, float2 *out, const float2 *tw, int M, int Ns,
-                                               int bs, int pitch, int sign) {
+                                               int bs, int pitch) {
     const int nb = M / R, step = M / (Ns * R);
     const FastDiv dns((uint32_t)Ns);
     const int total = nb << bs, bmask = (1 << bs) - 1;
@@ -130,28 +224,40 @@ __device__ __forceinline__ void stockham_stage(const float2 *in, float2 *out, co
 #pragma unroll
             for (int q = 1; q < R; ++q) {
                 float2 w = tw[q * k * step];
-                if (sign > 0) w.y = -w.y;
+                if (S > 0) w.y = -w.y;
                 v[q] = cmul(v[q], w);
             }
         }
-        dft_small<R>(v, sign);
+        dft_any<R, S>(v);
 #pragma unroll
         for (int q = 0; q < R; ++q) out[(dst + q * Ns) * pitch + b] = v[q];
     }
 }
 
-// Transform B = 2^bs columns of length M held in x[m*pitch + b]; returns the
-// buffer holding the result.  sign = -1: forward (e^{-i}), +1: inverse.
-__device__ float2 *fft_columns(float2 *x, float2 *y, const float2 *tw, int M, int bs, int pitch, int sign) {
+// Transform B = 2^bs columns of length M held in x[m*pitch + b] by the stages
+// of `plan`; returns the buffer holding the result.  S = -1: forward (e^{-i}),
+// +1: inverse.
+template <int S>
+__device__ float2 *fft_columns(float2 *x, float2 *y, const float2 *tw, int M, uint32_t plan, int bs, int pitch) {
     int Ns = 1;
     float2 *in = x, *out = y;
-    while (Ns < M) {
-        const int r = stage_radix(M / Ns);
+    for (; plan; plan >>= 5) {
+        const int r = plan & 31;
         switch (r) {
-            case 4: stockham_stage<4>(in, out, tw, M, Ns, bs, pitch, sign); break;
-            case 2: stockham_stage<2>(in, out, tw, M, Ns, bs, pitch, sign); break;
-            case 3: stockham_stage<3>(in, out, tw, M, Ns, bs, pitch, sign); break;
-            default: stockham_stage<5>(in, out, tw, M, Ns, bs, pitch, sign); break;
+#define CUCO_STAGE(R) \
+    case R: stockham_stage<R, S>(in, out, tw, M, Ns, bs, pitch); break
+            CUCO_STAGE(2);
+            CUCO_STAGE(3);
+            CUCO_STAGE(4);
+            CUCO_STAGE(5);
+            CUCO_STAGE(6);
+            CUCO_STAGE(8);
+            CUCO_STAGE(9);
+            CUCO_STAGE(10);
+            CUCO_STAGE(12);
+            CUCO_STAGE(15);
+            default: stockham_stage<16, S>(in, out, tw, M, Ns, bs, pitch); break;
+#undef CUCO_STAGE
         }
         __syncthreads();
         float2 *t = in;
@@ -236,11 +342,17 @@ __device__ __forceinline__ void dft_reg(float2 (&v)[N]) {
     }
 }
 
+// Shared memory: point `row` of column b is at (row + row / M2) * pitch + b, one
+// spare row after every M2.  The second level's threads read rows M2 apart;
+// without the spare row those are a multiple of 16 float2 apart and all fall
+// on one bank.
 template <int M1, int M2>
 struct RegFFT {
-    static constexpr int M = M1 * M2, N1 = M1, N2 = M2;
-    // a column takes max(M1, M2) threads
+    static constexpr int M = M1 * M2, N1 = M1, N2 = M2, T = M1 > M2 ? M1 : M2;
+    static constexpr int ROWS = M + M1;  // a column's rows with the spare ones
+    // a column takes T threads
     __device__ static int slot(int k) { return M2 * (k & (M1 - 1)) + k / M1; }
+    __device__ static int at(int row, int pitch) { return (row + row / M2) * pitch; }
     // twiddle exp(S 2 pi i j / M) from the table of exp(-2 pi i j / M)
     template <int S>
     __device__ static float2 tw(const float2 *tw_s, int j) {
@@ -248,29 +360,50 @@ struct RegFFT {
         if (S > 0) w.y = -w.y;
         return w;
     }
-    // the 2^lb columns x[m * pitch + b]: natural order in, slot order out
+    // first level: the M1-point transforms over points M2 apart, twiddled
+    template <int S>
+    __device__ static void forward_first(float2 *x, const float2 *tw_s, int pitch, int b, int n2) {
+        float2 v[M1];
+#pragma unroll
+        for (int n1 = 0; n1 < M1; ++n1) v[n1] = x[at(M2 * n1 + n2, pitch) + b];
+        dft_reg<M1, S>(v);
+#pragma unroll
+        for (int k1 = 0; k1 < M1; ++k1) x[at(M2 * k1 + n2, pitch) + b] = k1 ? cmul(v[k1], tw<S>(tw_s, n2 * k1)) : v[k1];
+    }
+    // second level: u[k2] = X[k1 + M1 k2]
+    template <int S>
+    __device__ static void forward_second(const float2 *x, int pitch, int b, int k1, float2 (&u)[M2]) {
+#pragma unroll
+        for (int n2 = 0; n2 < M2; ++n2) u[n2] = x[at(M2 * k1 + n2, pitch) + b];
+        dft_reg<M2, S>(u);
+    }
+    // the inverse's first level, from u[k2] = X[k1 + M1 k2]
+    template <int S>
+    __device__ static void inverse_first(float2 *x, const float2 *tw_s, int pitch, int b, int k1, float2 (&u)[M2]) {
+        dft_reg<M2, S>(u);
+#pragma unroll
+        for (int n2 = 0; n2 < M2; ++n2) x[at(M2 * k1 + n2, pitch) + b] = k1 ? cmul(u[n2], tw<S>(tw_s, n2 * k1)) : u[n2];
+    }
+    template <int S>
+    __device__ static void inverse_second(float2 *x, int pitch, int b, int n2) {
+        float2 v[M1];
+#pragma unroll
+        for (int k1 = 0; k1 < M1; ++k1) v[k1] = x[at(M2 * k1 + n2, pitch) + b];
+        dft_reg<M1, S>(v);
+#pragma unroll
+        for (int n1 = 0; n1 < M1; ++n1) x[at(M2 * n1 + n2, pitch) + b] = v[n1];
+    }
+    // the 2^lb columns of x: natural order in, slot order out
     template <int S>
     __device__ static void forward(float2 *x, const float2 *tw_s, int pitch, int lb) {
         const int b = threadIdx.x & ((1 << lb) - 1), r = threadIdx.x >> lb;
-        if (r < M2) {
-            const int n2 = r;
-            float2 v[M1];
-#pragma unroll
-            for (int n1 = 0; n1 < M1; ++n1) v[n1] = x[(M2 * n1 + n2) * pitch + b];
-            dft_reg<M1, S>(v);
-#pragma unroll
-            for (int k1 = 0; k1 < M1; ++k1)
-                x[(M2 * k1 + n2) * pitch + b] = k1 ? cmul(v[k1], tw<S>(tw_s, n2 * k1)) : v[k1];
-        }
+        if (r < M2) forward_first<S>(x, tw_s, pitch, b, r);
         __syncthreads();
         if (r < M1) {
-            const int k1 = r;
             float2 u[M2];
+            forward_second<S>(x, pitch, b, r, u);
 #pragma unroll
-            for (int n2 = 0; n2 < M2; ++n2) u[n2] = x[(M2 * k1 + n2) * pitch + b];
-            dft_reg<M2, S>(u);
-#pragma unroll
-            for (int k2 = 0; k2 < M2; ++k2) x[(M2 * k1 + k2) * pitch + b] = u[k2];
+            for (int k2 = 0; k2 < M2; ++k2) x[at(M2 * r + k2, pitch) + b] = u[k2];
         }
         __syncthreads();
     }
@@ -279,25 +412,34 @@ struct RegFFT {
     __device__ static void inverse(float2 *x, const float2 *tw_s, int pitch, int lb) {
         const int b = threadIdx.x & ((1 << lb) - 1), r = threadIdx.x >> lb;
         if (r < M1) {
-            const int k1 = r;
             float2 u[M2];
 #pragma unroll
-            for (int k2 = 0; k2 < M2; ++k2) u[k2] = x[(M2 * k1 + k2) * pitch + b];
-            dft_reg<M2, S>(u);
-#pragma unroll
-            for (int n2 = 0; n2 < M2; ++n2)
-                x[(M2 * k1 + n2) * pitch + b] = k1 ? cmul(u[n2], tw<S>(tw_s, n2 * k1)) : u[n2];
+            for (int k2 = 0; k2 < M2; ++k2) u[k2] = x[at(M2 * r + k2, pitch) + b];
+            inverse_first<S>(x, tw_s, pitch, b, r, u);
         }
         __syncthreads();
-        if (r < M2) {
-            const int n2 = r;
-            float2 v[M1];
+        if (r < M2) inverse_second<S>(x, pitch, b, r);
+        __syncthreads();
+    }
+    // natural order in and out: forward transform, each X[m] times mul(m),
+    // inverse transform; the spectrum stays in the second level's registers
+    template <typename Mul>
+    __device__ static void filter(float2 *x, const float2 *tw_s, int pitch, int lb, Mul mul) {
+        const int b = threadIdx.x & ((1 << lb) - 1), r = threadIdx.x >> lb;
+        if (r < M2) forward_first<-1>(x, tw_s, pitch, b, r);
+        __syncthreads();
+        if (r < M1) {
+            float2 u[M2];
+            forward_second<-1>(x, pitch, b, r, u);
 #pragma unroll
-            for (int k1 = 0; k1 < M1; ++k1) v[k1] = x[(M2 * k1 + n2) * pitch + b];
-            dft_reg<M1, S>(v);
-#pragma unroll
-            for (int n1 = 0; n1 < M1; ++n1) x[(M2 * n1 + n2) * pitch + b] = v[n1];
+            for (int k2 = 0; k2 < M2; ++k2) {
+                const float g = mul(r + M1 * k2);
+                u[k2] = make_float2(u[k2].x * g, u[k2].y * g);
+            }
+            inverse_first<+1>(x, tw_s, pitch, b, r, u);
         }
+        __syncthreads();
+        if (r < M2) inverse_second<+1>(x, pitch, b, r);
         __syncthreads();
     }
 };
@@ -322,112 +464,140 @@ __host__ __device__ inline bool reg_fft_ok(int M, int cols) {
 }
 
 // The passes below with the register transforms (M = FT::M; one buffer of
-// M * pitch points, the twiddle table after it).
+// FT::ROWS * pitch points, the twiddle table after it).
+//
+// z passes: the pitch P + 1 keeps a row's consecutive points on different
+// banks where global rows are read or written along m or k, and (M2 + 1)
+// (P + 1), odd, does so for the slot order: the two rows' spectra are taken
+// straight from the transform's slots, and the inverse's slots filled
+// straight from the rows, with no staging block.
 template <typename FT>
 __device__ __forceinline__ void fft_z_r2c_reg(unsigned long long *__restrict__ rho64, float mscale,
                                               float2 *__restrict__ spec, const float2 *tw, int P, int blk) {
-    constexpr int M = FT::M, Mh = M / 2 + 1;
+    constexpr int M = FT::M, stride = spec_stride(M), kBatch = 4;
     extern __shared__ float2 sm[];
     const int pitch = P + 1;
-    float2 *x = sm, *tw_s = sm + M * pitch;
+    float2 *x = sm, *tw_s = sm + FT::ROWS * pitch;
     const size_t r0 = (size_t)blk * 2 * P;
     load_twiddles(tw_s, tw, M);
-    // rows 2pr and 2pr+1 packed as one complex column, one float2 per thread
-    // and element (both reads coalesced along the rows); every sum read is
-    // cleared for the next deposit
-    for (int e0 = threadIdx.x; e0 < P * M; e0 += kLoadBatch * blockDim.x) {
-        float2 v[kLoadBatch];
+    // rows 2pr and 2pr+1 packed as one complex column, two points a thread
+    // and load; every sum read is cleared for the next deposit
+    const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
+    for (int e0 = threadIdx.x; e0 < P * (M / 2); e0 += kBatch * blockDim.x) {
+        ulonglong2 a[kBatch], c[kBatch];
 #pragma unroll
-        for (int u = 0; u < kLoadBatch; ++u) {
+        for (int u = 0; u < kBatch; ++u) {
             const int e = e0 + u * blockDim.x;
-            v[u] = make_float2(0.f, 0.f);
-            if (e < P * M) {
-                const int pr = e / M, m = e & (M - 1);
-                const size_t g = (r0 + 2 * pr) * M + m;
-                v[u] = make_float2(__fmul_rn(__ull2float_rn(rho64[g]), mscale),
-                                   __fmul_rn(__ull2float_rn(rho64[g + M]), mscale));
+            if (e < P * (M / 2)) {
+                const int pr = e / (M / 2), m = 2 * (e & (M / 2 - 1));
+                const ulonglong2 *g = reinterpret_cast<const ulonglong2 *>(rho64 + (r0 + 2 * pr) * M + m);
+                a[u] = g[0];
+                c[u] = g[M / 2];
             }
         }
 #pragma unroll
-        for (int u = 0; u < kLoadBatch; ++u) {
+        for (int u = 0; u < kBatch; ++u) {
             const int e = e0 + u * blockDim.x;
-            if (e < P * M) {
-                const int pr = e / M, m = e & (M - 1);
-                const size_t g = (r0 + 2 * pr) * M + m;
-                rho64[g] = 0ull;
-                rho64[g + M] = 0ull;
-                x[m * pitch + pr] = v[u];
+            if (e < P * (M / 2)) {
+                const int pr = e / (M / 2), m = 2 * (e & (M / 2 - 1));
+                ulonglong2 *g = reinterpret_cast<ulonglong2 *>(rho64 + (r0 + 2 * pr) * M + m);
+                g[0] = zero;
+                g[M / 2] = zero;
+                x[FT::at(m, pitch) + pr] = make_float2(__fmul_rn(__ull2float_rn(a[u].x), mscale),
+                                                       __fmul_rn(__ull2float_rn(c[u].x), mscale));
+                x[FT::at(m + 1, pitch) + pr] = make_float2(__fmul_rn(__ull2float_rn(a[u].y), mscale),
+                                                           __fmul_rn(__ull2float_rn(c[u].y), mscale));
             }
         }
     }
     __syncthreads();
-    const int ps = ilog2(P);
-    FT::template forward<-1>(x, tw_s, pitch, ps);
-    // Both rows of a pair from the same two transform values, columns
-    // fastest (consecutive banks), into the row-major block y (after the
-    // twiddles; 2P (M/2+1) <= M (P+1) points as P <= M/2); then the block
-    // goes out whole: the CTA's 2P spectrum rows are contiguous.
-    float2 *y = tw_s + M;
-    for (int e = threadIdx.x; e < P * Mh; e += blockDim.x) {
-        const int pr = e & (P - 1), k = e >> ps;
-        const float2 z = x[FT::slot(k) * pitch + pr];
-        float2 zc = x[FT::slot((M - k) & (M - 1)) * pitch + pr];
-        zc.y = -zc.y;
-        y[(2 * pr) * Mh + k] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
-        // (z - zc) / (2i)
-        y[(2 * pr + 1) * Mh + k] = make_float2(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
+    FT::template forward<-1>(x, tw_s, pitch, ilog2(P));
+    // both rows of a pair from the same two transform values, consecutive k
+    for (int e = threadIdx.x; e < P * (M / 2); e += blockDim.x) {
+        const int pr = e / (M / 2), k = e & (M / 2 - 1);
+        auto put = [&](int k) {
+            const float2 z = x[FT::at(FT::slot(k), pitch) + pr];
+            float2 zc = x[FT::at(FT::slot((M - k) & (M - 1)), pitch) + pr];
+            zc.y = -zc.y;
+            float2 *row = spec + (r0 + 2 * pr) * stride + k;
+            row[0] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
+            // (z - zc) / (2i)
+            row[stride] = make_float2(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
+        };
+        put(k);
+        if (k == 0) put(M / 2);
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < 2 * P * Mh; e += blockDim.x) spec[r0 * Mh + e] = y[e];
 }
 
 template <typename FT>
 __device__ __forceinline__ void fft_z_c2r_reg(const float2 *__restrict__ spec, float *__restrict__ out,
                                               const float2 *tw, int P, int blk) {
-    constexpr int M = FT::M, Mh = M / 2 + 1;
+    constexpr int M = FT::M, stride = spec_stride(M);
     extern __shared__ float2 sm[];
     const int pitch = P + 1;
-    float2 *x = sm, *tw_s = sm + M * pitch;
+    float2 *x = sm, *tw_s = sm + FT::ROWS * pitch;
     const size_t r0 = (size_t)blk * 2 * P;
     load_twiddles(tw_s, tw, M);
-    // the CTA's 2P spectrum rows, contiguous, into the row-major block y
-    float2 *y = tw_s + M;
-    for (int e0 = threadIdx.x; e0 < 2 * P * Mh; e0 += kLoadBatch * blockDim.x) {
-        float2 v[kLoadBatch];
-#pragma unroll
-        for (int u = 0; u < kLoadBatch; ++u) {
-            const int e = e0 + u * blockDim.x;
-            v[u] = e < 2 * P * Mh ? spec[r0 * Mh + e] : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < kLoadBatch; ++u) {
-            const int e = e0 + u * blockDim.x;
-            if (e < 2 * P * Mh) y[e] = v[u];
-        }
-    }
-    __syncthreads();
     // row pair pr packed as one complex column a + i b (a, b the Hermitian
     // rows 2pr and 2pr+1, imaginary parts at k = 0 and M/2 dropped), placed
-    // in the slot order the inverse transform starts from; columns fastest
-    const int ps = ilog2(P);
-    for (int e = threadIdx.x; e < P * M; e += blockDim.x) {
-        const int pr = e & (P - 1), k = e >> ps;
-        const int kk = k <= M / 2 ? k : M - k;
-        float2 a = y[(2 * pr) * Mh + kk], b = y[(2 * pr + 1) * Mh + kk];
-        if (k == 0 || k == M / 2) a.y = b.y = 0.f;
-        if (k > M / 2) a.y = -a.y, b.y = -b.y;
-        x[FT::slot(k) * pitch + pr] = make_float2(a.x - b.y, a.y + b.x);  // a + i b
+    // in the slot order the inverse transform starts from: a pair's values at
+    // k give the column's at k and M - k
+    for (int e0 = threadIdx.x; e0 < P * (M / 2); e0 += kLoadBatch * blockDim.x) {
+        float2 a[kLoadBatch], b[kLoadBatch];
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u) {
+            const int e = e0 + u * blockDim.x;
+            if (e < P * (M / 2)) {
+                const float2 *row = spec + (r0 + 2 * (e / (M / 2))) * stride + (e & (M / 2 - 1));
+                a[u] = row[0];
+                b[u] = row[stride];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kLoadBatch; ++u) {
+            const int e = e0 + u * blockDim.x;
+            if (e < P * (M / 2)) {
+                const int pr = e / (M / 2), k = e & (M / 2 - 1);
+                if (k) {
+                    x[FT::at(FT::slot(k), pitch) + pr] = make_float2(a[u].x - b[u].y, a[u].y + b[u].x);      // a + i b
+                    x[FT::at(FT::slot(M - k), pitch) + pr] = make_float2(a[u].x + b[u].y, b[u].x - a[u].y);  // conj a + i conj b
+                } else {
+                    const float2 *row = spec + (r0 + 2 * pr) * stride + M / 2;
+                    x[FT::at(FT::slot(0), pitch) + pr] = make_float2(a[u].x, b[u].x);
+                    x[FT::at(FT::slot(M / 2), pitch) + pr] = make_float2(row[0].x, row[stride].x);
+                }
+            }
+        }
     }
     __syncthreads();
     FT::template inverse<+1>(x, tw_s, pitch, ilog2(P));
     // the pair's two real rows from one transform value
     for (int e = threadIdx.x; e < P * M; e += blockDim.x) {
         const int pr = e / M, m = e & (M - 1);
-        const float2 z = x[m * pitch + pr];
+        const float2 z = x[FT::at(m, pitch) + pr];
         out[(r0 + 2 * pr) * M + m] = z.x;
         out[(r0 + 2 * pr + 1) * M + m] = z.y;
     }
 }
+
+// The Green's factor of the transform index m along x for one (ky, kz):
+// -g(kx) g(ky) g(kz) / k^2, 0 at k = 0.
+struct GreenColumn {
+    const float *green1d;
+    float gy, gz;
+    int c, M;
+    __device__ __forceinline__ GreenColumn(const float *g1, int M_, int o, int kz, bool valid) : green1d(g1), M(M_) {
+        const int ky = o <= M / 2 ? o : M - o;
+        gy = g1[ky];
+        gz = valid ? g1[kz] : 0.f;
+        c = ky * ky + kz * kz;
+    }
+    __device__ __forceinline__ float operator()(int m) const {
+        const int kx = m <= M / 2 ? m : M - m;
+        const int k2 = kx * kx + c;
+        return k2 > 0 ? -green1d[kx] * gy * gz * __frcp_rn((float)k2) : 0.f;
+    }
+};
 
 template <typename FT>
 __device__ __forceinline__ void fft_axis_reg(float2 *__restrict__ spec, const float2 *tw,
@@ -436,10 +606,10 @@ __device__ __forceinline__ void fft_axis_reg(float2 *__restrict__ spec, const fl
     constexpr int M = FT::M, Mh = M / 2 + 1;
     extern __shared__ float2 sm[];
     const int pitch = B;
-    float2 *x = sm, *tw_s = sm + M * pitch;
+    float2 *x = sm, *tw_s = sm + FT::ROWS * pitch;
     const int o = by, kz0 = bx * B, bsh = ilog2(B), nb = min(B, Mh - kz0);
-    const size_t sm_stride = axis == 1 ? (size_t)Mh : (size_t)M * Mh;
-    const size_t base = axis == 1 ? (size_t)o * M * Mh : (size_t)o * Mh;
+    const size_t sm_stride = axis == 1 ? (size_t)spec_stride(M) : (size_t)M * spec_stride(M);
+    const size_t base = (size_t)o * (axis == 1 ? M : 1) * spec_stride(M);
     // an inverse-only pass starts from the slot order
     const bool to_slots = sign > 0;
     load_twiddles(tw_s, tw, M);
@@ -456,142 +626,129 @@ __device__ __forceinline__ void fft_axis_reg(float2 *__restrict__ spec, const fl
             const int e = e0 + u * blockDim.x;
             if (e < M * B) {
                 const int m = e >> bsh, b = e & (B - 1);
-                x[(to_slots ? FT::slot(m) : m) * pitch + b] = v[u];
+                x[FT::at(to_slots ? FT::slot(m) : m, pitch) + b] = v[u];
             }
         }
     }
     __syncthreads();
     bool natural = true;
-    if (sign < 0) {
+    if (sign < 0 && green) {
+        const int b = threadIdx.x & (B - 1);
+        FT::filter(x, tw_s, pitch, bsh, GreenColumn(green1d, M, o, kz0 + b, b < nb));
+    } else if (sign < 0) {
         FT::template forward<-1>(x, tw_s, pitch, bsh);
         natural = false;
-        if (green) {
-            // slot s = M2 k1 + k2 holds X[k1 + M1 k2]
-            const int ky = o <= M / 2 ? o : M - o;
-            const float gy = green1d[ky];
-            for (int e = threadIdx.x; e < M * B; e += blockDim.x) {
-                const int sl = e >> bsh, b = e & (B - 1);
-                const int k1 = sl / FT::N2, k2 = sl - k1 * FT::N2;
-                const int m = k1 + FT::N1 * k2;  // the transform index along x
-                const int kx = m <= M / 2 ? m : M - m;
-                const int kz = kz0 + b;
-                const float2 v = x[sl * pitch + b];
-                float g = 0.f;
-                if (b < nb) {
-                    const int k2s = kx * kx + ky * ky + kz * kz;
-                    if (k2s > 0) g = -green1d[kx] * gy * green1d[kz] * __frcp_rn((float)k2s);
-                }
-                x[sl * pitch + b] = make_float2(v.x * g, v.y * g);
-            }
-            __syncthreads();
-            FT::template inverse<+1>(x, tw_s, pitch, bsh);
-            natural = true;
-        }
     } else {
         FT::template inverse<+1>(x, tw_s, pitch, bsh);
     }
     for (int e = threadIdx.x; e < M * B; e += blockDim.x) {
         const int m = e >> bsh, b = e & (B - 1);
-        if (b < nb) spec[base + m * sm_stride + kz0 + b] = x[(natural ? m : FT::slot(m)) * pitch + b];
+        if (b < nb) spec[base + m * sm_stride + kz0 + b] = x[FT::at(natural ? m : FT::slot(m), pitch) + b];
     }
 }
 
-// rows r0 .. r0+2P-1 of the M^3 real grid (row = x*M + y) -> spectrum rows
+// rows r0 .. r0+2P-1 of the M^3 real grid (row = x*M + y) -> spectrum rows,
+// as fft_z_r2c_reg
 __device__ __forceinline__ void fft_z_r2c(unsigned long long *__restrict__ rho64, float mscale,
-                                          float2 *__restrict__ spec, const float2 *tw, int M, int P, int blk) {
+                                          float2 *__restrict__ spec, const float2 *tw, int M, uint32_t plan, int P,
+                                          int blk) {
+    constexpr int kBatch = 4;
     extern __shared__ float2 sm[];
-    const int pitch = P + 1;
+    const int pitch = P + 1, half = M / 2, stride = spec_stride(M);
     float2 *x = sm, *y = sm + M * pitch, *tw_s = sm + 2 * M * pitch;
-    const int Mh = M / 2 + 1;
     const size_t r0 = (size_t)blk * 2 * P;
-    const FastDiv dM((uint32_t)M), dMh((uint32_t)Mh);
-    const int ps = ilog2(P);  // P is a power of two
+    const FastDiv dH((uint32_t)half);
     load_twiddles(tw_s, tw, M);
-    // kLoadBatch loads in flight per thread before their shared-memory stores
-    for (int e0 = threadIdx.x; e0 < 2 * P * M; e0 += kLoadBatch * blockDim.x) {
-        float v[kLoadBatch];
+    const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
+    for (int e0 = threadIdx.x; e0 < P * half; e0 += kBatch * blockDim.x) {
+        ulonglong2 a[kBatch], c[kBatch];
+        ulonglong2 *g[kBatch];
+        int at[kBatch];
 #pragma unroll
-        for (int u = 0; u < kLoadBatch; ++u) {
-            int e = e0 + u * blockDim.x;
-            // the deposit's exact integer sums, rounded once to float
-            v[u] = e < 2 * P * M ? __fmul_rn(__ull2float_rn(rho64[r0 * M + e]), mscale) : 0.f;
+        for (int u = 0; u < kBatch; ++u) {
+            const int e = e0 + u * blockDim.x;
+            if (e < P * half) {
+                const int pr = (int)dH.div((uint32_t)e), m = 2 * (e - pr * half);
+                g[u] = reinterpret_cast<ulonglong2 *>(rho64 + (r0 + 2 * pr) * M + m);
+                at[u] = m * pitch + pr;
+                a[u] = g[u][0];
+                c[u] = g[u][half];
+            }
         }
 #pragma unroll
-        for (int u = 0; u < kLoadBatch; ++u) {
-            int e = e0 + u * blockDim.x;
-            if (e < 2 * P * M) {
-                rho64[r0 * M + e] = 0ull;  // cleared for the next deposit
-                const int row = (int)dM.div((uint32_t)e), m = e - row * M;
-                float *slot = reinterpret_cast<float *>(&x[m * pitch + (row >> 1)]);
-                slot[row & 1] = v[u];
+        for (int u = 0; u < kBatch; ++u) {
+            if (e0 + u * blockDim.x < P * half) {
+                g[u][0] = zero;  // cleared for the next deposit
+                g[u][half] = zero;
+                // the deposit's exact integer sums, rounded once to float
+                x[at[u]] = make_float2(__fmul_rn(__ull2float_rn(a[u].x), mscale),
+                                       __fmul_rn(__ull2float_rn(c[u].x), mscale));
+                x[at[u] + pitch] = make_float2(__fmul_rn(__ull2float_rn(a[u].y), mscale),
+                                               __fmul_rn(__ull2float_rn(c[u].y), mscale));
             }
         }
     }
     __syncthreads();
-    float2 *res = fft_columns(x, y, tw_s, M, ps, pitch, -1);
-    for (int e = threadIdx.x; e < 2 * P * Mh; e += blockDim.x) {
-        const int row = (int)dMh.div((uint32_t)e), k = e - row * Mh, pr = row >> 1;
-        float2 z = res[k * pitch + pr];
-        float2 zc = res[((M - k) % M) * pitch + pr];
-        zc.y = -zc.y;
-        float2 o;
-        if ((row & 1) == 0)
-            o = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
-        else  // (z - zc) / (2i)
-            o = make_float2(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
-        spec[(r0 + row) * Mh + k] = o;
+    float2 *res = fft_columns<-1>(x, y, tw_s, M, plan, ilog2(P), pitch);
+    for (int e = threadIdx.x; e < P * half; e += blockDim.x) {
+        const int pr = (int)dH.div((uint32_t)e), k = e - pr * half;
+        auto put = [&](int k) {
+            const float2 z = res[k * pitch + pr];
+            float2 zc = res[(k ? M - k : 0) * pitch + pr];
+            zc.y = -zc.y;
+            float2 *row = spec + (r0 + 2 * pr) * stride + k;
+            row[0] = make_float2(0.5f * (z.x + zc.x), 0.5f * (z.y + zc.y));
+            // (z - zc) / (2i)
+            row[stride] = make_float2(0.5f * (z.y - zc.y), -0.5f * (z.x - zc.x));
+        };
+        put(k);
+        if (k == 0) put(half);
     }
 }
 
 __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float *__restrict__ out,
-                                          const float2 *tw, int M, int P, int blk) {
+                                          const float2 *tw, int M, uint32_t plan, int P, int blk) {
     extern __shared__ float2 sm[];
-    const int pitch = P + 1;
+    const int pitch = P + 1, half = M / 2, stride = spec_stride(M);
     float2 *x = sm, *y = sm + M * pitch, *tw_s = sm + 2 * M * pitch;
-    const int Mh = M / 2 + 1;
     const size_t r0 = (size_t)blk * 2 * P;
-    const FastDiv dM((uint32_t)M), dMh((uint32_t)Mh);
-    const int ps = ilog2(P);  // P is a power of two
+    const FastDiv dH((uint32_t)half), dM((uint32_t)M);
     load_twiddles(tw_s, tw, M);
-    // rows into y as h[row*Mh + k]
-    for (int e0 = threadIdx.x; e0 < 2 * P * Mh; e0 += kLoadBatch * blockDim.x) {
-        float2 v[kLoadBatch];
+    for (int e0 = threadIdx.x; e0 < P * half; e0 += kLoadBatch * blockDim.x) {
+        float2 a[kLoadBatch], b[kLoadBatch];
 #pragma unroll
         for (int u = 0; u < kLoadBatch; ++u) {
-            int e = e0 + u * blockDim.x;
-            v[u] = e < 2 * P * Mh ? spec[r0 * Mh + e] : make_float2(0.f, 0.f);
+            const int e = e0 + u * blockDim.x;
+            if (e < P * half) {
+                const int pr = (int)dH.div((uint32_t)e);
+                const float2 *row = spec + (r0 + 2 * pr) * stride + (e - pr * half);
+                a[u] = row[0];
+                b[u] = row[stride];
+            }
         }
 #pragma unroll
         for (int u = 0; u < kLoadBatch; ++u) {
-            int e = e0 + u * blockDim.x;
-            if (e < 2 * P * Mh) {
-                const int k = e - (int)dMh.div((uint32_t)e) * Mh;
-                if (k == 0 || k == M / 2) v[u].y = 0.f;
-                y[e] = v[u];
+            const int e = e0 + u * blockDim.x;
+            if (e < P * half) {
+                const int pr = (int)dH.div((uint32_t)e), k = e - pr * half;
+                if (k) {
+                    x[k * pitch + pr] = make_float2(a[u].x - b[u].y, a[u].y + b[u].x);        // a + i b
+                    x[(M - k) * pitch + pr] = make_float2(a[u].x + b[u].y, b[u].x - a[u].y);  // conj a + i conj b
+                } else {
+                    const float2 *row = spec + (r0 + 2 * pr) * stride + half;
+                    x[pr] = make_float2(a[u].x, b[u].x);
+                    x[half * pitch + pr] = make_float2(row[0].x, row[stride].x);
+                }
             }
         }
     }
     __syncthreads();
+    float2 *res = fft_columns<+1>(x, y, tw_s, M, plan, ilog2(P), pitch);
     for (int e = threadIdx.x; e < P * M; e += blockDim.x) {
-        const int pr = e & (P - 1), k = e >> ps;
-        float2 a, b;
-        if (k <= M / 2) {
-            a = y[(2 * pr) * Mh + k];
-            b = y[(2 * pr + 1) * Mh + k];
-        } else {
-            a = y[(2 * pr) * Mh + (M - k)];
-            b = y[(2 * pr + 1) * Mh + (M - k)];
-            a.y = -a.y;
-            b.y = -b.y;
-        }
-        x[k * pitch + pr] = make_float2(a.x - b.y, a.y + b.x);  // a + i b
-    }
-    __syncthreads();
-    float2 *res = fft_columns(x, y, tw_s, M, ps, pitch, +1);
-    for (int e = threadIdx.x; e < 2 * P * M; e += blockDim.x) {
-        const int row = (int)dM.div((uint32_t)e), m = e - row * M;
-        float2 z = res[m * pitch + (row >> 1)];
-        out[(r0 + row) * M + m] = (row & 1) ? z.y : z.x;
+        const int pr = (int)dM.div((uint32_t)e), m = e - pr * M;
+        const float2 z = res[m * pitch + pr];
+        out[(r0 + 2 * pr) * M + m] = z.x;
+        out[(r0 + 2 * pr + 1) * M + m] = z.y;
     }
 }
 
@@ -599,7 +756,7 @@ __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float
 // with the Green's multiply and inverse transform when green != 0; columns
 // kz0 = bx * B ...
 __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2 *tw,
-                                         const float *__restrict__ green1d, int M, int B, int axis,
+                                         const float *__restrict__ green1d, int M, uint32_t plan, int B, int axis,
                                          int sign, int green, int bx, int by) {
     extern __shared__ float2 sm[];
     const int pitch = B;
@@ -609,8 +766,8 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
     const int kz0 = bx * B;
     const int bsh = ilog2(B);  // B is a power of two
     const int nb = min(B, Mh - kz0);
-    const size_t sm_stride = axis == 1 ? (size_t)Mh : (size_t)M * Mh;
-    const size_t base = axis == 1 ? (size_t)o * M * Mh : (size_t)o * Mh;
+    const size_t sm_stride = axis == 1 ? (size_t)spec_stride(M) : (size_t)M * spec_stride(M);
+    const size_t base = (size_t)o * (axis == 1 ? M : 1) * spec_stride(M);
     load_twiddles(tw_s, tw, M);
     for (int e0 = threadIdx.x; e0 < M * B; e0 += kLoadBatch * blockDim.x) {
         float2 v[kLoadBatch];
@@ -627,7 +784,8 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
         }
     }
     __syncthreads();
-    float2 *res = fft_columns(x, y, tw_s, M, bsh, pitch, sign);
+    float2 *res = sign < 0 ? fft_columns<-1>(x, y, tw_s, M, plan, bsh, pitch)
+                           : fft_columns<+1>(x, y, tw_s, M, plan, bsh, pitch);
     if (green) {
         // res holds the full forward transform: k index m along x, y index o, kz0+b
         const int ky = o <= M / 2 ? o : M - o;
@@ -646,7 +804,7 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
         }
         __syncthreads();
         float2 *other = res == x ? y : x;
-        res = fft_columns(res, other, tw_s, M, bsh, pitch, +1);
+        res = fft_columns<+1>(res, other, tw_s, M, plan, bsh, pitch);
     }
     for (int e = threadIdx.x; e < M * B; e += blockDim.x) {
         const int m = e >> bsh, b = e & (B - 1);
@@ -656,19 +814,19 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
 
 __global__ void __launch_bounds__(kFFTThreads)
     k_fft_z_r2c(unsigned long long *__restrict__ rho64, float mscale, float2 *__restrict__ spec,
-                const float2 *tw, int M, int P) {
-    fft_z_r2c(rho64, mscale, spec, tw, M, P, blockIdx.x);
+                const float2 *tw, int M, uint32_t plan, int P) {
+    fft_z_r2c(rho64, mscale, spec, tw, M, plan, P, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kFFTThreads)
-    k_fft_z_c2r(const float2 *__restrict__ spec, float *__restrict__ out, const float2 *tw, int M, int P) {
-    fft_z_c2r(spec, out, tw, M, P, blockIdx.x);
+    k_fft_z_c2r(const float2 *__restrict__ spec, float *__restrict__ out, const float2 *tw, int M, uint32_t plan, int P) {
+    fft_z_c2r(spec, out, tw, M, plan, P, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kFFTThreads)
-    k_fft_axis(float2 *__restrict__ spec, const float2 *tw, const float *__restrict__ green1d, int M, int B,
-               int axis, int sign, int green) {
-    fft_axis(spec, tw, green1d, M, B, axis, sign, green, blockIdx.x, blockIdx.y);
+    k_fft_axis(float2 *__restrict__ spec, const float2 *tw, const float *__restrict__ green1d, int M,
+               uint32_t plan, int B, int axis, int sign, int green) {
+    fft_axis(spec, tw, green1d, M, plan, B, axis, sign, green, blockIdx.x, blockIdx.y);
 }
 
 // fft_axis_reg for one box, with the batch B a compile-time constant
@@ -685,12 +843,12 @@ __device__ __forceinline__ void fft_axis_reg_fixed(float2 *__restrict__ spec, co
     constexpr int bsh = ilog2(B), rs = kFFTThreads / B, per = M * B / kFFTThreads;
     static_assert(kFFTThreads % B == 0 && (M * B) % kFFTThreads == 0, "batch layout");
     extern __shared__ float2 sm[];
-    float2 *x = sm, *tw_s = sm + M * B;
+    float2 *x = sm, *tw_s = sm + FT::ROWS * B;
     const int o = by, kz0 = bx * B, nb = min(B, Mh - kz0);
     const int b = threadIdx.x & (B - 1), r0 = threadIdx.x >> bsh;
     const bool valid = b < nb;
-    const size_t sm_stride = axis == 1 ? (size_t)Mh : (size_t)M * Mh;
-    float2 *col = spec + (axis == 1 ? (size_t)o * M * Mh : (size_t)o * Mh) + kz0 + b;
+    const size_t sm_stride = axis == 1 ? (size_t)spec_stride(M) : (size_t)M * spec_stride(M);
+    float2 *col = spec + (size_t)o * (axis == 1 ? M : 1) * spec_stride(M) + kz0 + b;
     // an inverse-only pass starts from the slot order
     const bool to_slots = sign > 0;
     load_twiddles(tw_s, tw, M);
@@ -704,39 +862,16 @@ __device__ __forceinline__ void fft_axis_reg_fixed(float2 *__restrict__ spec, co
         for (int u = 0; u < kLoadBatch; ++u)
             if (j0 + u < per) {
                 const int m = r0 + (j0 + u) * rs;
-                x[(to_slots ? FT::slot(m) : m) * B + b] = v[u];
+                x[FT::at(to_slots ? FT::slot(m) : m, B) + b] = v[u];
             }
     }
     __syncthreads();
     bool natural = true;
-    if (sign < 0) {
+    if (sign < 0 && green) {
+        FT::filter(x, tw_s, B, bsh, GreenColumn(green1d, M, o, kz0 + b, valid));
+    } else if (sign < 0) {
         FT::template forward<-1>(x, tw_s, B, bsh);
         natural = false;
-        if (green) {
-            // slot s = M2 k1 + k2 holds X[k1 + M1 k2]
-            const int ky = o <= M / 2 ? o : M - o;
-            const float gy = green1d[ky];
-            const int kz = kz0 + b;
-            const float gz = valid ? green1d[kz] : 0.f;
-            const int c = ky * ky + kz * kz;
-#pragma unroll 4
-            for (int j = 0; j < per; ++j) {
-                const int sl = r0 + j * rs;
-                const int k1 = sl / FT::N2, k2 = sl - k1 * FT::N2;
-                const int m = k1 + FT::N1 * k2;  // the transform index along x
-                const int kx = m <= M / 2 ? m : M - m;
-                const float2 v = x[sl * B + b];
-                float g = 0.f;
-                if (valid) {
-                    const int k2s = kx * kx + c;
-                    if (k2s > 0) g = -green1d[kx] * gy * gz * __frcp_rn((float)k2s);
-                }
-                x[sl * B + b] = make_float2(v.x * g, v.y * g);
-            }
-            __syncthreads();
-            FT::template inverse<+1>(x, tw_s, B, bsh);
-            natural = true;
-        }
     } else {
         FT::template inverse<+1>(x, tw_s, B, bsh);
     }
@@ -744,22 +879,30 @@ __device__ __forceinline__ void fft_axis_reg_fixed(float2 *__restrict__ spec, co
 #pragma unroll 4
         for (int j = 0; j < per; ++j) {
             const int m = r0 + j * rs;
-            col[(size_t)m * sm_stride] = x[(natural ? m : FT::slot(m)) * B + b];
+            col[(size_t)m * sm_stride] = x[FT::at(natural ? m : FT::slot(m), B) + b];
         }
     }
 }
 
 // One box, power-of-two mesh M = M1 * M2: the register transforms, one
 // instantiation per split (its registers sized for its DFT lengths).
+// The z passes' CTAs are as many threads as the batch's transforms take (P = 8
+// pairs; 4 at M = 1024), which leaves none idle and more CTAs an SM.
+constexpr int kMaxP = 8;
+__host__ __device__ constexpr int z_threads(int M1, int M2) {
+    const int T = M1 > M2 ? M1 : M2, P = M1 * M2 == 1024 ? 4 : kMaxP;
+    return T * P < 128 ? 128 : T * P;
+}
+
 template <int M1, int M2>
-__global__ void __launch_bounds__(kFFTThreads, M1 * M2 >= 512 ? 2 : 4)
+__global__ void __launch_bounds__(z_threads(M1, M2), M1 * M2 == 1024 ? 4 : M1 * M2 == 512 ? 2 : 6)
     k_fft_z_r2c_r(unsigned long long *__restrict__ rho64, float mscale, float2 *__restrict__ spec,
                   const float2 *tw, int P) {
     fft_z_r2c_reg<RegFFT<M1, M2>>(rho64, mscale, spec, tw, P, blockIdx.x);
 }
 
 template <int M1, int M2>
-__global__ void __launch_bounds__(kFFTThreads, M1 * M2 >= 512 ? 2 : 4)
+__global__ void __launch_bounds__(z_threads(M1, M2), M1 * M2 == 1024 ? 4 : M1 * M2 == 512 ? 2 : 6)
     k_fft_z_c2r_r(const float2 *__restrict__ spec, float *__restrict__ out, const float2 *tw, int P) {
     fft_z_c2r_reg<RegFFT<M1, M2>>(spec, out, tw, P, blockIdx.x);
 }
@@ -779,10 +922,9 @@ __global__ void __launch_bounds__(kFFTThreads, M1 * M2 >= 512 ? 2 : 4)
 template <int M1, int M2>
 cudaError_t fft_passes_reg(const PMPlan &plan, int P, cudaStream_t stream) {
     constexpr int M = M1 * M2, Mh = M / 2 + 1, B = axis_batch(M);
-    // z passes: the transform buffer, the twiddles and the block of 2P
-    // spectrum rows; axis passes: the buffer and the twiddles
-    const size_t smz = sizeof(float2) * ((size_t)M * (P + 1) + M + (size_t)2 * P * Mh),
-                 sma = sizeof(float2) * ((size_t)M * B + M);
+    // the transform buffer and the twiddles
+    constexpr int rows = RegFFT<M1, M2>::ROWS, zt = z_threads(M1, M2);
+    const size_t smz = sizeof(float2) * ((size_t)rows * (P + 1) + M), sma = sizeof(float2) * ((size_t)rows * B + M);
     static bool attr = [&] {
         cudaFuncSetAttribute(k_fft_z_r2c_r<M1, M2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         cudaFuncSetAttribute(k_fft_z_c2r_r<M1, M2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -791,13 +933,13 @@ cudaError_t fft_passes_reg(const PMPlan &plan, int P, cudaStream_t stream) {
     }();
     (void)attr;
     const unsigned zblocks = (unsigned)((size_t)M * M / (2 * P));
-    k_fft_z_r2c_r<M1, M2><<<zblocks, kFFTThreads, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
+    k_fft_z_r2c_r<M1, M2><<<zblocks, zt, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
                                                                  plan.twiddle, P);
     dim3 ag((Mh + B - 1) / B, M);
     k_fft_axis_r<M1, M2><<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, 1, -1, 0);
     k_fft_axis_r<M1, M2><<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, 0, -1, 1);
     k_fft_axis_r<M1, M2><<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, 1, +1, 0);
-    k_fft_z_c2r_r<M1, M2><<<zblocks, kFFTThreads, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, P);
+    k_fft_z_c2r_r<M1, M2><<<zblocks, zt, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, P);
     return cudaGetLastError();
 }
 
@@ -828,7 +970,7 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
             default: fft_z_r2c_reg<RegFFT<16, 16>>(d.rho64, d.mscale, d.spec, d.twiddle, d.P, m.y); break;
         }
     } else {
-        fft_z_r2c(d.rho64, d.mscale, d.spec, d.twiddle, d.M, d.P, m.y);
+        fft_z_r2c(d.rho64, d.mscale, d.spec, d.twiddle, d.M, d.stages, d.P, m.y);
     }
 }
 
@@ -852,7 +994,7 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
             default: fft_z_c2r_reg<RegFFT<16, 16>>(d.spec, d.rho, d.twiddle, d.P, m.y); break;
         }
     } else {
-        fft_z_c2r(d.spec, d.rho, d.twiddle, d.M, d.P, m.y);
+        fft_z_c2r(d.spec, d.rho, d.twiddle, d.M, d.stages, d.P, m.y);
     }
 }
 
@@ -879,7 +1021,7 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
             default: fft_axis_reg<RegFFT<16, 16>>(d.spec, d.twiddle, d.green1d, d.B, axis, sign, green, bx, by); break;
         }
     } else {
-        fft_axis(d.spec, d.twiddle, d.green1d, d.M, d.B, axis, sign, green, bx, by);
+        fft_axis(d.spec, d.twiddle, d.green1d, d.M, d.stages, d.B, axis, sign, green, bx, by);
     }
 }
 
@@ -1107,6 +1249,8 @@ bool pm_fft_batches_ok(int M, int P, int B) {
     return !pow2 || (reg_fft_ok(M, P) && reg_fft_ok(M, B));
 }
 
+size_t pm_spec_points(int M) { return (size_t)M * M * spec_stride(M); }
+uint32_t pm_stage_plan(int M) { return stage_plan(M); }
 int pm_batch_z(int M) { return fft_batch_z(M); }
 int pm_batch_axis(int M) { return fft_batch_axis(M); }
 
@@ -1198,6 +1342,7 @@ cuco_status_t pm_plan_create(PMPlan *plan, int M, float boxsize, float asmth, fl
         return CUCO_ERR_UNSUPPORTED;
     }
     plan->M = M;
+    plan->stages = stage_plan(M);
     plan->fixed = fixed;
     plan->boxsize = boxsize;
     plan->to_slab_fac = (float)M / boxsize;
@@ -1209,7 +1354,7 @@ cuco_status_t pm_plan_create(PMPlan *plan, int M, float boxsize, float asmth, fl
     CUCO_TRY_CUDA(cudaMalloc(&plan->rho, sizeof(float) * (size_t)M * M * M));
     CUCO_TRY_CUDA(cudaMalloc(&plan->rho64, sizeof(unsigned long long) * (size_t)M * M * M));
     plan->rho64_dirty = true;
-    CUCO_TRY_CUDA(cudaMalloc(&plan->spec, sizeof(float2) * (size_t)M * M * Mh));
+    CUCO_TRY_CUDA(cudaMalloc(&plan->spec, sizeof(float2) * pm_spec_points(M)));
     CUCO_TRY_CUDA(cudaMalloc(&plan->green1d, sizeof(float) * Mh));
     CUCO_TRY_CUDA(cudaMalloc(&plan->twiddle, sizeof(float2) * M));
     std::vector<float> g(Mh);
@@ -1269,7 +1414,7 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, uint32_t n, float4 *acc
     const int M = plan.M, Mh = M / 2 + 1;
     // at most 8 row pairs per z-pass CTA: half the shared memory of 16, so
     // more CTAs fit beside the sort's (9 us faster per force at M = 256)
-    const int P = std::min(fft_batch_z(M), 8), B = fft_batch_axis(M);
+    const int P = std::min(fft_batch_z(M), kMaxP), B = fft_batch_axis(M);
     const size_t smz = sizeof(float2) * (2 * (size_t)M * (P + 1) + M);
     const size_t sma = sizeof(float2) * (2 * (size_t)M * B + M);
     // The z r2c pass clears the sums it reads, so the grid is zero again when
@@ -1301,12 +1446,12 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, uint32_t n, float4 *acc
     } else {
         const unsigned zblocks = (unsigned)((size_t)M * M / (2 * P));
         k_fft_z_r2c<<<zblocks, kFFTThreads, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
-                                                           plan.twiddle, M, P);
+                                                           plan.twiddle, M, plan.stages, P);
         dim3 ag((Mh + B - 1) / B, M);
-        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, B, 1, -1, 0);
-        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, B, 0, -1, 1);
-        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, B, 1, +1, 0);
-        k_fft_z_c2r<<<zblocks, kFFTThreads, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, M, P);
+        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, -1, 0);
+        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 0, -1, 1);
+        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, +1, 0);
+        k_fft_z_c2r<<<zblocks, kFFTThreads, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, M, plan.stages, P);
         CUCO_TRY_CUDA(cudaGetLastError());
     }
     plan.rho64_dirty = false;
