@@ -176,7 +176,7 @@ struct SRWork {
     uint2 *units;
     uint32_t cap;
     uint32_t *ctl;  // kSRCtlWords: [0] dense slices listed, [1] next unit, [2] other units listed
-                    // (reset per launch), [3] timeout word (kept until read), [4] spare
+                    // (reset per launch), [3] timeout word (kept until read), [4], [5] spare
 };
 uint32_t shortrange_unit_cap(uint32_t n, uint64_t segments);
 constexpr int kSRCtlWords = 8;
@@ -241,8 +241,9 @@ bool pm_mesh_supported(int M);
 cuco_status_t pm_plan_create(PMPlan *plan, int M, float boxsize, float asmth, float mass,
                              double G, bool fixed = false);
 void pm_plan_destroy(PMPlan *plan);
-// Long-range acceleration of n positions (any order) into acc (same order).
-cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, uint32_t n, float4 *acc,
+// Long-range acceleration of n positions (any order) into acc, in the same
+// order or, with perm, of position i into acc[perm[i]].
+cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, const uint32_t *perm, uint32_t n, float4 *acc,
                         cudaStream_t stream, cudaEvent_t *ev_deposit_done,
                         cudaEvent_t *ev_fft_done, int *launches);
 

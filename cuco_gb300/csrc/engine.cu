@@ -101,14 +101,20 @@ __global__ void k_to_fixed(const float *__restrict__ a, float4 *__restrict__ b, 
     b[i] = make_float4(__uint_as_float(c[0]), __uint_as_float(c[1]), __uint_as_float(c[2]), 0.f);
 }
 
-// fixed point -> float positions in [0, L)
-__global__ void k_from_fixed(const float4 *__restrict__ b, float *__restrict__ a, uint32_t n, double length_per_unit) {
+// fixed point -> float positions in [0, L].  The product u * L / 2^32 in two
+// float parts of u, the upper 24 bits fused with the rounded lower 8 bits'
+// part: one rounding to 24 bits of a sum that is off by 2^-40 of the result at
+// most (a double product, which this replaces, ran at the FP64 rate: 512^3
+// 2.14 ms, now bound by memory).
+__global__ void k_from_fixed(const float4 *__restrict__ b, float *__restrict__ a, uint32_t n, float length_per_unit) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 v = b[i];
-    a[3 * i + 0] = (float)((double)__float_as_uint(v.x) * length_per_unit);
-    a[3 * i + 1] = (float)((double)__float_as_uint(v.y) * length_per_unit);
-    a[3 * i + 2] = (float)((double)__float_as_uint(v.z) * length_per_unit);
+    const uint32_t u[3] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z)};
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        a[3 * (size_t)i + d] = __fmaf_rn((float)(u[d] >> 8), 256.0f * length_per_unit,
+                                         __fmul_rn((float)(u[d] & 255u), length_per_unit));
 }
 
 __global__ void k_scatter4(const float4 *__restrict__ src_sorted, const uint32_t *__restrict__ perm,
@@ -261,7 +267,7 @@ cuco_status_t to_fixed(const float *a, float4 *b, uint32_t n, float boxsize, cud
 
 cuco_status_t from_fixed(const float4 *b, float *a, uint32_t n, float boxsize, cudaStream_t stream) {
     if (!n) return CUCO_OK;
-    k_from_fixed<<<(n + 255) / 256, 256, 0, stream>>>(b, a, n, (double)boxsize / 4294967296.0);
+    k_from_fixed<<<(n + 255) / 256, 256, 0, stream>>>(b, a, n, ldexpf(boxsize, -32));
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
@@ -299,7 +305,7 @@ void shortrange_table(float *t) {
 
 using namespace cuco;
 
-constexpr int kPhaseEvents = 10;
+constexpr int kPhaseEvents = 11;
 
 struct cuco_box {
     cuco_config_t cfg;
@@ -327,13 +333,15 @@ struct cuco_box {
     float *stage3 = nullptr;  // n x 3 staging for host/device float3 transfers
     PMPlan pm{};
     bool has_state = false;
+    bool scattered = false;  // consecutive particles of the uploaded state are mostly far apart
     bool timing = false;
     bool count_pairs = false;
     // phase events, two sets: a step records into ev[ev_cur] and the set of
     // the step before is read then, so timing never waits on the step just
     // enqueued.  0 start, 1 positions and keys done (the PM fork), 2 sort
     // done, 3 cell order done, 4/5/6 deposit/FFT/interpolation done (PM
-    // stream), 8 short range starts (after the join), 7 end.
+    // stream), 8 short range starts (after the join), 7 end, 10 the PM's start
+    // (PM stream).
     cudaEvent_t ev[2][kPhaseEvents] = {};
     int ev_cur = 0;
     bool ev_pending = false;  // ev[ev_cur ^ 1] holds a recorded step not yet read
@@ -397,6 +405,15 @@ void record(cuco_box *b, int i, cudaStream_t s = nullptr) {
 // compare them).
 constexpr uint32_t kSplitMinParticles = 1u << 20;
 
+// Sizes from which the PM of scattered particles waits for the cell order.
+constexpr uint32_t kScatteredMinParticles = 512000;
+constexpr int kScatteredMinMesh = 160;
+// Mesh from which the transforms' CTAs (128 registers a thread) do not fit
+// beside three short-range CTAs, and the split launch only costs: 256^3 9.11
+// -> 9.14 ms a step, 512^3 71.2 -> 71.7 (128^3 clustered 2.16 -> 2.06 ms with
+// it, at z = 49 1.10 -> 1.09).
+constexpr int kSplitMaxMesh = 512;
+
 uint32_t split_min_particles() {
     const char *env = getenv("CUCO_SPLIT_MIN_PARTICLES");
     if (!env || !*env) return kSplitMinParticles;
@@ -414,18 +431,31 @@ cuco_status_t join_pm(cuco_box *b) {
 
 // keys must already be in b->keys; runs sort, reorder, PM, short range (+kick)
 cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kick) {
-    // The PM reads the positions in original order and writes its
-    // accelerations in original order (its results do not depend on the
-    // order: integer deposit sums, one interpolation per particle), so it
-    // needs nothing from the sort and runs beside it.
-    if (pm) {
+    // The PM's results do not depend on the particles' order (integer deposit
+    // sums, one interpolation per particle).  It reads the positions in
+    // original order, needs nothing from the sort and runs beside it.  Where
+    // that order scatters many particles over a large mesh it reads them in
+    // cell order, after the sort: the deposit's atomics and the
+    // interpolation's 72 loads a particle then stay in a few sectors.  Random
+    // order, PM alone, beside the sort against after it: 192^3 particles on
+    // 384^3 4.37 -> 2.12 ms, 100^3 on 200^3 0.47 -> 0.41, 80^3 on 160^3 0.27
+    // -> 0.26, but 64^3 on 128^3 0.137 -> 0.152; lattice order, early or
+    // clustered, is 2 to 8 % faster beside the sort at every size.
+    const bool cell_ordered_pm = pm && b->scattered && b->n >= kScatteredMinParticles && b->M >= kScatteredMinMesh;
+    auto fork_pm = [&](const float4 *pos, const uint32_t *perm) -> cuco_status_t {
         CUCO_TRY_CUDA(cudaEventRecord(b->fork, b->stream));
         CUCO_TRY_CUDA(cudaStreamWaitEvent(b->pm_stream, b->fork, 0));
-        CUCO_TRY(pm_forces(b->pm, b->pos, b->n, b->acc_pm, b->pm_stream,
+        record(b, 10, b->pm_stream);
+        CUCO_TRY(pm_forces(b->pm, pos, perm, b->n, b->acc_pm, b->pm_stream,
                            b->timing ? &b->ev[b->ev_cur][4] : nullptr, b->timing ? &b->ev[b->ev_cur][5] : nullptr,
                            &b->launches));
         record(b, 6, b->pm_stream);
-    } else {
+        return CUCO_OK;
+    };
+    if (pm && !cell_ordered_pm) {
+        CUCO_TRY(fork_pm(b->pos, nullptr));
+    } else if (!pm) {
+        record(b, 10);
         record(b, 4);
         record(b, 5);
         record(b, 6);
@@ -448,6 +478,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
                                  nullptr, 1, b->cfg.mode == CUCO_MODE_FIXED, b->stream));
     b->launches += 2;
     record(b, 3);
+    if (cell_ordered_pm) CUCO_TRY(fork_pm(b->spos, perm_s));
     // The short range needs nothing from the PM: in a large box it starts
     // when the cell order is ready, one CTA per SM short of a full persistent
     // grid, so the PM's remaining kernels keep running beside it; its last
@@ -455,7 +486,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     // left then, and the PM half of the kick follows once both are done.  A
     // small box's step is launch-bound: its short range waits for the PM and
     // applies both halves of the kick in its epilogue (fewer launches).
-    const bool split = pm && b->n >= b->split_min;
+    const bool split = pm && b->n >= b->split_min && b->M < kSplitMaxMesh;
     if (pm && !split) CUCO_TRY(join_pm(b));
     record(b, 8);
     const bool kick_on = kick && kick->vel;
@@ -492,7 +523,7 @@ cuco_status_t read_pending(cuco_box *b) {
     // overlap the sort, the cell order and the start of the short range); the
     // short range from the cell order to the end of both parts of its launch;
     // the whole pass
-    static const int from[8] = {0, 1, 2, 1, 4, 5, 8, 0}, to[8] = {1, 2, 3, 4, 5, 6, 9, 7};
+    static const int from[8] = {0, 1, 2, 10, 4, 5, 8, 0}, to[8] = {1, 2, 3, 4, 5, 6, 9, 7};
     for (int i = 0; i < 8; ++i) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e[from[i]], e[to[i]]);
@@ -654,38 +685,64 @@ cuco_status_t cuco_box_destroy(cuco_box_t *b) {
 }  // extern "C"
 
 namespace state_check {
-__global__ void k_count_nonfinite(const float *__restrict__ v, size_t n, uint32_t *__restrict__ count) {
-    uint32_t bad = 0;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        bad += !isfinite(v[i]);
+// counts[0]: components that are not finite; counts[1] (far > 0): components
+// further than `far` from the particle's before, the periodic image aside
+__global__ void k_check_triplets(const float *__restrict__ v, size_t n3, float far, float boxsize,
+                                 uint32_t *__restrict__ counts) {
+    uint32_t bad = 0, apart = 0;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n3; e += (size_t)gridDim.x * blockDim.x) {
+        const float x = v[e];
+        bad += !isfinite(x);
+        if (far > 0.f && e >= 3) {
+            const float s = fabsf(x - v[e - 3]);
+            apart += s > far && boxsize - s > far;
+        }
+    }
     bad = __reduce_add_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0 && bad) atomicAdd(count, bad);
+    apart = __reduce_add_sync(0xffffffffu, apart);
+    if ((threadIdx.x & 31) == 0) {
+        if (bad) atomicAdd(&counts[0], bad);
+        if (apart) atomicAdd(&counts[1], apart);
+    }
 }
 
-// The staged triplets (b->stage3) must all be finite: a state with a NaN or
-// an infinity is refused before it reaches the box (CUCO_ERR_INVALID).
-cuco_status_t check_finite(cuco_box_t *b, const char *what) {
-    uint32_t *count = b->work.ctl + 4;  // the plan's spare control word
-    CUCO_TRY_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), b->stream));
-    const size_t n = 3 * (size_t)b->n;
-    if (n) {
-        const unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 4096);
-        k_count_nonfinite<<<blocks, 256, 0, b->stream>>>(b->stage3, n, count);
+// Counts for n triplets into counts (zeroed here): pos says whether they are
+// positions, whose order is looked at too.
+cuco_status_t count_triplets(cuco_box_t *b, const float *v, bool pos, uint32_t *counts) {
+    CUCO_TRY_CUDA(cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), b->stream));
+    const size_t n3 = 3 * (size_t)b->n;
+    if (n3) {
+        const unsigned blocks = (unsigned)std::min<size_t>((n3 + 255) / 256, 4096);
+        k_check_triplets<<<blocks, 256, 0, b->stream>>>(v, n3, pos ? 8.f * b->cfg.boxsize / b->M : 0.f,
+                                                        b->cfg.boxsize, counts);
         CUCO_TRY_CUDA(cudaGetLastError());
     }
-    uint32_t bad = 0;
-    CUCO_TRY_CUDA(cudaMemcpyAsync(&bad, count, sizeof bad, cudaMemcpyDeviceToHost, b->stream));
+    return CUCO_OK;
+}
+
+// The triplets counted must all be finite: a state with a NaN or an infinity
+// is refused before it reaches the box (CUCO_ERR_INVALID).  pos/vel: whether
+// the first/second pair of counts (work.ctl + 4) was taken.  Positions also
+// say whether their order scatters them: half of their components further
+// than eight PM cells from the particle's before (a lattice's order, early or
+// late in a clustered run, leaves a few per cent there; random order most).
+cuco_status_t read_counts(cuco_box_t *b, bool pos, bool vel) {
+    uint32_t got[4] = {0, 0, 0, 0};
+    CUCO_TRY_CUDA(cudaMemcpyAsync(got, b->work.ctl + 4, sizeof got, cudaMemcpyDeviceToHost, b->stream));
     CUCO_TRY_CUDA(cudaStreamSynchronize(b->stream));
-    if (bad) {
-        set_error(std::string("cuco_box_set_state: ") + std::to_string(bad) + " " + what +
-                  " components are not finite");
-        return CUCO_ERR_INVALID;
-    }
+    for (int k = 0; k < 2; ++k)
+        if ((k ? vel : pos) && got[2 * k]) {
+            set_error(std::string("cuco_box_set_state: ") + std::to_string(got[2 * k]) +
+                      (k ? " velocity" : " position") + " components are not finite");
+            return CUCO_ERR_INVALID;
+        }
+    if (pos) b->scattered = 2 * (uint64_t)got[1] > 3 * (uint64_t)b->n;
     return CUCO_OK;
 }
 }  // namespace state_check
 
-using state_check::check_finite;
+using state_check::count_triplets;
+using state_check::read_counts;
 
 extern "C" {
 
@@ -695,17 +752,33 @@ cuco_status_t cuco_box_set_state(cuco_box_t *b, const float *pos, const float *v
         return CUCO_ERR_INVALID;
     }
     const size_t bytes = sizeof(float) * 3 * b->n;
-    cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, pos, bytes, kind, b->stream));
-    CUCO_TRY(check_finite(b, "position"));
-    if (b->cfg.mode == CUCO_MODE_FIXED)
-        CUCO_TRY(to_fixed(b->stage3, b->pos, b->n, b->cfg.boxsize, b->stream));
-    else
-        CUCO_TRY(pack3to4(b->stage3, b->pos, b->n, b->stream));
-    if (vel) {
-        CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, vel, bytes, kind, b->stream));
-        CUCO_TRY(check_finite(b, "velocity"));
-        CUCO_TRY(pack3to4(b->stage3, b->vel, b->n, b->stream));
+    uint32_t *counts = b->work.ctl + 4;  // the plan's spare control words
+    auto put = [&](const float *p, const float *v) -> cuco_status_t {
+        if (p && b->cfg.mode == CUCO_MODE_FIXED)
+            CUCO_TRY(to_fixed(p, b->pos, b->n, b->cfg.boxsize, b->stream));
+        else if (p)
+            CUCO_TRY(pack3to4(p, b->pos, b->n, b->stream));
+        return v ? pack3to4(v, b->vel, b->n, b->stream) : CUCO_OK;
+    };
+    if (on_device) {
+        // the caller's arrays are checked and read in place (no staging
+        // copies: 512^3 set 6.9 -> 4.9 ms), and read to the end on return
+        CUCO_TRY(count_triplets(b, pos, true, counts));
+        if (vel) CUCO_TRY(count_triplets(b, vel, false, counts + 2));
+        CUCO_TRY(read_counts(b, true, vel != nullptr));
+        CUCO_TRY(put(pos, vel));
+        CUCO_TRY_CUDA(cudaStreamSynchronize(b->stream));
+    } else {
+        CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, pos, bytes, cudaMemcpyHostToDevice, b->stream));
+        CUCO_TRY(count_triplets(b, b->stage3, true, counts));
+        CUCO_TRY(read_counts(b, true, false));
+        CUCO_TRY(put(b->stage3, nullptr));
+        if (vel) {
+            CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, vel, bytes, cudaMemcpyHostToDevice, b->stream));
+            CUCO_TRY(count_triplets(b, b->stage3, false, counts + 2));
+            CUCO_TRY(read_counts(b, false, true));
+            CUCO_TRY(put(nullptr, b->stage3));
+        }
     }
     b->has_state = true;
     return CUCO_OK;
@@ -718,19 +791,18 @@ cuco_status_t cuco_box_get_state(cuco_box_t *b, float *pos, float *vel, float *a
         return CUCO_ERR_INVALID;
     }
     const size_t bytes = sizeof(float) * 3 * b->n;
-    cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     float *dst[4] = {pos, vel, acc_pp, acc_pm};
     float4 *src[4] = {b->pos, b->vel, b->acc_pp, b->acc_pm};
     for (int k = 0; k < 4; ++k) {
         if (!dst[k]) continue;
+        float *out = on_device ? dst[k] : b->stage3;
         if (k == 0 && b->cfg.mode == CUCO_MODE_FIXED)
-            CUCO_TRY(from_fixed(src[k], b->stage3, b->n, b->cfg.boxsize, b->stream));
+            CUCO_TRY(from_fixed(src[k], out, b->n, b->cfg.boxsize, b->stream));
         else
-            CUCO_TRY(unpack4to3(src[k], b->stage3, b->n, b->stream));
-        CUCO_TRY_CUDA(cudaMemcpyAsync(dst[k], b->stage3, bytes, kind, b->stream));
+            CUCO_TRY(unpack4to3(src[k], out, b->n, b->stream));
+        if (!on_device) CUCO_TRY_CUDA(cudaMemcpyAsync(dst[k], out, bytes, cudaMemcpyDeviceToHost, b->stream));
     }
-    CUCO_TRY_CUDA(cudaStreamSynchronize(b->stream));
-    return shortrange_check(b->work.ctl, b->stream);
+    return shortrange_check(b->work.ctl, b->stream);  // waits for the stream
 }
 
 cuco_status_t cuco_box_set_state_fixed(cuco_box_t *b, const uint32_t *pos, const float *vel, int on_device) {
@@ -743,9 +815,11 @@ cuco_status_t cuco_box_set_state_fixed(cuco_box_t *b, const uint32_t *pos, const
     // the uint32 triplets move as bit patterns: pack3to4 only copies words
     CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, pos, bytes, kind, b->stream));
     CUCO_TRY(pack3to4(b->stage3, b->pos, b->n, b->stream));
+    b->scattered = false;  // not known
     if (vel) {
         CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, vel, bytes, kind, b->stream));
-        CUCO_TRY(check_finite(b, "velocity"));
+        CUCO_TRY(count_triplets(b, b->stage3, false, b->work.ctl + 6));
+        CUCO_TRY(read_counts(b, false, true));
         CUCO_TRY(pack3to4(b->stage3, b->vel, b->n, b->stream));
     }
     b->has_state = true;
@@ -844,8 +918,7 @@ cuco_status_t cuco_box_selftest_timeout(cuco_box_t *b, double seconds) {
 
 cuco_status_t cuco_box_sync(cuco_box_t *b) {
     if (!b) return CUCO_ERR_INVALID;
-    CUCO_TRY_CUDA(cudaStreamSynchronize(b->stream));
-    return shortrange_check(b->work.ctl, b->stream);
+    return shortrange_check(b->work.ctl, b->stream);  // waits for the stream
 }
 
 cuco_status_t cuco_box_stream(cuco_box_t *b, void **stream) {
@@ -1007,6 +1080,7 @@ __attribute__((visibility("hidden"))) cuco_status_t cuco_box_internal_arrays(
 
 __attribute__((visibility("hidden"))) cuco_status_t cuco_box_mark_state(cuco_box_t *b) {
     b->has_state = true;
+    b->scattered = false;  // not known
     return CUCO_OK;
 }
 

@@ -1188,11 +1188,13 @@ __global__ void k_deposit(const float4 *__restrict__ pos, uint32_t n, unsigned l
     if (i < n) deposit_one<FIXED>(pos[i], rho64, M, to_slab_fac);
 }
 
+// perm (or null): where each result goes, for positions in cell order
 template <bool FIXED>
-__global__ void k_interp(const float4 *__restrict__ pos, uint32_t n, const float *__restrict__ phi,
-                         int M, float to_slab_fac, float fac, float4 *__restrict__ acc) {
+__global__ void k_interp(const float4 *__restrict__ pos, const uint32_t *__restrict__ perm, uint32_t n,
+                         const float *__restrict__ phi, int M, float to_slab_fac, float fac,
+                         float4 *__restrict__ acc) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) acc[i] = interp_one<FIXED>(pos[i], phi, M, to_slab_fac, fac);
+    if (i < n) acc[perm ? perm[i] : i] = interp_one<FIXED>(pos[i], phi, M, to_slab_fac, fac);
 }
 
 template <bool FIXED>
@@ -1408,7 +1410,7 @@ void pm_plan_destroy(PMPlan *plan) {
     plan->spec = nullptr;
 }
 
-cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, uint32_t n, float4 *acc,
+cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, const uint32_t *perm, uint32_t n, float4 *acc,
                         cudaStream_t stream, cudaEvent_t *ev_deposit_done, cudaEvent_t *ev_fft_done,
                         int *launches) {
     const int M = plan.M, Mh = M / 2 + 1;
@@ -1458,9 +1460,9 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, uint32_t n, float4 *acc
     if (ev_fft_done) CUCO_TRY_CUDA(cudaEventRecord(*ev_fft_done, stream));
     if (n) {
         if (plan.fixed)
-            k_interp<true><<<(n + 255) / 256, 256, 0, stream>>>(pos, n, plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc);
+            k_interp<true><<<(n + 255) / 256, 256, 0, stream>>>(pos, perm, n, plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc);
         else
-            k_interp<false><<<(n + 255) / 256, 256, 0, stream>>>(pos, n, plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc);
+            k_interp<false><<<(n + 255) / 256, 256, 0, stream>>>(pos, perm, n, plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc);
     }
     CUCO_TRY_CUDA(cudaGetLastError());
     if (launches) *launches += 5 + (n ? 2 : 0);  // five transform passes, deposit and interpolation
