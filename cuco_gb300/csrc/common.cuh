@@ -79,10 +79,13 @@ size_t sort_hist_entries(uint32_t n, int key_bits, int max_radix_bits);
 // be null: the values are then the input positions 0..n-1.  The sorted data
 // ends in (keys, vals) when `result_in_alt` comes back false, else in
 // (keys_alt, vals_alt).  max_radix_bits bounds the digit width (4..8).
+// offsets_done (or null): a sort that is one launch also writes cell_off (as
+// launch_reorder_offsets) and says so.
 cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in,
                          uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *hist, size_t hist_words,
                          uint32_t n, int key_bits, int max_radix_bits, cudaStream_t stream,
-                         bool *result_in_alt, int *launches);
+                         bool *result_in_alt, int *launches, uint32_t *cell_off = nullptr, uint32_t ncells = 0,
+                         bool *offsets_done = nullptr);
 
 // Cell keys of float4 positions (calcHashD rule); idx gets 0..n-1 when non-null.
 cuco_status_t launch_cell_keys(const float4 *pos, uint32_t *keys, uint32_t *idx, uint32_t n,
@@ -96,10 +99,8 @@ cuco_status_t launch_reorder_start_end(uint32_t *cell_start, uint32_t *cell_end,
                                        uint32_t ncells, cudaStream_t stream);
 
 // Engine cell-bound format: cell_off[c] = first sorted index with key >= c,
-// for c in [0, ncells], plus the gather (none when sorted_pos is null).
-cuco_status_t launch_reorder_offsets(uint32_t *cell_off, float4 *sorted_pos,
-                                     const uint32_t *sorted_keys, const uint32_t *perm,
-                                     const float4 *pos, uint32_t n, uint32_t ncells,
+// for c in [0, ncells].
+cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_keys, uint32_t n, uint32_t ncells,
                                      cudaStream_t stream);
 
 // The reference's cell bounds (cell_end is read where cell_start is not

@@ -442,8 +442,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     // -> 0.26, but 64^3 on 128^3 0.137 -> 0.152; lattice order, early or
     // clustered, is 2 to 8 % faster beside the sort at every size.
     const bool cell_ordered_pm = pm && b->scattered && b->n >= kScatteredMinParticles && b->M >= kScatteredMinMesh;
-    auto fork_pm = [&](const float4 *pos, const uint32_t *perm) -> cuco_status_t {
-        CUCO_TRY_CUDA(cudaEventRecord(b->fork, b->stream));
+    auto run_pm = [&](const float4 *pos, const uint32_t *perm) -> cuco_status_t {
         CUCO_TRY_CUDA(cudaStreamWaitEvent(b->pm_stream, b->fork, 0));
         record(b, 10, b->pm_stream);
         CUCO_TRY(pm_forces(b->pm, pos, perm, b->n, b->acc_pm, b->pm_stream,
@@ -452,22 +451,27 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
         record(b, 6, b->pm_stream);
         return CUCO_OK;
     };
-    if (pm && !cell_ordered_pm) {
-        CUCO_TRY(fork_pm(b->pos, nullptr));
-    } else if (!pm) {
+    if (pm && !cell_ordered_pm) CUCO_TRY_CUDA(cudaEventRecord(b->fork, b->stream));
+    if (!pm) {
         record(b, 10);
         record(b, 4);
         record(b, 5);
         record(b, 6);
     }
-    bool in_alt = false;
+    bool in_alt = false, offsets_done = false;
     CUCO_TRY(sort_pairs(b->keys, b->perm, nullptr, b->keys_alt, b->perm_alt, b->hist, b->hist_words,
-                        b->n, b->key_bits, 8, b->stream, &in_alt, &b->launches));
+                        b->n, b->key_bits, 8, b->stream, &in_alt, &b->launches, b->cell_off, b->ncells,
+                        &offsets_done));
+    record(b, 2);
+    // (the sort is handed over before the PM: a small box's step waits for the
+    // host, and the sort heads the longer chain)
+    if (pm && !cell_ordered_pm) CUCO_TRY(run_pm(b->pos, nullptr));
     b->sorted_keys = in_alt ? b->keys_alt : b->keys;
     b->sorted_perm = in_alt ? b->perm_alt : b->perm;
-    record(b, 2);
-    CUCO_TRY(launch_reorder_offsets(b->cell_off, nullptr, b->sorted_keys, b->sorted_perm, b->pos,
-                                    b->n, b->ncells, b->stream));
+    if (!offsets_done) {
+        CUCO_TRY(launch_reorder_offsets(b->cell_off, b->sorted_keys, b->n, b->ncells, b->stream));
+        b->launches += 1;
+    }
     // the cell order refined by z slice (the short range trims its column
     // ranges to the slices a target reaches); its map to original indices
     // goes to the sort's spare buffer
@@ -476,9 +480,12 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     const CellBox cb{(uint32_t)b->G, 0u, b->cfg.boxsize, b->gridfac};
     CUCO_TRY(launch_cell_subsort(b->cell_off, b->sorted_perm, b->pos, b->spos, perm_s, b->cell_sl, b->ncells, cb,
                                  nullptr, 1, b->cfg.mode == CUCO_MODE_FIXED, b->stream));
-    b->launches += 2;
+    b->launches += 1;
     record(b, 3);
-    if (cell_ordered_pm) CUCO_TRY(fork_pm(b->spos, perm_s));
+    if (cell_ordered_pm) {
+        CUCO_TRY_CUDA(cudaEventRecord(b->fork, b->stream));
+        CUCO_TRY(run_pm(b->spos, perm_s));
+    }
     // The short range needs nothing from the PM: in a large box it starts
     // when the cell order is ready, one CTA per SM short of a full persistent
     // grid, so the PM's remaining kernels keep running beside it; its last

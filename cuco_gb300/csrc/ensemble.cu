@@ -357,19 +357,22 @@ cuco_status_t ensemble_pass(cuco_ensemble *e, int do_drift, bool kick) {
     CUCO_TRY_CUDA(cudaStreamWaitEvent(e->pm_stream, e->fork, 0));
     CUCO_TRY(pm_forces_multi(e->pm, e->pos, e->n, e->acc_pm, e->pm_stream, &e->launches));
     CUCO_TRY_CUDA(cudaEventRecord(e->join, e->pm_stream));
-    bool in_alt = false;
+    bool in_alt = false, offsets_done = false;
     CUCO_TRY(sort_pairs(e->keys, e->perm, nullptr, e->keys_alt, e->perm_alt, e->hist, e->cap_hist, e->n,
-                        e->key_bits, 8, e->stream, &in_alt, &e->launches));
+                        e->key_bits, 8, e->stream, &in_alt, &e->launches, e->cell_off, (uint32_t)e->ncells,
+                        &offsets_done));
     const uint32_t *skeys = in_alt ? e->keys_alt : e->keys;
     e->sorted_perm = in_alt ? e->perm_alt : e->perm;
-    CUCO_TRY(launch_reorder_offsets(e->cell_off, nullptr, skeys, e->sorted_perm, e->pos, e->n, (uint32_t)e->ncells,
-                                    e->stream));
+    if (!offsets_done) {
+        CUCO_TRY(launch_reorder_offsets(e->cell_off, skeys, e->n, (uint32_t)e->ncells, e->stream));
+        e->launches++;
+    }
     // cells refined by z slice, as for one box; the map to original indices
     // goes to the sort's spare buffer
     uint32_t *perm_s = in_alt ? e->perm : e->perm_alt;
     CUCO_TRY(launch_cell_subsort(e->cell_off, e->sorted_perm, e->pos, e->spos, perm_s, e->cell_sl,
                                  (uint32_t)e->ncells, CellBox{}, e->d_drift, e->nbox, e->fixed, e->stream));
-    e->launches += 2;
+    e->launches += 1;
     CUCO_TRY_CUDA(cudaStreamWaitEvent(e->stream, e->join, 0));
     KickArgs k{};
     k.vel = kick ? e->vel : nullptr;

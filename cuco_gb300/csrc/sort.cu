@@ -26,7 +26,17 @@
 // where that would leave SMs without four tiles (sort_items).  Measured alone,
 // before and after, a pass over 4M pairs: histogram 27 -> 6, scan 5 -> 4,
 // scatter 33 -> 26 us; three passes over 32K pairs 93 -> 36 us.
+//
+// Up to kClusterMax keys take one launch instead: a cluster of eight CTAs holds
+// every key in shared memory, ranks each pass's digits, exchanges the digit
+// totals and scatters the pairs through distributed shared memory.  What
+// bounds such a sort is launches: 32K pairs of 18 bits were nine of them and
+// 36 us of kernels, and two copies back where the pass count is odd.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cuco {
 
@@ -127,11 +137,10 @@ __global__ void __launch_bounds__(kScanThreads) k_sort_scan(uint32_t *__restrict
     }
 }
 
-// SINGLE: one tile, whose own digit starts are the global ones.
 // The values are read when the ranks are known: held through the ranking they
 // took 88 registers, two CTAs an SM.  (At 16 keys a thread three CTAs without
 // spills beat four: 4 passes over 4M pairs 132 against 140 us.)
-template <int RB, int ITEMS, bool WITH_VALS, bool SINGLE>
+template <int RB, int ITEMS, bool WITH_VALS>
 __global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 3 : 4)
     k_sort_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint32_t *__restrict__ kout,
                    uint32_t *__restrict__ vout, uint32_t n, int shift, const uint32_t *__restrict__ hist,
@@ -162,7 +171,7 @@ __global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 3 : 4)
     }
     // this thread's digit: the prefix over the tiles up to this one, the total
     uint32_t gp = 0, gt = 0;
-    if (!SINGLE && tid < RADIX) {
+    if (tid < RADIX) {
         gp = hist[(size_t)tid * tiles + tile];
         gt = hist[(size_t)tid * tiles + tiles - 1];
     }
@@ -235,7 +244,7 @@ __global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 3 : 4)
         dstart[tid] = incl - v;
         // the digit's run from this tile starts after the lower digits'
         // totals and this digit's runs from earlier tiles
-        gofs[tid] = SINGLE ? 0u : (tincl - gt) + (gp - v) - (incl - v);
+        gofs[tid] = (tincl - gt) + (gp - v) - (incl - v);
     }
     __syncthreads();
 #pragma unroll
@@ -263,10 +272,8 @@ __global__ void __launch_bounds__(kSortThreads, ITEMS == 16 ? 3 : 4)
 
 // Keys per thread of a tile: the most that leave four tiles for each of ~150
 // SMs (2M pairs, three passes: 8 keys 70 us, 16 keys 83 us; at 4M they are
-// level), in a table of at most hist_words counts (16 always fits); up to
-// 4096 keys are one tile, which needs no histogram.
+// level), in a table of at most hist_words counts (16 always fits).
 int sort_items(uint32_t n, int rb, size_t hist_words) {
-    if (n <= 16u * kSortThreads) return 16;
     for (int items : {4, 8}) {
         const uint32_t next = kSortThreads * items * 2;
         const size_t tiles = (n + kSortThreads * items - 1) / (kSortThreads * items);
@@ -281,28 +288,13 @@ cuco_status_t sort_pass_items(const uint32_t *kin, const uint32_t *vin, uint32_t
                               bool with_vals, uint32_t *hist, uint32_t n, int shift, cudaStream_t stream,
                               int *launches) {
     const uint32_t tiles = (n + kSortThreads * ITEMS - 1) / (kSortThreads * ITEMS);
-    auto scatter = [&](auto kernel) {
-        kernel<<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, hist, tiles);
-        *launches += 1;
-    };
-    bool single = false;
-    if constexpr (ITEMS == 16) single = tiles == 1;
-    if (single) {
-        if constexpr (ITEMS == 16) {
-            if (with_vals)
-                scatter(k_sort_scatter<RB, ITEMS, true, true>);
-            else
-                scatter(k_sort_scatter<RB, ITEMS, false, true>);
-        }
-    } else {
-        k_sort_hist<RB, ITEMS><<<tiles, kSortThreads, 0, stream>>>(kin, n, shift, hist, tiles);
-        k_sort_scan<<<1u << RB, kScanThreads, 0, stream>>>(hist, tiles);
-        *launches += 2;
-        if (with_vals)
-            scatter(k_sort_scatter<RB, ITEMS, true, false>);
-        else
-            scatter(k_sort_scatter<RB, ITEMS, false, false>);
-    }
+    k_sort_hist<RB, ITEMS><<<tiles, kSortThreads, 0, stream>>>(kin, n, shift, hist, tiles);
+    k_sort_scan<<<1u << RB, kScanThreads, 0, stream>>>(hist, tiles);
+    if (with_vals)
+        k_sort_scatter<RB, ITEMS, true><<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, hist, tiles);
+    else
+        k_sort_scatter<RB, ITEMS, false><<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, hist, tiles);
+    *launches += 3;
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
@@ -315,6 +307,192 @@ cuco_status_t sort_pass(int items, const uint32_t *kin, const uint32_t *vin, uin
         case 8: return sort_pass_items<RB, 8>(kin, vin, kout, vout, with_vals, hist, n, shift, stream, launches);
         default: return sort_pass_items<RB, 16>(kin, vin, kout, vout, with_vals, hist, n, shift, stream, launches);
     }
+}
+
+// ---- the one-launch sort of up to kClusterMax keys
+constexpr int kClusterCtas = 8, kClusterThreads = 1024, kClusterWarps = kClusterThreads / 32;
+constexpr uint32_t kClusterMax = 8u * kClusterCtas * kClusterThreads;
+
+// Cells (prev, cur] start at sorted index i: a lane's few by itself, a long
+// gap by the whole warp.  Every lane of the warp calls it together (`has`: it
+// holds an index; prev + 1 = first for the first).
+__device__ __forceinline__ void fill_offsets(uint32_t *__restrict__ cell_off, bool has, uint32_t first, uint32_t cur,
+                                             uint32_t i) {
+    const bool is_long = has && cur >= first && cur - first >= 8u;
+    if (has && !is_long)
+        for (uint32_t c = first; c <= cur; ++c) cell_off[c] = i;
+    for (uint32_t rest = __ballot_sync(kFull, is_long); rest; rest &= rest - 1) {
+        const int src = __ffs(rest) - 1;
+        const uint32_t a = __shfl_sync(kFull, first, src), b = __shfl_sync(kFull, cur, src), v = __shfl_sync(kFull, i, src);
+        for (uint32_t c = a + (threadIdx.x & 31); c <= b; c += 32) cell_off[c] = v;
+    }
+}
+
+// Shared memory of a CTA: its pairs, the same staged in digit order (so that
+// the pairs a warp sends to another CTA are runs: single pairs sent as they
+// came took 10 us a pass), each warp's digit counts, the CTA's digit totals
+// (read by the others), each digit's first place in the stage and its offset
+// to the global order.
+template <int ITEMS>
+struct ClusterMem {
+    uint2 pair[kClusterThreads * ITEMS], stage[kClusterThreads * ITEMS];
+    uint16_t cnt[kClusterWarps][256];
+    uint32_t total[256], lstart[256], gofs[256], wsum[2][8];
+};
+
+// In place: (keys, vals) sorted by the low passes * rb bits, vals_in null: the
+// input positions; vals null: keys only.  cell_off (or null): also the cells'
+// first sorted indices, cell_off[c] for c in [0, ncells].
+template <int ITEMS>
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
+    k_sort_cluster(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in, uint32_t n, int passes, int rb,
+                   uint32_t *__restrict__ cell_off, uint32_t ncells) {
+    constexpr uint32_t E = kClusterThreads * ITEMS;  // keys of a CTA
+    extern __shared__ __align__(16) unsigned char cluster_smem[];
+    ClusterMem<ITEMS> &sm = *reinterpret_cast<ClusterMem<ITEMS> *>(cluster_smem);
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank();
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lt = (1u << lane) - 1u;
+    const uint32_t radix = 1u << rb;
+    // item k of this thread: CTA position `first + 32 k`, input order over
+    // (CTA, warp, item, lane)
+    const uint32_t first = warp * (32 * ITEMS) + lane, g0 = rank * E + first;
+    uint32_t key[ITEMS], val[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const uint32_t g = g0 + 32 * k;
+        key[k] = g < n ? keys[g] : 0xffffffffu;
+        val[k] = vals && vals_in && g < n ? vals_in[g] : g;
+    }
+    for (int p = 0; p < passes; ++p) {
+        const int shift = p * rb;
+        for (uint32_t d = lane; d < radix; d += 32) sm.cnt[warp][d] = 0;
+        __syncwarp();
+        uint32_t place[ITEMS];  // rank within the warp's keys of the digit
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const bool valid = g0 + 32 * k < n;
+            const uint32_t d = (key[k] >> shift) & (radix - 1);
+            uint32_t peers = __ballot_sync(kFull, valid);
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+                if (b < rb) {
+                    const uint32_t bit = (d >> b) & 1u;
+                    const uint32_t m = __ballot_sync(kFull, bit);
+                    peers &= bit ? m : ~m;
+                }
+            if (!valid) peers = 1u << lane;
+            const int lead = __ffs(peers) - 1;
+            uint32_t c = 0;
+            if (valid && lane == (uint32_t)lead) {
+                c = sm.cnt[warp][d];
+                sm.cnt[warp][d] = (uint16_t)(c + __popc(peers));
+            }
+            place[k] = __shfl_sync(kFull, c, lead) + __popc(peers & lt);
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t mine = 0;  // thread d: this CTA's keys of digit d
+        if (tid < radix) {
+#pragma unroll
+            for (int w0 = 0; w0 < kClusterWarps; w0 += 8) {
+                uint32_t c[8];
+#pragma unroll
+                for (int w = 0; w < 8; ++w) c[w] = sm.cnt[w0 + w][tid];
+#pragma unroll
+                for (int w = 0; w < 8; ++w) {
+                    sm.cnt[w0 + w][tid] = (uint16_t)mine;
+                    mine += c[w];
+                }
+            }
+            sm.total[tid] = mine;
+        }
+        cluster.sync();  // totals complete, and the last pass's pairs read
+        uint32_t all = 0, before = 0, incl = 0, lincl = mine;
+        if (tid < 256) {
+            if (tid < radix) {
+#pragma unroll
+                for (uint32_t c = 0; c < (uint32_t)kClusterCtas; ++c) {
+                    const uint32_t v = cluster.map_shared_rank(sm.total, c)[tid];
+                    all += v;
+                    if (c < rank) before += v;
+                }
+            }
+            incl = all;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, incl, off), ly = __shfl_up_sync(kFull, lincl, off);
+                if (lane >= (uint32_t)off) incl += y, lincl += ly;
+            }
+            if (lane == 31) sm.wsum[0][warp] = incl, sm.wsum[1][warp] = lincl;
+        }
+        __syncthreads();
+        if (tid < radix) {
+#pragma unroll
+            for (uint32_t w = 0; w < 8; ++w)
+                if (w < warp) incl += sm.wsum[0][w], lincl += sm.wsum[1][w];
+            sm.lstart[tid] = lincl - mine;
+            sm.gofs[tid] = (incl - all + before) - (lincl - mine);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            if (g0 + 32 * k < n) {
+                const uint32_t d = (key[k] >> shift) & (radix - 1);
+                sm.stage[CUCO_IDX(sm.lstart[d] + sm.cnt[warp][d] + place[k], E)] = make_uint2(key[k], val[k]);
+            }
+        }
+        __syncthreads();
+        const uint32_t held = n > rank * E ? min(n - rank * E, E) : 0u;
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint32_t j = k * kClusterThreads + tid;
+            if (j < held) {
+                const uint2 kv = sm.stage[j];
+                const uint32_t o = CUCO_IDX(sm.gofs[(kv.x >> shift) & (radix - 1)] + j, n);
+                cluster.map_shared_rank(sm.pair, o / E)[o & (E - 1)] = kv;
+            }
+        }
+        cluster.sync();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint2 kv = sm.pair[first + 32 * k];
+            key[k] = kv.x, val[k] = kv.y;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const uint32_t g = g0 + 32 * k;
+        if (g < n) {
+            keys[g] = key[k];
+            if (vals) vals[g] = val[k];
+        }
+    }
+    if (cell_off) {
+        // the key before a thread's item (the previous CTA's last for a CTA's
+        // first), and the cells past the last key
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const uint32_t e = first + 32 * k, g = g0 + 32 * k;
+            uint32_t from = 0;
+            if (g && g < n) from = 1u + (e ? sm.pair[e - 1].x : cluster.map_shared_rank(sm.pair, rank - 1)[E - 1].x);
+            fill_offsets(cell_off, g < n, from, key[k], g);
+            fill_offsets(cell_off, g == n - 1, key[k] + 1u, ncells, n);
+        }
+        cluster.sync();  // no CTA leaves while its keys may be read
+    }
+}
+
+template <int ITEMS>
+cuco_status_t launch_sort_cluster(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in, uint32_t n, int passes,
+                                  int rb, uint32_t *cell_off, uint32_t ncells, cudaStream_t stream) {
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterMem<ITEMS>));
+    CUCO_TRY_CUDA(attr);
+    k_sort_cluster<ITEMS><<<kClusterCtas, kClusterThreads, sizeof(ClusterMem<ITEMS>), stream>>>(
+        keys, vals, vals_in, n, passes, rb, cell_off, ncells);
+    CUCO_TRY_CUDA(cudaGetLastError());
+    return CUCO_OK;
 }
 
 void split_bits(int key_bits, int max_radix_bits, int *passes, int *rb) {
@@ -342,17 +520,13 @@ __global__ void k_reorder_start_end(uint32_t *__restrict__ cell_start, uint32_t 
     sorted_pos[i] = pos[perm[i]];
 }
 
-__global__ void k_reorder_offsets(uint32_t *__restrict__ cell_off, float4 *__restrict__ sorted_pos,
-                                  const uint32_t *__restrict__ skeys,
-                                  const uint32_t *__restrict__ perm,
-                                  const float4 *__restrict__ pos, uint32_t n, uint32_t ncells) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > n) return;
+__global__ void k_reorder_offsets(uint32_t *__restrict__ cell_off, const uint32_t *__restrict__ skeys, uint32_t n,
+                                  uint32_t ncells) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     // cells (prev, cur] start at i; thread n closes the tail up to ncells
-    uint32_t prev = i == 0 ? 0u : skeys[i - 1] + 1u;
-    uint32_t cur = i == n ? ncells : skeys[i];
-    for (uint32_t c = prev; c <= cur; ++c) cell_off[c] = i;
-    if (i < n && sorted_pos) sorted_pos[i] = pos[perm[i]];
+    const uint32_t first = i == 0 || i > n ? 0u : skeys[i - 1] + 1u;
+    const uint32_t cur = i >= n ? ncells : skeys[i];
+    fill_offsets(cell_off, i <= n, first, cur, i);
 }
 
 // A stable counting sort of each cell's particles by z slice.  A lane's
@@ -524,12 +698,24 @@ size_t sort_hist_entries(uint32_t n, int key_bits, int max_radix_bits) {
 cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in,
                          uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *hist, size_t hist_words, uint32_t n,
                          int key_bits, int max_radix_bits, cudaStream_t stream,
-                         bool *result_in_alt, int *launches) {
+                         bool *result_in_alt, int *launches, uint32_t *cell_off, uint32_t ncells,
+                         bool *offsets_done) {
     int passes, rb;
     split_bits(key_bits, max_radix_bits, &passes, &rb);
     bool with_vals = vals != nullptr;
     *result_in_alt = false;
+    if (offsets_done) *offsets_done = false;
     if (n == 0) return CUCO_OK;
+    if (n <= kClusterMax) {
+        uint32_t *off = offsets_done ? cell_off : nullptr;
+        if (offsets_done) *offsets_done = true;
+        *launches += 1;
+        const uint32_t ctas = kClusterCtas * kClusterThreads;
+        auto launch = n <= ctas ? launch_sort_cluster<1>
+                                : (n <= 2 * ctas ? launch_sort_cluster<2>
+                                                 : (n <= 4 * ctas ? launch_sort_cluster<4> : launch_sort_cluster<8>));
+        return launch(keys, vals, vals_in, n, passes, rb, off, ncells, stream);
+    }
     uint32_t *kbuf[2] = {keys, keys_alt};
     uint32_t *vbuf[2] = {vals, vals_alt};
     const int items = sort_items(n, rb, hist_words);
@@ -577,12 +763,9 @@ cuco_status_t launch_reorder_start_end(uint32_t *cell_start, uint32_t *cell_end,
     return CUCO_OK;
 }
 
-cuco_status_t launch_reorder_offsets(uint32_t *cell_off, float4 *sorted_pos,
-                                     const uint32_t *sorted_keys, const uint32_t *perm,
-                                     const float4 *pos, uint32_t n, uint32_t ncells,
+cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_keys, uint32_t n, uint32_t ncells,
                                      cudaStream_t stream) {
-    k_reorder_offsets<<<(n + 1 + 255) / 256, 256, 0, stream>>>(cell_off, sorted_pos, sorted_keys,
-                                                             perm, pos, n, ncells);
+    k_reorder_offsets<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, stream>>>(cell_off, sorted_keys, n, ncells);
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
