@@ -133,7 +133,7 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
         cudaFree(w.units);
         cudaFree(w.ctl);
         w = SRWork{};
-        capi_check(cudaMalloc(&w.units, sizeof(uint2) * cap), "cudaForceEvaluateShortrange");
+        capi_check(cudaMalloc(&w.units, sizeof(uint4) * cap), "cudaForceEvaluateShortrange");
         capi_check(cudaMalloc(&w.ctl, kSRCtlWords * sizeof(uint32_t)), "cudaForceEvaluateShortrange");
         capi_check(cudaMemset(w.ctl, 0, kSRCtlWords * sizeof(uint32_t)), "cudaForceEvaluateShortrange");
         w.cap = cap;
@@ -147,7 +147,7 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
     capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, off + numCells + 1, 0),
                 "cudaForceEvaluateShortrange");
     capi_status(launch_shortrange(p, (const float4 *)sortedPos, gridParticleIndex, off, s.table, (float4 *)gravAccel,
-                                  k, w, 0),
+                                  k, w, false, 0),
                 "cudaForceEvaluateShortrange");
     capi_status(shortrange_check(w.ctl, 0), "cudaForceEvaluateShortrange");
 }

@@ -11,6 +11,9 @@
 
 namespace cuco {
 
+struct SRPlan;
+struct SRWork;
+
 constexpr uint32_t kEmptyCell = 0xffffffffu;
 constexpr int kNTab = CUCO_NTAB;
 
@@ -85,7 +88,7 @@ cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in
                          uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *hist, size_t hist_words,
                          uint32_t n, int key_bits, int max_radix_bits, cudaStream_t stream,
                          bool *result_in_alt, int *launches, uint32_t *cell_off = nullptr, uint32_t ncells = 0,
-                         bool *offsets_done = nullptr);
+                         bool *offsets_done = nullptr, uint32_t *plan_ctl = nullptr);
 
 // Cell keys of float4 positions (calcHashD rule); idx gets 0..n-1 when non-null.
 cuco_status_t launch_cell_keys(const float4 *pos, uint32_t *keys, uint32_t *idx, uint32_t n,
@@ -99,9 +102,9 @@ cuco_status_t launch_reorder_start_end(uint32_t *cell_start, uint32_t *cell_end,
                                        uint32_t ncells, cudaStream_t stream);
 
 // Engine cell-bound format: cell_off[c] = first sorted index with key >= c,
-// for c in [0, ncells].
+// for c in [0, ncells].  plan_ctl (or null): the first three words are cleared.
 cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_keys, uint32_t n, uint32_t ncells,
-                                     cudaStream_t stream);
+                                     cudaStream_t stream, uint32_t *plan_ctl = nullptr);
 
 // The reference's cell bounds (cell_end is read where cell_start is not
 // empty) -> the engine's offsets (ncells + 1).  scratch: offsets_scratch(ncells)
@@ -124,13 +127,14 @@ struct CellBox {
 // slices[c] holds eight u16: entry j = the cell's particles in slices 0..j
 // (all 0xffff for a cell of 65535 or more).  Boxes: one (boxes null, `one`)
 // or nbox descriptors sorted by cell_base.  fixed: positions are 32-bit fixed
-// point.
+// point.  plan, work (one box): the launch also writes the short range's work
+// plan (its counters cleared by the kernel that wrote cell_off: plan_ctl).
 constexpr int kZSubBits = 3;
 constexpr int kZSub = 1 << kZSubBits;
 cuco_status_t launch_cell_subsort(const uint32_t *cell_off, const uint32_t *perm, const float4 *pos,
                                   float4 *sorted_pos, uint32_t *perm_s, uint4 *slices, uint32_t ncells,
                                   const CellBox &one, const CellBox *boxes, int nbox, bool fixed,
-                                  cudaStream_t stream);
+                                  cudaStream_t stream, const SRPlan *plan = nullptr, const SRWork *work = nullptr);
 
 // ----------------------------------------------------------- short range
 
@@ -156,6 +160,9 @@ struct ShortRangeParams {
     // flag cut, rcut^2 in double
     float rc2_lo, rc2_hi, hmin2, alo, ahi, r_hi;
     double rcut2_d;
+    // the 2^32 grid's cell corners: 2^32 = grid_q * grid + grid_r
+    uint32_t grid_q, grid_r;
+    float grid_inv;
     // the z-slice counts of the cells (launch_cell_subsort), indexed by cell
     // id; null when the sources are not in slice order
     const uint4 *slices;
@@ -170,16 +177,23 @@ struct KickArgs {
     const float4 *acc_pm_o;   // PM acceleration in original order (used when acc_pm_s is null)
 };
 
-// Device scratch of a launch's work plan: the units (first target, segment)
-// and the control words.  cap must be at least shortrange_unit_cap(n, segments)
+// Device scratch of a launch's work plan: the units (shortrange_plan.cuh) and
+// the control words.  cap must be at least shortrange_unit_cap(n, segments)
 // of the launch (G^3 bounds a box's segments).
 struct SRWork {
-    uint2 *units;
+    uint4 *units;
     uint32_t cap;
     uint32_t *ctl;  // kSRCtlWords: [0] dense slices listed, [1] next unit, [2] other units listed
                     // (reset per launch), [3] timeout word (kept until read), [4], [5] spare
 };
 uint32_t shortrange_unit_cap(uint32_t n, uint64_t segments);
+// What a box's plan needs: cells a segment, the cell grid, segments, targets a
+// unit.
+struct SRPlan {
+    int S, G;
+    uint32_t nseg, slice;
+};
+cuco_status_t shortrange_plan(const ShortRangeParams &p, SRPlan *plan);
 constexpr int kSRCtlWords = 8;
 // Reads and clears the short range's timeout word (ctl[3]) after the work on
 // `stream` is done: CUCO_ERR_TIMEOUT when a bounded wait gave up.
@@ -188,6 +202,7 @@ cuco_status_t shortrange_check(uint32_t *ctl, cudaStream_t stream);
 // `limit_cycles`: returns what shortrange_check then reports.
 cuco_status_t shortrange_timeout_probe(uint32_t *ctl, long long limit_cycles, cudaStream_t stream);
 
+// planned: the work plan is in `work` already (launch_cell_subsort wrote it).
 // pair_counter: when non-null, the launch adds its in-range pair count to it.
 // late_stream (with plan_done, an event of the caller's): the persistent grid
 // is split, one CTA per SM fewer on `stream` and the rest queued on
@@ -198,8 +213,8 @@ cuco_status_t shortrange_timeout_probe(uint32_t *ctl, long long limit_cycles, cu
 // spreads over both.  The launch is complete when both streams have run it.
 cuco_status_t launch_shortrange(const ShortRangeParams &p, const float4 *sorted_pos,
                                 const uint32_t *perm, const uint32_t *cell_off, const float *table,
-                                float4 *acc_out, const KickArgs &kick, const SRWork &work, cudaStream_t stream,
-                                unsigned long long *pair_counter = nullptr, cudaStream_t late_stream = nullptr,
+                                float4 *acc_out, const KickArgs &kick, const SRWork &work, bool planned,
+                                cudaStream_t stream, unsigned long long *pair_counter = nullptr, cudaStream_t late_stream = nullptr,
                                 cudaEvent_t plan_done = nullptr);
 
 // Many boxes in one launch (the batched form).  A box's descriptor holds its

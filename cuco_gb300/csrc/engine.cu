@@ -461,7 +461,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     bool in_alt = false, offsets_done = false;
     CUCO_TRY(sort_pairs(b->keys, b->perm, nullptr, b->keys_alt, b->perm_alt, b->hist, b->hist_words,
                         b->n, b->key_bits, 8, b->stream, &in_alt, &b->launches, b->cell_off, b->ncells,
-                        &offsets_done));
+                        &offsets_done, b->work.ctl));
     record(b, 2);
     // (the sort is handed over before the PM: a small box's step waits for the
     // host, and the sort heads the longer chain)
@@ -469,7 +469,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     b->sorted_keys = in_alt ? b->keys_alt : b->keys;
     b->sorted_perm = in_alt ? b->perm_alt : b->perm;
     if (!offsets_done) {
-        CUCO_TRY(launch_reorder_offsets(b->cell_off, b->sorted_keys, b->n, b->ncells, b->stream));
+        CUCO_TRY(launch_reorder_offsets(b->cell_off, b->sorted_keys, b->n, b->ncells, b->stream, b->work.ctl));
         b->launches += 1;
     }
     // the cell order refined by z slice (the short range trims its column
@@ -478,8 +478,12 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     uint32_t *perm_s = in_alt ? b->perm : b->perm_alt;
     b->perm_s = perm_s;
     const CellBox cb{(uint32_t)b->G, 0u, b->cfg.boxsize, b->gridfac};
+    // (and the short range's work plan, in the same launch)
+    SRPlan plan{};
+    const bool planned = pp && shortrange_plan(make_sr_params(b), &plan) == CUCO_OK;
     CUCO_TRY(launch_cell_subsort(b->cell_off, b->sorted_perm, b->pos, b->spos, perm_s, b->cell_sl, b->ncells, cb,
-                                 nullptr, 1, b->cfg.mode == CUCO_MODE_FIXED, b->stream));
+                                 nullptr, 1, b->cfg.mode == CUCO_MODE_FIXED, b->stream, planned ? &plan : nullptr,
+                                 &b->work));
     b->launches += 1;
     record(b, 3);
     if (cell_ordered_pm) {
@@ -503,10 +507,10 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
         k.acc_pm_s = nullptr;
         k.acc_pm_out = nullptr;
         k.acc_pm_o = pm && !split ? b->acc_pm : nullptr;
-        CUCO_TRY(launch_shortrange(make_sr_params(b), b->spos, perm_s, b->cell_off, b->table, b->acc_pp, k, b->work, b->stream,
+        CUCO_TRY(launch_shortrange(make_sr_params(b), b->spos, perm_s, b->cell_off, b->table, b->acc_pp, k, b->work, planned, b->stream,
                                    b->count_pairs ? b->pair_counter : nullptr, split ? b->pm_stream : nullptr,
                                    b->sr_plan));
-        b->launches += split ? 3 : 2;  // work plan + persistent short range (in two parts beside the PM)
+        b->launches += split ? 2 : 1;  // the persistent short range (in two parts beside the PM)
     }
     if (split) CUCO_TRY(join_pm(b));
     record(b, 9);  // the short range done (both parts)
@@ -619,6 +623,10 @@ cuco_status_t cuco_box_create(const cuco_config_t *cfg, cuco_box_t **out) {
     }
     const size_t n = b->n;
     b->hist_words = sort_hist_entries(b->n, b->key_bits, 8);
+    // (a cell grid that rcut does not fit has no segments: its passes without
+    // the short range still run)
+    SRPlan plan{};
+    const uint32_t units = shortrange_unit_cap(b->n, shortrange_plan(make_sr_params(b), &plan) == CUCO_OK ? plan.nseg : 0);
     if ((s = alloc(&b->pos, n)) || (s = alloc(&b->vel, n)) || (s = alloc(&b->acc_pp, n)) ||
         (s = alloc(&b->acc_pm, n)) || (s = alloc(&b->spos, n)) ||
         (s = alloc(&b->keys, n)) || (s = alloc(&b->perm, n)) || (s = alloc(&b->keys_alt, n)) ||
@@ -627,11 +635,11 @@ cuco_status_t cuco_box_create(const cuco_config_t *cfg, cuco_box_t **out) {
         (s = alloc(&b->cell_off, (size_t)b->ncells + 1)) || (s = alloc(&b->cell_sl, (size_t)b->ncells)) ||
         (s = alloc(&b->table, kNTab)) ||
         (s = alloc(&b->stage3, 3 * n)) || (s = alloc(&b->pair_counter, 1)) ||
-        (s = alloc(&b->work.units, shortrange_unit_cap(b->n, b->ncells))) ||
+        (s = alloc(&b->work.units, units)) ||
         (s = alloc(&b->work.ctl, kSRCtlWords)))
         return fail(s);
     cudaMemset(b->work.ctl, 0, sizeof(uint32_t) * kSRCtlWords);
-    b->work.cap = shortrange_unit_cap(b->n, b->ncells);  // G^3 covers every segment length
+    b->work.cap = units;
     cudaMemset(b->pair_counter, 0, sizeof(unsigned long long));
     std::vector<float> t(kNTab);
     shortrange_table(t.data());

@@ -335,7 +335,7 @@ struct cuco_ensemble {
            cap_hkicks[2] = {0, 0},
            cap_mapz = 0, cap_mapa = 0, cap_units = 0, cap_ctl = 0, cap_cellsl = 0;
     // the short range's work-plan scratch
-    uint2 *sr_units = nullptr;
+    uint4 *sr_units = nullptr;
     uint32_t *sr_ctl = nullptr;
 };
 

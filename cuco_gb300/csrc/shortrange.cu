@@ -65,6 +65,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "shortrange_plan.cuh"
 
 namespace cuco {
 
@@ -79,11 +80,6 @@ constexpr int kMaxSeg = 8;
 // targets of a group (a warp's lanes are kGroup targets x 32 / kGroup list
 // slots, or fewer targets and more slots)
 constexpr int kGroup = 16;
-// A unit is kUnitMin to kUnitMax targets; the units of a segment of more than
-// kDense targets are one group each (their boxes hardly grow with the group,
-// as a dense cell's slices are thin) and listed ahead of the others.
-constexpr int kUnitMin = 8, kUnitMax = 32;
-constexpr uint32_t kDense = 128;
 // A warp's list is evaluated when it holds kListFull sources; one more window
 // pair (64) may be appended before that is seen, and the last evaluation pads
 // it to whole iterations.
@@ -234,9 +230,9 @@ __global__ void k_staging_timeout_probe(uint32_t *__restrict__ err, long long li
     if (__syncthreads_or(!ok) && threadIdx.x == 0) atomicOr(err, 1u);
 }
 
-// One unit: the targets from sorted index t_begin on, at most `tmax` of them
-// and none past the end of segment `seg` of one box (p; ncols, R, S, margin of
-// its column set, dxdy(col) its columns' offsets).  kick_pp/kick_pm are that
+// One unit (its record: plan_segment) of one box (p; ncols, R, S, margin of its
+// column set, dxdy(col) its columns' offsets); dense: its targets are one
+// group.  kick_pp/kick_pm are that
 // box's kick factors.  Every lane of the warp calls it together; wm is the
 // warp's shared memory, tab the split table.
 // `law`: the pair law's constants (rc2_lo, rc2_hi, hmin2, alo, ahi, rcut2_d,
@@ -248,19 +244,17 @@ __global__ void k_staging_timeout_probe(uint32_t *__restrict__ err, long long li
 template <bool KICK, bool COUNT, bool FIXED, bool PIN_LAW, typename Columns>
 __device__ __forceinline__ void shortrange_unit(
     const ShortRangeParams &p, const ShortRangeParams &law, const int ncols, const int R, const int S,
-    const float margin, Columns dxdy, const int seg, const uint32_t t_begin, const uint32_t tmax, const bool dense,
+    const float margin, Columns dxdy, const uint4 unit, const bool dense,
     const double kick_pp, const double kick_pm, const float4 *__restrict__ spos, const uint32_t *__restrict__ perm,
     const uint32_t *__restrict__ cell_off, float4 *__restrict__ acc_out, const KickArgs &kick, WarpMem &wm,
     const float *tab, uint32_t &npairs) {
     const int lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u, le_mask = lt_mask | (1u << lane);
     const int G = p.grid, nz = S + 2 * R;
-    const int segs = G / S;
-    const int ix = seg / (G * segs), iy = (seg / segs) % G, iz0 = (seg % segs) * S;
+    const int ix = unit.w & 1023, iy = (unit.w >> 10) & 1023, iz0 = unit.w >> 20;
+    const uint32_t t_begin = unit.x, len = unit.y & 255u;
     const float L = p.boxsize, w = p.cellw, winv = 1.0f / w, fs = p.fscale;
     const bool ZS = p.slices != nullptr;  // sources in z-slice order within cells, with slice counts
-    const uint32_t t_end = cell_off[p.cell_base + ((uint32_t)ix * G + iy) * G + iz0 + S];
-    const uint32_t len = min(tmax, t_end - t_begin);
 
     // integer origin at the segment corner (see the file comment), and the
     // corner's offset from it
@@ -269,9 +263,10 @@ __device__ __forceinline__ void shortrange_unit(
     // Fixed-point positions: the origin is the segment corner on the 2^32
     // grid, and an int32 difference from it is the periodic image for free
     // (every source lies within S + R < G/2 cells of it).
-    const uint32_t oxu = (uint32_t)(((uint64_t)ix << 32) / (uint32_t)G);
-    const uint32_t oyu = (uint32_t)(((uint64_t)iy << 32) / (uint32_t)G);
-    const uint32_t ozu = (uint32_t)(((uint64_t)iz0 << 32) / (uint32_t)G);
+    // floor(i 2^32 / G) = i q + floor(i r / G), 2^32 = q G + r (i r < 2^20: the
+    // float quotient of the odd numerator is never a whole number off)
+    auto corner = [&](int i) { return (uint32_t)i * p.grid_q + (uint32_t)(((float)(i * (int)p.grid_r) + 0.5f) * p.grid_inv); };
+    const uint32_t oxu = FIXED ? corner(ix) : 0u, oyu = FIXED ? corner(iy) : 0u, ozu = FIXED ? corner(iz0) : 0u;
     // __fmul_rn: a target's coordinates must equal its own list entry bit
     // for bit (the self pair then has r = 0 exactly), so the product may not
     // be contracted into the later subtraction
@@ -676,51 +671,9 @@ __device__ __forceinline__ void shortrange_unit(
     __syncwarp();
 }
 
-// The work plan of one launch, by the warps of a grid over all segments: the
-// units of one segment (nt targets from sorted index tb on), appended in any
-// order (which warp computes a target does not change its result): the slices
-// of a dense segment from the front of the list, the others' from its back.
-__device__ __forceinline__ void plan_segment(uint32_t tb, uint32_t nt, uint32_t gseg, uint32_t slice, const SRWork &w) {
-    const uint32_t lane = threadIdx.x & 31;
-    const bool dense = nt > kDense;
-    // this lane's first place among the places of the warp's lanes
-    auto place = [&](uint32_t c, uint32_t *counter) {
-        uint32_t incl = c;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t v = __shfl_up_sync(kFull, incl, off);
-            if (lane >= off) incl += v;
-        }
-        uint32_t first = 0;
-        if (lane == 31 && incl) first = atomicAdd(counter, incl);
-        return __shfl_sync(kFull, first, 31) + incl - c;
-    };
-    const uint32_t c = dense ? 0u : (nt + slice - 1) / slice;
-    const uint32_t o = place(c, &w.ctl[2]);
-    for (uint32_t k = 0; k < c; ++k) w.units[CUCO_IDX(w.cap - 1u - (o + k), w.cap)] = make_uint2(tb + k * slice, gseg);
-    uint32_t any = __ballot_sync(kFull, dense);
-    if (!any) return;
-    const uint32_t cd = dense ? (nt + slice - 1) / slice : 0u;
-    const uint32_t od = place(cd, &w.ctl[0]);
-    // the warp writes one dense segment's slices after the other
-    for (; any; any &= any - 1) {
-        const int src = __ffs(any) - 1;
-        const uint32_t cs = __shfl_sync(kFull, cd, src), os = __shfl_sync(kFull, od, src),
-                       ts = __shfl_sync(kFull, tb, src), gs = __shfl_sync(kFull, gseg, src);
-        for (uint32_t k = lane; k < cs; k += 32) w.units[CUCO_IDX(os + k, w.cap)] = make_uint2(ts + k * slice, gs);
-    }
-}
-
-__global__ void k_sr_plan(const __grid_constant__ ShortRangeParams p, int S, uint32_t nseg,
-                          const uint32_t *__restrict__ cell_off, uint32_t slice, const __grid_constant__ SRWork w) {
-    const uint32_t seg = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t tb = 0, nt = 0;
-    if (seg < nseg) {
-        // segments are numbered in cell order: seg's first cell is seg * S
-        tb = cell_off[(size_t)seg * S];
-        nt = cell_off[(size_t)seg * S + S] - tb;
-    }
-    plan_segment(tb, nt, seg, slice, w);
+__global__ void k_sr_plan(const __grid_constant__ SRPlan plan, const uint32_t *__restrict__ cell_off,
+                          const __grid_constant__ SRWork w) {
+    plan_box_segment(plan, blockIdx.x * blockDim.x + threadIdx.x, cell_off, 0u, 0u, w);
 }
 
 // The next unit for a warp: the dense slices first (the longest work).  Takes
@@ -743,7 +696,7 @@ struct UnitQueue {
         return i + fixed;
     }
     // false when none is left; dense_unit: a slice of a dense segment
-    __device__ __forceinline__ bool next(uint2 *unit, bool *dense_unit) {
+    __device__ __forceinline__ bool next(uint4 *unit, bool *dense_unit) {
         const uint32_t i = __shfl_sync(kFull, item, 0);
         if (i >= total) return false;
         item = fetch();
@@ -767,7 +720,7 @@ __device__ __forceinline__ void add_pairs(uint32_t npairs, unsigned long long *p
 // none is left.
 template <bool KICK, bool COUNT, bool FIXED>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
-    k_shortrange(const __grid_constant__ ShortRangeParams p, const __grid_constant__ ColumnSet cs, uint32_t slice,
+    k_shortrange(const __grid_constant__ ShortRangeParams p, const __grid_constant__ ColumnSet cs,
                  uint32_t fixed, int late, const __grid_constant__ SRWork w, const float4 *__restrict__ spos,
                  const uint32_t *__restrict__ perm, const uint32_t *__restrict__ cell_off,
                  const float *__restrict__ table_g, float4 *__restrict__ acc_out,
@@ -780,14 +733,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     __syncthreads();
     WarpMem &wm = s_warp[threadIdx.x >> 5];
     UnitQueue q(w, fixed, late != 0);
-    uint2 u;
+    uint4 u;
     bool dense;
     while (q.next(&u, &dense)) {
         uint32_t npairs = 0;
         shortrange_unit<KICK, COUNT, FIXED, false>(p, p, cs.ncols, cs.R, cs.S, cs.margin,
-                                                   [&](int col) { return s_col[col]; }, (int)u.y, u.x,
-                                                   slice, dense, kick.kick_pp, kick.kick_pm, spos,
-                                                   perm, cell_off, acc_out, kick, wm, s_tab, npairs);
+                                                   [&](int col) { return s_col[col]; }, u, dense, kick.kick_pp,
+                                                   kick.kick_pm, spos, perm, cell_off, acc_out, kick, wm, s_tab,
+                                                   npairs);
         if (COUNT) add_pairs(npairs, pair_counter);
     }
 }
@@ -799,15 +752,16 @@ __global__ void k_sr_plan_multi(const SRBoxDesc *__restrict__ boxes, const uint3
                                 int nbox, uint32_t nseg, const uint32_t *__restrict__ cell_off, uint32_t slice,
                                 const __grid_constant__ SRWork w) {
     const uint32_t gseg = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t tb = 0, nt = 0;
+    SRPlan plan{1, 1, 0u, slice};
+    uint32_t b = 0, seg = 0, base = 0;
     if (gseg < nseg) {
-        const int b = find_box(seg_base, nbox, gseg);
+        b = find_box(seg_base, nbox, gseg);
         const SRBoxDesc &d = boxes[b];
-        const uint32_t c0 = d.p.cell_base + (gseg - seg_base[b]) * (uint32_t)d.cs.S;
-        tb = cell_off[c0];
-        nt = cell_off[c0 + d.cs.S] - tb;
+        seg = gseg - seg_base[b];
+        plan = SRPlan{d.cs.S, d.p.grid, 0xffffffffu, slice};
+        base = d.p.cell_base;
     }
-    plan_segment(tb, nt, gseg, slice, w);
+    plan_box_segment(plan, seg, cell_off, base, b, w);
 }
 
 // UNIFORM: every box has the pair law of `law` (a kernel parameter, read as
@@ -815,7 +769,6 @@ __global__ void k_sr_plan_multi(const SRBoxDesc *__restrict__ boxes, const uint3
 template <bool KICK, bool COUNT, bool FIXED, bool UNIFORM>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
     k_shortrange_multi(const SRBoxDesc *__restrict__ boxes, const double2 *__restrict__ kicks,
-                       const uint32_t *__restrict__ seg_base, int nbox, uint32_t slice,
                        uint32_t fixed, const __grid_constant__ SRWork w, const float4 *__restrict__ spos,
                        const uint32_t *__restrict__ perm, const uint32_t *__restrict__ cell_off,
                        const float *__restrict__ table_g, float4 *__restrict__ acc_out,
@@ -827,17 +780,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     __syncthreads();
     WarpMem &wm = s_warp[threadIdx.x >> 5];
     UnitQueue q(w, fixed, false);
-    uint2 u;
+    uint4 u;
     bool dense;
     while (q.next(&u, &dense)) {
-        const int b = find_box(seg_base, nbox, u.y);
+        const uint32_t b = u.y >> 8;
         const SRBoxDesc &d = boxes[b];
         const double2 k = KICK ? kicks[b] : make_double2(0.0, 0.0);
         uint32_t npairs = 0;
         shortrange_unit<KICK, COUNT, FIXED, !UNIFORM>(
             d.p, UNIFORM ? law : d.p, d.cs.ncols, d.cs.R, d.cs.S, d.cs.margin,
-            [&](int col) { return make_char2(d.cs.dx[col], d.cs.dy[col]); }, (int)(u.y - seg_base[b]), u.x,
-            slice, dense, k.x, k.y, spos, perm, cell_off, acc_out, kick, wm, s_tab, npairs);
+            [&](int col) { return make_char2(d.cs.dx[col], d.cs.dy[col]); }, u, dense, k.x, k.y, spos, perm, cell_off, acc_out, kick, wm, s_tab, npairs);
         if (COUNT) add_pairs(npairs, pair_counter);
     }
 }
@@ -905,12 +857,11 @@ void launch_kick(cudaStream_t stream, cudaStream_t late_stream, const ShortRange
     auto launch = [&](auto kernel) {
         const PersistentGrid g = persistent_grid(kernel);
         const unsigned late = late_stream && g.per > 1 ? g.sms : 0u;
-        const uint32_t slice = unit_slice(p.n);
         const unsigned first = g.sms * g.per - late;
-        kernel<<<first, kThreads, 0, stream>>>(p, cs, slice, first * kWarps, 0, work, sorted_pos, perm, cell_off,
+        kernel<<<first, kThreads, 0, stream>>>(p, cs, first * kWarps, 0, work, sorted_pos, perm, cell_off,
                                                table, acc_out, kick, counter);
         if (late)
-            kernel<<<late, kThreads, 0, late_stream>>>(p, cs, slice, first * kWarps, 1, work, sorted_pos, perm,
+            kernel<<<late, kThreads, 0, late_stream>>>(p, cs, first * kWarps, 1, work, sorted_pos, perm,
                                                        cell_off, table, acc_out, kick, counter);
     };
     if (counter)
@@ -920,9 +871,9 @@ void launch_kick(cudaStream_t stream, cudaStream_t late_stream, const ShortRange
 }
 
 uint32_t shortrange_unit_cap(uint32_t n, uint64_t segments) {
-    // a dense segment: ceil(nt / kUnitMin) <= nt / kUnitMin + nt / kDense;
-    // another: at most nt / kUnitMin + 1
-    return n / kUnitMin + n / kDense + (uint32_t)std::min<uint64_t>(n, segments) + 16u;
+    // a dense segment: ceil(nt / slice) <= nt / slice + nt / kDense; another:
+    // at most nt / slice + 1
+    return n / unit_slice(n) + n / kDense + (uint32_t)std::min<uint64_t>(n, segments) + 16u;
 }
 
 cuco_status_t shortrange_timeout_probe(uint32_t *ctl, long long limit_cycles, cudaStream_t stream) {
@@ -954,31 +905,48 @@ static void finish_pair_law(ShortRangeParams &p) {
     p.alo = p.fixed ? p.asmthfac : p.asmthfac * (1.f - kEdge);
     p.ahi = p.fixed ? p.asmthfac : p.asmthfac * (1.f + kEdge);
     p.rcut2_d = (double)p.rcut * (double)p.rcut;
+    p.grid_q = (uint32_t)((1ull << 32) / (uint32_t)p.grid);
+    p.grid_r = (uint32_t)((1ull << 32) % (uint32_t)p.grid);
+    p.grid_inv = 1.0f / (float)p.grid;
     p.r_hi = (float)(sqrt((double)p.rc2_hi) * (1.0 + 1e-6));
+}
+
+namespace {
+cuco_status_t columns_of(const ShortRangeParams &p, ColumnSet *cs) {
+    if (build_columns(p, cs)) return CUCO_OK;
+    set_error("short range: cell grid does not fit rcut (need rcut <= 8 cell widths, "
+              "rcut < L/2 and at least S+2R cells per dimension)");
+    return CUCO_ERR_UNSUPPORTED;
+}
+}  // namespace
+
+cuco_status_t shortrange_plan(const ShortRangeParams &p, SRPlan *plan) {
+    ColumnSet cs;
+    CUCO_TRY(columns_of(p, &cs));
+    *plan = SRPlan{cs.S, p.grid, (uint32_t)p.grid * p.grid * (p.grid / cs.S), unit_slice(p.n)};
+    return CUCO_OK;
 }
 
 cuco_status_t launch_shortrange(const ShortRangeParams &p_in, const float4 *sorted_pos, const uint32_t *perm,
                                 const uint32_t *cell_off, const float *table, float4 *acc_out, const KickArgs &kick,
-                                const SRWork &work, cudaStream_t stream, unsigned long long *pair_counter,
-                                cudaStream_t late_stream, cudaEvent_t plan_done) {
+                                const SRWork &work, bool planned, cudaStream_t stream,
+                                unsigned long long *pair_counter, cudaStream_t late_stream, cudaEvent_t plan_done) {
     ColumnSet cs;
     ShortRangeParams p = p_in;
     finish_pair_law(p);
-    if (!build_columns(p, &cs)) {
-        set_error("short range: cell grid does not fit rcut (need rcut <= 8 cell widths, "
-                  "rcut < L/2 and at least S+2R cells per dimension)");
-        return CUCO_ERR_UNSUPPORTED;
-    }
+    CUCO_TRY(columns_of(p, &cs));
     if (p.n == 0) return CUCO_OK;
-    const int G = p.grid;
-    const uint32_t nseg = (uint32_t)G * G * (G / cs.S);
-    if (work.cap < shortrange_unit_cap(p.n, nseg)) {
+    SRPlan plan;
+    CUCO_TRY(shortrange_plan(p, &plan));
+    if (work.cap < shortrange_unit_cap(p.n, plan.nseg)) {
         set_error("short range: work-plan scratch too small for this grid or particle count");
         return CUCO_ERR_INVALID;
     }
     const bool kick_on = kick.vel != nullptr;
-    CUCO_TRY_CUDA(cudaMemsetAsync(work.ctl, 0, 3 * sizeof(uint32_t), stream));
-    k_sr_plan<<<(nseg + 255) / 256, 256, 0, stream>>>(p, cs.S, nseg, cell_off, unit_slice(p.n), work);
+    if (!planned) {
+        CUCO_TRY_CUDA(cudaMemsetAsync(work.ctl, 0, 3 * sizeof(uint32_t), stream));
+        k_sr_plan<<<(plan.nseg + 255) / 256, 256, 0, stream>>>(plan, cell_off, work);
+    }
     if (late_stream) {
         if (!plan_done) {
             set_error("short range: a split launch needs the caller's plan event");
@@ -1000,11 +968,7 @@ cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32
     SRBoxDesc d{};
     d.p = p;
     finish_pair_law(d.p);
-    if (!build_columns(p, &d.cs)) {
-        set_error("short range: cell grid does not fit rcut (need rcut <= 8 cell widths, "
-                  "rcut < L/2 and at least S+2R cells per dimension)");
-        return CUCO_ERR_UNSUPPORTED;
-    }
+    CUCO_TRY(columns_of(p, &d.cs));
     memcpy(desc, &d, sizeof d);
     *segments = (uint32_t)p.grid * p.grid * (p.grid / d.cs.S);
     return CUCO_OK;
@@ -1046,7 +1010,7 @@ cuco_status_t launch_shortrange_multi(const void *descs, const double2 *kicks, c
     do {                                                                                                \
         const PersistentGrid g = persistent_grid(k_shortrange_multi<K, C, F, U>);                        \
         k_shortrange_multi<K, C, F, U><<<g.sms * g.per, kThreads, 0, stream>>>(                          \
-            d, kicks, seg_base, nbox, slice, g.sms * g.per * kWarps, work, sorted_pos, perm, cell_off, table, acc_out, kick,        \
+            d, kicks, g.sms * g.per * kWarps, work, sorted_pos, perm, cell_off, table, acc_out, kick,        \
             pair_counter, law);                                                                         \
     } while (0)
 #define CUCO_SR_MULTI(K, C, F)                 \

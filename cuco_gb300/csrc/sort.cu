@@ -35,6 +35,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "shortrange_plan.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -346,7 +347,7 @@ struct ClusterMem {
 template <int ITEMS>
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
     k_sort_cluster(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in, uint32_t n, int passes, int rb,
-                   uint32_t *__restrict__ cell_off, uint32_t ncells) {
+                   uint32_t *__restrict__ cell_off, uint32_t ncells, uint32_t *__restrict__ plan_ctl) {
     constexpr uint32_t E = kClusterThreads * ITEMS;  // keys of a CTA
     extern __shared__ __align__(16) unsigned char cluster_smem[];
     ClusterMem<ITEMS> &sm = *reinterpret_cast<ClusterMem<ITEMS> *>(cluster_smem);
@@ -354,6 +355,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     const uint32_t rank = cluster.block_rank();
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lt = (1u << lane) - 1u;
     const uint32_t radix = 1u << rb;
+    if (plan_ctl && rank == 0 && tid < 3) plan_ctl[tid] = 0u;
     // item k of this thread: CTA position `first + 32 k`, input order over
     // (CTA, warp, item, lane)
     const uint32_t first = warp * (32 * ITEMS) + lane, g0 = rank * E + first;
@@ -485,12 +487,13 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
 
 template <int ITEMS>
 cuco_status_t launch_sort_cluster(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in, uint32_t n, int passes,
-                                  int rb, uint32_t *cell_off, uint32_t ncells, cudaStream_t stream) {
+                                  int rb, uint32_t *cell_off, uint32_t ncells, uint32_t *plan_ctl,
+                                  cudaStream_t stream) {
     static const cudaError_t attr = cudaFuncSetAttribute(
         k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterMem<ITEMS>));
     CUCO_TRY_CUDA(attr);
     k_sort_cluster<ITEMS><<<kClusterCtas, kClusterThreads, sizeof(ClusterMem<ITEMS>), stream>>>(
-        keys, vals, vals_in, n, passes, rb, cell_off, ncells);
+        keys, vals, vals_in, n, passes, rb, cell_off, ncells, plan_ctl);
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
@@ -521,8 +524,9 @@ __global__ void k_reorder_start_end(uint32_t *__restrict__ cell_start, uint32_t 
 }
 
 __global__ void k_reorder_offsets(uint32_t *__restrict__ cell_off, const uint32_t *__restrict__ skeys, uint32_t n,
-                                  uint32_t ncells) {
+                                  uint32_t ncells, uint32_t *__restrict__ plan_ctl) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (plan_ctl && i < 3) plan_ctl[i] = 0u;
     // cells (prev, cur] start at i; thread n closes the tail up to ncells
     const uint32_t first = i == 0 || i > n ? 0u : skeys[i - 1] + 1u;
     const uint32_t cur = i >= n ? ncells : skeys[i];
@@ -649,10 +653,16 @@ __global__ void k_cell_subsort(const uint32_t *__restrict__ cell_off, const uint
                                const float4 *__restrict__ pos, float4 *__restrict__ sorted_pos,
                                uint32_t *__restrict__ perm_s, uint4 *__restrict__ slices, uint32_t ncells,
                                const __grid_constant__ CellBox one, const CellBox *__restrict__ boxes, int nbox,
-                               int fixed) {
+                               int fixed, uint32_t plan_blocks, const __grid_constant__ SRPlan plan,
+                               const __grid_constant__ SRWork work) {
+    // the first blocks write the short range's work plan (a launch less)
+    if (blockIdx.x < plan_blocks) {
+        plan_box_segment(plan, blockIdx.x * blockDim.x + threadIdx.x, cell_off, 0u, 0u, work);
+        return;
+    }
     constexpr uint32_t kCells = 32 / kSubLanes;
     const uint32_t lane = threadIdx.x & 31, grp = lane / kSubLanes;
-    const uint32_t c0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kCells;
+    const uint32_t c0 = (((blockIdx.x - plan_blocks) * blockDim.x + threadIdx.x) >> 5) * kCells;
     if (c0 >= ncells) return;  // warp-uniform
     const uint32_t c = c0 + grp;
     const bool valid = c < ncells;
@@ -678,11 +688,13 @@ __global__ void k_cell_subsort(const uint32_t *__restrict__ cell_off, const uint
 cuco_status_t launch_cell_subsort(const uint32_t *cell_off, const uint32_t *perm, const float4 *pos,
                                   float4 *sorted_pos, uint32_t *perm_s, uint4 *slices, uint32_t ncells,
                                   const CellBox &one, const CellBox *boxes, int nbox, bool fixed,
-                                  cudaStream_t stream) {
+                                  cudaStream_t stream, const SRPlan *plan, const SRWork *work) {
     if (ncells == 0) return CUCO_OK;
     const uint64_t threads = 32ull * ((ncells + 32 / kSubLanes - 1) / (32 / kSubLanes));
-    k_cell_subsort<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>(
-        cell_off, perm, pos, sorted_pos, perm_s, slices, ncells, one, boxes, nbox, fixed ? 1 : 0);
+    const uint32_t plan_blocks = plan ? (plan->nseg + 255) / 256 : 0u;
+    k_cell_subsort<<<plan_blocks + (unsigned)((threads + 255) / 256), 256, 0, stream>>>(
+        cell_off, perm, pos, sorted_pos, perm_s, slices, ncells, one, boxes, nbox, fixed ? 1 : 0, plan_blocks,
+        plan ? *plan : SRPlan{}, work ? *work : SRWork{});
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
@@ -699,7 +711,7 @@ cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in
                          uint32_t *keys_alt, uint32_t *vals_alt, uint32_t *hist, size_t hist_words, uint32_t n,
                          int key_bits, int max_radix_bits, cudaStream_t stream,
                          bool *result_in_alt, int *launches, uint32_t *cell_off, uint32_t ncells,
-                         bool *offsets_done) {
+                         bool *offsets_done, uint32_t *plan_ctl) {
     int passes, rb;
     split_bits(key_bits, max_radix_bits, &passes, &rb);
     bool with_vals = vals != nullptr;
@@ -714,7 +726,7 @@ cuco_status_t sort_pairs(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in
         auto launch = n <= ctas ? launch_sort_cluster<1>
                                 : (n <= 2 * ctas ? launch_sort_cluster<2>
                                                  : (n <= 4 * ctas ? launch_sort_cluster<4> : launch_sort_cluster<8>));
-        return launch(keys, vals, vals_in, n, passes, rb, off, ncells, stream);
+        return launch(keys, vals, vals_in, n, passes, rb, off, ncells, plan_ctl, stream);
     }
     uint32_t *kbuf[2] = {keys, keys_alt};
     uint32_t *vbuf[2] = {vals, vals_alt};
@@ -764,8 +776,9 @@ cuco_status_t launch_reorder_start_end(uint32_t *cell_start, uint32_t *cell_end,
 }
 
 cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_keys, uint32_t n, uint32_t ncells,
-                                     cudaStream_t stream) {
-    k_reorder_offsets<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, stream>>>(cell_off, sorted_keys, n, ncells);
+                                     cudaStream_t stream, uint32_t *plan_ctl) {
+    k_reorder_offsets<<<(unsigned)(((size_t)n + 1 + 255) / 256), 256, 0, stream>>>(cell_off, sorted_keys, n, ncells,
+                                                                                   plan_ctl);
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
