@@ -205,22 +205,27 @@ int tune_cell_grid(const cuco_config_t &c0, cudaStream_t stream) {
     return best;
 }
 
-// FFT batching (columns per CTA) by timing one-box multi launches.
+// FFT batching (columns per CTA) by timing multi launches over as many copies
+// of the mesh as fill the GPU (2^24 points): alone, a small mesh is fastest
+// in batches so small that its CTAs' threads idle, which is what a full
+// ensemble then pays (the z passes of 16 boxes of 16^3 to 80^3: 357 us for
+// batches timed alone, 260 for these).
 void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out, int *B_out) {
     *P_out = pm_batch_z(M);
     *B_out = pm_batch_axis(M);
-    const size_t Mh = M / 2 + 1;
+    const size_t Mh = M / 2 + 1, points = (size_t)M * M * M;
+    const int copies = (int)std::min<size_t>(std::max<size_t>(((size_t)1 << 24) / points, 1), 64);
     float *rho = nullptr, *green = nullptr;
     unsigned long long *rho64 = nullptr;
     float2 *spec = nullptr, *tw = nullptr;
     PMBoxDesc *dd = nullptr;
     uint32_t *pbeg = nullptr;
     uint2 *mz = nullptr, *ma = nullptr;
-    bool ok = dalloc(&rho, (size_t)M * M * M) == CUCO_OK && dalloc(&rho64, (size_t)M * M * M) == CUCO_OK &&
-              dalloc(&spec, pm_spec_points(M)) == CUCO_OK &&
-              dalloc(&green, Mh) == CUCO_OK && dalloc(&tw, (size_t)M) == CUCO_OK && dalloc(&dd, 1) == CUCO_OK &&
-              dalloc(&pbeg, 2) == CUCO_OK && dalloc(&mz, (size_t)M * M) == CUCO_OK &&
-              dalloc(&ma, (size_t)M * Mh) == CUCO_OK;
+    bool ok = dalloc(&rho, points * copies) == CUCO_OK && dalloc(&rho64, points * copies) == CUCO_OK &&
+              dalloc(&spec, pm_spec_points(M) * copies) == CUCO_OK &&
+              dalloc(&green, Mh) == CUCO_OK && dalloc(&tw, (size_t)M) == CUCO_OK &&
+              dalloc(&dd, (size_t)copies) == CUCO_OK && dalloc(&pbeg, (size_t)copies + 1) == CUCO_OK &&
+              dalloc(&mz, (size_t)M * M * copies) == CUCO_OK && dalloc(&ma, (size_t)M * Mh * copies) == CUCO_OK;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (ok) {
         std::vector<float> g(Mh);
@@ -228,9 +233,8 @@ void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out
         pm_tables(M, boxsize, asmth, g.data(), t.data());
         cudaMemcpy(green, g.data(), sizeof(float) * Mh, cudaMemcpyHostToDevice);
         cudaMemcpy(tw, t.data(), sizeof(float2) * M, cudaMemcpyHostToDevice);
-        cudaMemset(rho, 0, sizeof(float) * (size_t)M * M * M);
-        const uint32_t pb[2] = {0, 0};
-        cudaMemcpy(pbeg, pb, sizeof pb, cudaMemcpyHostToDevice);
+        cudaMemset(rho, 0, sizeof(float) * points * copies);
+        cudaMemset(pbeg, 0, sizeof(uint32_t) * (copies + 1));
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
         float best = 1e30f;
@@ -238,17 +242,20 @@ void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out
             if (P > M / 2 || (M * M / 2) % P || pm_smem_z(M, P) > 200 * 1024) continue;
             for (int B : {4, 8, 16}) {
                 if (pm_smem_axis(M, B) > 200 * 1024 || !pm_fft_batches_ok(M, P, B)) continue;
-                PMBoxDesc d{M, P, B, pm_stage_plan(M), 1.f, 0.f, 0.f, rho, rho64, 1.f, spec, green, tw};
-                cudaMemcpy(dd, &d, sizeof d, cudaMemcpyHostToDevice);
-                const uint32_t nz = (uint32_t)(M * M / (2 * P)), nbx = (uint32_t)((Mh + B - 1) / B),
-                               na = nbx * M;
-                std::vector<uint2> vz(nz), va(na);
-                for (uint32_t k = 0; k < nz; ++k) vz[k] = make_uint2(0, k);
-                for (uint32_t k = 0; k < na; ++k) va[k] = make_uint2(0, k);
-                cudaMemcpy(mz, vz.data(), sizeof(uint2) * nz, cudaMemcpyHostToDevice);
-                cudaMemcpy(ma, va.data(), sizeof(uint2) * na, cudaMemcpyHostToDevice);
-                PMMulti m{1, false, dd, pbeg, mz, ma, nz, na, pm_smem_z(M, P), pm_smem_axis(M, B), rho64,
-                          (size_t)M * M * M};
+                const uint32_t nz = (uint32_t)(M * M / (2 * P)), na = (uint32_t)((Mh + B - 1) / B) * M;
+                std::vector<PMBoxDesc> d;
+                std::vector<uint2> vz, va;
+                for (int k = 0; k < copies; ++k) {
+                    d.push_back(PMBoxDesc{M, P, B, pm_stage_plan(M), 1.f, 0.f, 0.f, rho + points * k,
+                                          rho64 + points * k, 1.f, spec + pm_spec_points(M) * k, green, tw});
+                    for (uint32_t i = 0; i < nz; ++i) vz.push_back(make_uint2(k, i));
+                    for (uint32_t i = 0; i < na; ++i) va.push_back(make_uint2(k, i));
+                }
+                cudaMemcpy(dd, d.data(), sizeof(PMBoxDesc) * d.size(), cudaMemcpyHostToDevice);
+                cudaMemcpy(mz, vz.data(), sizeof(uint2) * vz.size(), cudaMemcpyHostToDevice);
+                cudaMemcpy(ma, va.data(), sizeof(uint2) * va.size(), cudaMemcpyHostToDevice);
+                PMMulti m{copies, false, dd, pbeg, mz, ma, (uint32_t)vz.size(), (uint32_t)va.size(),
+                          pm_smem_z(M, P), pm_smem_axis(M, B), rho64, points * copies};
                 m.big = pm_big_fft(M, P, B);
                 if (pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr) != CUCO_OK) continue;  // warm-up
                 cudaEventRecord(e0, stream);
@@ -807,9 +814,10 @@ cuco_status_t cuco_ensemble_get_state(cuco_ensemble_t *e, int box, float *pos, f
             CUCO_TRY(from_fixed(src[k] + b0, e->stage3, nb, e->cfg[box].boxsize, e->stream));
         else
             CUCO_TRY(unpack4to3(src[k] + b0, e->stage3, nb, e->stream));
+        // (the next quantity's unpack is behind this copy on the stream)
         CUCO_TRY_CUDA(cudaMemcpyAsync(dst[k], e->stage3, sizeof(float) * 3 * nb, cudaMemcpyDeviceToHost, e->stream));
-        CUCO_TRY_CUDA(cudaStreamSynchronize(e->stream));
     }
+    CUCO_TRY_CUDA(cudaStreamSynchronize(e->stream));
     return CUCO_OK;
 }
 

@@ -608,44 +608,66 @@ __device__ __forceinline__ void subsort_cell(bool valid, uint32_t c, uint32_t a,
     if (n_cell == 0) put_counts(0);
     const uint32_t gbase = lane - gl;  // the group's first lane
     uint32_t base = 0;                  // lane gl < kZSub: slice gl's next offset in the cell
+    // Chunks are loaded kAhead at a time: a chunk's two dependent loads (the
+    // permutation, then the position) are most of a dense cell's time.
+    constexpr uint32_t kAhead = W == 32 ? 4 : 1;
     if (__any_sync(0xffffffffu, multi)) {
         // cells of more than one chunk count their slices first
-        for (uint32_t j = 0; j < chunks_max; ++j) {
-            const uint32_t i = a + j * W + gl;
-            const uint32_t s = multi && i < b ? z_slice(pos[perm[i]], d, cz, fixed) : (uint32_t)kZSub;
-            const uint32_t b0 = __ballot_sync(0xffffffffu, s & 1), b1 = __ballot_sync(0xffffffffu, s & 2),
-                           b2 = __ballot_sync(0xffffffffu, s & 4), none = __ballot_sync(0xffffffffu, s == kZSub);
-            if (gl < kZSub) base += __popc(lanes_of(gl, b0, b1, b2, none));
+        for (uint32_t j = 0; j < chunks_max; j += kAhead) {
+            uint32_t o[kAhead], s[kAhead];
+#pragma unroll
+            for (uint32_t u = 0; u < kAhead; ++u) {
+                const uint32_t i = a + (j + u) * W + gl;
+                o[u] = multi && i < b ? perm[i] : 0xffffffffu;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kAhead; ++u)
+                s[u] = o[u] != 0xffffffffu ? z_slice(pos[o[u]], d, cz, fixed) : (uint32_t)kZSub;
+#pragma unroll
+            for (uint32_t u = 0; u < kAhead; ++u) {
+                const uint32_t b0 = __ballot_sync(0xffffffffu, s[u] & 1), b1 = __ballot_sync(0xffffffffu, s[u] & 2),
+                               b2 = __ballot_sync(0xffffffffu, s[u] & 4), none = __ballot_sync(0xffffffffu, s[u] == kZSub);
+                if (gl < kZSub) base += __popc(lanes_of(gl, b0, b1, b2, none));
+            }
         }
         const uint32_t incl = scan(base);
         if (multi) put_counts(incl);
         base = incl - base;
     }
-    for (uint32_t j = 0; j < chunks_max; ++j) {
-        const uint32_t i = a + j * W + gl;
-        uint32_t o = 0, s = kZSub;
-        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < b) {
-            o = perm[i];
-            p = pos[o];
-            s = z_slice(p, d, cz, fixed);
+    for (uint32_t j = 0; j < chunks_max; j += kAhead) {
+        uint32_t o[kAhead];
+        float4 p[kAhead];
+#pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u) {
+            const uint32_t i = a + (j + u) * W + gl;
+            o[u] = i < b ? perm[i] : 0u;
         }
-        const uint32_t b0 = __ballot_sync(0xffffffffu, s & 1), b1 = __ballot_sync(0xffffffffu, s & 2),
-                       b2 = __ballot_sync(0xffffffffu, s & 4), none = __ballot_sync(0xffffffffu, s == kZSub);
-        const uint32_t mine = lanes_of(s, b0, b1, b2, none);
-        const uint32_t cnt = gl < kZSub ? __popc(lanes_of(gl, b0, b1, b2, none)) : 0u;
-        const uint32_t incl = scan(cnt);
-        if (!multi && j == 0) {
-            // one chunk: the offsets are the exclusive scan of its counts
-            if (n_cell) put_counts(incl);
-            base = incl - cnt;
+#pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u)
+            p[u] = a + (j + u) * W + gl < b ? pos[o[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (uint32_t u = 0; u < kAhead; ++u) {
+            const bool in = a + (j + u) * W + gl < b;
+            const uint32_t s = in ? z_slice(p[u], d, cz, fixed) : (uint32_t)kZSub;
+            const uint32_t b0 = __ballot_sync(0xffffffffu, s & 1), b1 = __ballot_sync(0xffffffffu, s & 2),
+                           b2 = __ballot_sync(0xffffffffu, s & 4), none = __ballot_sync(0xffffffffu, s == kZSub);
+            const uint32_t mine = lanes_of(s, b0, b1, b2, none);
+            const uint32_t cnt = gl < kZSub ? __popc(lanes_of(gl, b0, b1, b2, none)) : 0u;
+            if (j + u == 0) {
+                // one chunk: the offsets are the exclusive scan of its counts
+                const uint32_t incl = scan(cnt);
+                if (!multi) {
+                    if (n_cell) put_counts(incl);
+                    base = incl - cnt;
+                }
+            }
+            const uint32_t at = __shfl_sync(0xffffffffu, base, gbase + (s & (kZSub - 1))) + __popc(mine & lt);
+            if (in) {
+                sorted_pos[CUCO_IDX(a + at, b)] = make_float4(p[u].x, p[u].y, p[u].z, (float)s);
+                perm_s[CUCO_IDX(a + at, b)] = o[u];
+            }
+            base += cnt;
         }
-        const uint32_t at = __shfl_sync(0xffffffffu, base, gbase + (s & (kZSub - 1))) + __popc(mine & lt);
-        if (i < b) {
-            sorted_pos[CUCO_IDX(a + at, b)] = make_float4(p.x, p.y, p.z, (float)s);
-            perm_s[CUCO_IDX(a + at, b)] = o;
-        }
-        base += cnt;
     }
 }
 
