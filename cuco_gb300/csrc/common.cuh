@@ -287,6 +287,7 @@ struct PMMulti {
     unsigned long long *rho64_all;  // all boxes' deposit grids, contiguous (one memset)
     size_t rho_all_count;
     bool big;  // some box's transforms need the large register kernels (pm_big_fft)
+    bool wide; // some box's stages are wide (pm_wide_stages)
 };
 // Whether a box of mesh M with transform batches P, B takes the large (32-point)
 // register transforms, which run in kernels of their own.
@@ -294,6 +295,8 @@ bool pm_big_fft(int M, int P, int B);
 bool pm_fft_batches_ok(int M, int P, int B);
 // Radices of a mesh's Stockham transform, five bits each.
 uint32_t pm_stage_plan(int M);
+// Whether they need the transforms with radices above 16 (more registers).
+bool pm_wide_stages(uint32_t stages);
 // Points of a mesh's half-spectrum array.
 size_t pm_spec_points(int M);
 int pm_batch_z(int M);

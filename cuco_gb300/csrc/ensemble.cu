@@ -257,6 +257,7 @@ void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out
                 PMMulti m{copies, false, dd, pbeg, mz, ma, (uint32_t)vz.size(), (uint32_t)va.size(),
                           pm_smem_z(M, P), pm_smem_axis(M, B), rho64, points * copies};
                 m.big = pm_big_fft(M, P, B);
+                m.wide = pm_wide_stages(pm_stage_plan(M));
                 if (pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr) != CUCO_OK) continue;  // warm-up
                 cudaEventRecord(e0, stream);
                 for (int r = 0; r < 3; ++r) pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr);
@@ -665,7 +666,11 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
         e->sr_law.assign(srd.begin(), srd.begin() + shortrange_desc_bytes());
     e->pm = PMMulti{nbox, e->fixed, e->d_pm, e->d_pbeg, e->d_mapz, e->d_mapa, (uint32_t)mapz.size(),
                     (uint32_t)mapa.size(), smz, sma, e->rho64, (size_t)mbase[nbox]};
-    for (int b = 0; b < nbox; ++b) e->pm.big = e->pm.big || pm_big_fft(cfg[b].pm_grid, P[b], B[b]);
+    for (int b = 0; b < nbox; ++b) {
+        const int M = cfg[b].pm_grid;
+        e->pm.big = e->pm.big || pm_big_fft(M, P[b], B[b]);
+        e->pm.wide = e->pm.wide || pm_wide_stages(pm_stage_plan(M));
+    }
     e->has_state = e->has_state || carry != nullptr;
     return CUCO_OK;
 }

@@ -46,6 +46,11 @@ namespace {
 constexpr int kFFTThreads = 256;
 constexpr int kLoadBatch = 8;  // global loads issued per thread before use
 
+// complex a + b, a - b: one packed instruction each (every element rounded as
+// the scalar operation rounds it)
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(make_float2(-1.f, -1.f), b, a); }
+
 // Points from one (x, y) row of the half spectrum to the next.  (Rounded up to
 // whole 32-byte sectors the axis passes gained 3 % at M = 512 and the inverse
 // z pass lost a quarter.)
@@ -56,12 +61,21 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
 }
 
 // The stages of a mesh's Stockham transform, largest radix first, five bits
-// each (0 ends): the fewest stages of radix at most 16, of those the smallest
-// radix sum.  Every stage is one round trip through shared memory and one CTA
-// barrier, which is what these passes spend their time on: M = 384 takes 3
-// stages (8 8 6) instead of the 5 of radices 4, 2, 3, and 5; M = 200 3 instead
-// of 4; most meshes to 240 take 2.
-constexpr int kRadices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+// each (0 ends): the fewest stages, of those the smallest radix sum.  Every
+// stage is one round trip through shared memory and one CTA barrier, which is
+// what these passes spend their time on: M = 200 takes 3 (8 5 5) instead of the
+// 4 of radices to 5, most meshes to 240 take 2.  Radices 18 and 24 make it 2
+// for 384 (24 16) and a few others, where 16 and less need 3: the five passes
+// at 384 1.08 -> 0.97 ms.  Their kernels hold 80 registers a thread instead of
+// 64, so only such meshes run them (0.4 % slower at 200 with them compiled in;
+// 200 as 20 10 was 2 % slower than 8 5 5).
+constexpr int kRadices[] = {24, 18, 16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+// Whether a plan has a radix above 16.
+__host__ __device__ __forceinline__ bool wide_plan(uint32_t plan) {
+    for (; plan; plan >>= 5)
+        if ((plan & 31) > 16) return true;
+    return false;
+}
 uint32_t stage_plan(int M) {
     struct Best {
         int stages = 99, sum = 0;
@@ -93,42 +107,37 @@ struct FastDiv {
 template <int R>
 __device__ __forceinline__ void dft_small(float2 (&v)[R], int sign) {
     if (R == 4) {
-        const float2 a0 = make_float2(v[0].x + v[2].x, v[0].y + v[2].y);
-        const float2 a1 = make_float2(v[0].x - v[2].x, v[0].y - v[2].y);
-        const float2 a2 = make_float2(v[1].x + v[3].x, v[1].y + v[3].y);
-        const float2 d = make_float2(v[1].x - v[3].x, v[1].y - v[3].y);
+        const float2 a0 = cadd(v[0], v[2]), a1 = csub(v[0], v[2]), a2 = cadd(v[1], v[3]), d = csub(v[1], v[3]);
         // (v1 - v3) * (sign * i)
         const float2 a3 = sign < 0 ? make_float2(d.y, -d.x) : make_float2(-d.y, d.x);
-        v[0] = make_float2(a0.x + a2.x, a0.y + a2.y);
+        v[0] = cadd(a0, a2);
         v[1] = make_float2(a1.x + a3.x, a1.y + a3.y);
-        v[2] = make_float2(a0.x - a2.x, a0.y - a2.y);
+        v[2] = csub(a0, a2);
         v[3] = make_float2(a1.x - a3.x, a1.y - a3.y);
     } else if (R == 2) {
         const float2 a = v[0], b = v[1];
-        v[0] = make_float2(a.x + b.x, a.y + b.y);
-        v[1] = make_float2(a.x - b.x, a.y - b.y);
+        v[0] = cadd(a, b);
+        v[1] = csub(a, b);
     } else if (R == 3) {
         // y1,2 = v0 - (v1+v2)/2 +- i s (v1-v2), s = sign sqrt(3)/2
         const float s3 = sign * 0.866025403784438647f;
-        const float2 t = make_float2(v[1].x + v[2].x, v[1].y + v[2].y);
-        const float2 d = make_float2(v[1].x - v[2].x, v[1].y - v[2].y);
-        const float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
-        v[0] = make_float2(v[0].x + t.x, v[0].y + t.y);
+        const float2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+        const float2 m = __ffma2_rn(make_float2(-0.5f, -0.5f), t, v[0]);
+        v[0] = cadd(v[0], t);
         v[1] = make_float2(m.x - s3 * d.y, m.y + s3 * d.x);
         v[2] = make_float2(m.x + s3 * d.y, m.y - s3 * d.x);
     } else {
         // five-point DFT by the conjugate pairs (1,4), (2,3)
         const float c1 = 0.309016994374947424f, c2 = -0.809016994374947424f;
         const float s1 = sign * 0.951056516295153572f, s2 = sign * 0.587785252292473129f;
-        const float2 a1 = make_float2(v[1].x + v[R - 1].x, v[1].y + v[R - 1].y);
-        const float2 b1 = make_float2(v[1].x - v[R - 1].x, v[1].y - v[R - 1].y);
-        const float2 a2 = make_float2(v[2].x + v[R - 2].x, v[2].y + v[R - 2].y);
-        const float2 b2 = make_float2(v[2].x - v[R - 2].x, v[2].y - v[R - 2].y);
-        const float2 t1 = make_float2(v[0].x + c1 * a1.x + c2 * a2.x, v[0].y + c1 * a1.y + c2 * a2.y);
-        const float2 t2 = make_float2(v[0].x + c2 * a1.x + c1 * a2.x, v[0].y + c2 * a1.y + c1 * a2.y);
-        const float2 u1 = make_float2(s1 * b1.x + s2 * b2.x, s1 * b1.y + s2 * b2.y);
-        const float2 u2 = make_float2(s2 * b1.x - s1 * b2.x, s2 * b1.y - s1 * b2.y);
-        v[0] = make_float2(v[0].x + a1.x + a2.x, v[0].y + a1.y + a2.y);
+        const float2 a1 = cadd(v[1], v[R - 1]), b1 = csub(v[1], v[R - 1]);
+        const float2 a2 = cadd(v[2], v[R - 2]), b2 = csub(v[2], v[R - 2]);
+        auto dup = [](float c) { return make_float2(c, c); };
+        const float2 t1 = __ffma2_rn(dup(c2), a2, __ffma2_rn(dup(c1), a1, v[0]));
+        const float2 t2 = __ffma2_rn(dup(c1), a2, __ffma2_rn(dup(c2), a1, v[0]));
+        const float2 u1 = __ffma2_rn(dup(s2), b2, __fmul2_rn(dup(s1), b1));
+        const float2 u2 = __ffma2_rn(dup(-s1), b2, __fmul2_rn(dup(s2), b1));
+        v[0] = cadd(cadd(v[0], a1), a2);
         v[1] = make_float2(t1.x - u1.y, t1.y + u1.x);      // t1 + i u1
         v[2] = make_float2(t2.x - u2.y, t2.y + u2.x);      // t2 + i u2
         v[R - 2] = make_float2(t2.x + u2.y, t2.y - u2.x);  // t2 - i u2
@@ -237,7 +246,7 @@ __device__ __forceinline__ void stockham_stage(const float2 *in, float2 *out, co
 // Transform B = 2^bs columns of length M held in x[m*pitch + b] by the stages
 // of `plan`; returns the buffer holding the result.  S = -1: forward (e^{-i}),
 // +1: inverse.
-template <int S>
+template <int S, bool WIDE>
 __device__ float2 *fft_columns(float2 *x, float2 *y, const float2 *tw, int M, uint32_t plan, int bs, int pitch) {
     int Ns = 1;
     float2 *in = x, *out = y;
@@ -256,6 +265,12 @@ __device__ float2 *fft_columns(float2 *x, float2 *y, const float2 *tw, int M, ui
             CUCO_STAGE(10);
             CUCO_STAGE(12);
             CUCO_STAGE(15);
+            case 18:
+                if (WIDE) stockham_stage<18, S>(in, out, tw, M, Ns, bs, pitch);
+                break;
+            case 24:
+                if (WIDE) stockham_stage<24, S>(in, out, tw, M, Ns, bs, pitch);
+                break;
             default: stockham_stage<16, S>(in, out, tw, M, Ns, bs, pitch); break;
 #undef CUCO_STAGE
         }
@@ -316,8 +331,8 @@ template <int N, int S>
 __device__ __forceinline__ void dft_reg(float2 (&v)[N]) {
     if constexpr (N == 2) {
         const float2 a = v[0], b = v[1];
-        v[0] = make_float2(a.x + b.x, a.y + b.y);
-        v[1] = make_float2(a.x - b.x, a.y - b.y);
+        v[0] = cadd(a, b);
+        v[1] = csub(a, b);
     } else if constexpr (N == 4) {
         dft_small<4>(v, S);
     } else {
@@ -649,6 +664,7 @@ __device__ __forceinline__ void fft_axis_reg(float2 *__restrict__ spec, const fl
 
 // rows r0 .. r0+2P-1 of the M^3 real grid (row = x*M + y) -> spectrum rows,
 // as fft_z_r2c_reg
+template <bool WIDE>
 __device__ __forceinline__ void fft_z_r2c(unsigned long long *__restrict__ rho64, float mscale,
                                           float2 *__restrict__ spec, const float2 *tw, int M, uint32_t plan, int P,
                                           int blk) {
@@ -689,7 +705,7 @@ __device__ __forceinline__ void fft_z_r2c(unsigned long long *__restrict__ rho64
         }
     }
     __syncthreads();
-    float2 *res = fft_columns<-1>(x, y, tw_s, M, plan, ilog2(P), pitch);
+    float2 *res = fft_columns<-1, WIDE>(x, y, tw_s, M, plan, ilog2(P), pitch);
     for (int e = threadIdx.x; e < P * half; e += blockDim.x) {
         const int pr = (int)dH.div((uint32_t)e), k = e - pr * half;
         auto put = [&](int k) {
@@ -706,6 +722,7 @@ __device__ __forceinline__ void fft_z_r2c(unsigned long long *__restrict__ rho64
     }
 }
 
+template <bool WIDE>
 __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float *__restrict__ out,
                                           const float2 *tw, int M, uint32_t plan, int P, int blk) {
     extern __shared__ float2 sm[];
@@ -743,7 +760,7 @@ __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float
         }
     }
     __syncthreads();
-    float2 *res = fft_columns<+1>(x, y, tw_s, M, plan, ilog2(P), pitch);
+    float2 *res = fft_columns<+1, WIDE>(x, y, tw_s, M, plan, ilog2(P), pitch);
     for (int e = threadIdx.x; e < P * M; e += blockDim.x) {
         const int pr = (int)dM.div((uint32_t)e), m = e - pr * M;
         const float2 z = res[m * pitch + pr];
@@ -755,6 +772,7 @@ __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float
 // axis 1: y transform for fixed x = by; axis 0: x transform for fixed y = by,
 // with the Green's multiply and inverse transform when green != 0; columns
 // kz0 = bx * B ...
+template <bool WIDE>
 __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2 *tw,
                                          const float *__restrict__ green1d, int M, uint32_t plan, int B, int axis,
                                          int sign, int green, int bx, int by) {
@@ -784,8 +802,8 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
         }
     }
     __syncthreads();
-    float2 *res = sign < 0 ? fft_columns<-1>(x, y, tw_s, M, plan, bsh, pitch)
-                           : fft_columns<+1>(x, y, tw_s, M, plan, bsh, pitch);
+    float2 *res = sign < 0 ? fft_columns<-1, WIDE>(x, y, tw_s, M, plan, bsh, pitch)
+                           : fft_columns<+1, WIDE>(x, y, tw_s, M, plan, bsh, pitch);
     if (green) {
         // res holds the full forward transform: k index m along x, y index o, kz0+b
         const int ky = o <= M / 2 ? o : M - o;
@@ -804,7 +822,7 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
         }
         __syncthreads();
         float2 *other = res == x ? y : x;
-        res = fft_columns<+1>(res, other, tw_s, M, plan, bsh, pitch);
+        res = fft_columns<+1, WIDE>(res, other, tw_s, M, plan, bsh, pitch);
     }
     for (int e = threadIdx.x; e < M * B; e += blockDim.x) {
         const int m = e >> bsh, b = e & (B - 1);
@@ -812,21 +830,24 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
     }
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kFFTThreads)
     k_fft_z_r2c(unsigned long long *__restrict__ rho64, float mscale, float2 *__restrict__ spec,
                 const float2 *tw, int M, uint32_t plan, int P) {
-    fft_z_r2c(rho64, mscale, spec, tw, M, plan, P, blockIdx.x);
+    fft_z_r2c<WIDE>(rho64, mscale, spec, tw, M, plan, P, blockIdx.x);
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kFFTThreads)
     k_fft_z_c2r(const float2 *__restrict__ spec, float *__restrict__ out, const float2 *tw, int M, uint32_t plan, int P) {
-    fft_z_c2r(spec, out, tw, M, plan, P, blockIdx.x);
+    fft_z_c2r<WIDE>(spec, out, tw, M, plan, P, blockIdx.x);
 }
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kFFTThreads)
     k_fft_axis(float2 *__restrict__ spec, const float2 *tw, const float *__restrict__ green1d, int M,
                uint32_t plan, int B, int axis, int sign, int green) {
-    fft_axis(spec, tw, green1d, M, plan, B, axis, sign, green, blockIdx.x, blockIdx.y);
+    fft_axis<WIDE>(spec, tw, green1d, M, plan, B, axis, sign, green, blockIdx.x, blockIdx.y);
 }
 
 // fft_axis_reg for one box, with the batch B a compile-time constant
@@ -950,7 +971,7 @@ __device__ __forceinline__ bool big_box(const PMBoxDesc &d, int cols) {
     return d.M >= 512 && reg_fft_ok(d.M, cols);
 }
 
-template <bool BIG>
+template <bool BIG, bool WIDE>
 __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
     k_fft_z_r2c_multi(const PMBoxDesc *__restrict__ boxes, const uint2 *__restrict__ map) {
     const uint2 m = map[blockIdx.x];
@@ -970,11 +991,11 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
             default: fft_z_r2c_reg<RegFFT<16, 16>>(d.rho64, d.mscale, d.spec, d.twiddle, d.P, m.y); break;
         }
     } else {
-        fft_z_r2c(d.rho64, d.mscale, d.spec, d.twiddle, d.M, d.stages, d.P, m.y);
+        fft_z_r2c<WIDE>(d.rho64, d.mscale, d.spec, d.twiddle, d.M, d.stages, d.P, m.y);
     }
 }
 
-template <bool BIG>
+template <bool BIG, bool WIDE>
 __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
     k_fft_z_c2r_multi(const PMBoxDesc *__restrict__ boxes, const uint2 *__restrict__ map) {
     const uint2 m = map[blockIdx.x];
@@ -994,11 +1015,11 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
             default: fft_z_c2r_reg<RegFFT<16, 16>>(d.spec, d.rho, d.twiddle, d.P, m.y); break;
         }
     } else {
-        fft_z_c2r(d.spec, d.rho, d.twiddle, d.M, d.stages, d.P, m.y);
+        fft_z_c2r<WIDE>(d.spec, d.rho, d.twiddle, d.M, d.stages, d.P, m.y);
     }
 }
 
-template <bool BIG>
+template <bool BIG, bool WIDE>
 __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
     k_fft_axis_multi(const PMBoxDesc *__restrict__ boxes, const uint2 *__restrict__ map, int axis, int sign,
                      int green) {
@@ -1021,7 +1042,7 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
             default: fft_axis_reg<RegFFT<16, 16>>(d.spec, d.twiddle, d.green1d, d.B, axis, sign, green, bx, by); break;
         }
     } else {
-        fft_axis(d.spec, d.twiddle, d.green1d, d.M, d.stages, d.B, axis, sign, green, bx, by);
+        fft_axis<WIDE>(d.spec, d.twiddle, d.green1d, d.M, d.stages, d.B, axis, sign, green, bx, by);
     }
 }
 
@@ -1251,6 +1272,7 @@ bool pm_fft_batches_ok(int M, int P, int B) {
     return !pow2 || (reg_fft_ok(M, P) && reg_fft_ok(M, B));
 }
 
+bool pm_wide_stages(uint32_t stages) { return wide_plan(stages); }
 size_t pm_spec_points(int M) { return (size_t)M * M * spec_stride(M); }
 uint32_t pm_stage_plan(int M) { return stage_plan(M); }
 int pm_batch_z(int M) { return fft_batch_z(M); }
@@ -1286,14 +1308,10 @@ cuco_status_t pm_forces_multi(const PMMulti &m, const float4 *pos, uint32_t n, f
                               cudaStream_t stream, int *launches) {
     static bool attr = [] {
         const int mx = 227 * 1024;
-        for (bool big : {false, true}) {
-            cudaFuncSetAttribute(big ? k_fft_z_r2c_multi<true> : k_fft_z_r2c_multi<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-            cudaFuncSetAttribute(big ? k_fft_z_c2r_multi<true> : k_fft_z_c2r_multi<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-            cudaFuncSetAttribute(big ? k_fft_axis_multi<true> : k_fft_axis_multi<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        }
+        auto set = [&](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx); };
+        set(k_fft_z_r2c_multi<true, false>), set(k_fft_z_c2r_multi<true, false>), set(k_fft_axis_multi<true, false>);
+        set(k_fft_z_r2c_multi<false, false>), set(k_fft_z_c2r_multi<false, false>), set(k_fft_axis_multi<false, false>);
+        set(k_fft_z_r2c_multi<false, true>), set(k_fft_z_c2r_multi<false, true>), set(k_fft_axis_multi<false, true>);
         return true;
     }();
     (void)attr;
@@ -1306,18 +1324,20 @@ cuco_status_t pm_forces_multi(const PMMulti &m, const float4 *pos, uint32_t n, f
     }
     // each pass: the boxes of the common kernels, then (when the ensemble has
     // any) the boxes of the large register transforms
-    k_fft_z_r2c_multi<false><<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
-    if (m.big) k_fft_z_r2c_multi<true><<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
+    const auto r2c = m.wide ? k_fft_z_r2c_multi<false, true> : k_fft_z_r2c_multi<false, false>;
+    const auto c2r = m.wide ? k_fft_z_c2r_multi<false, true> : k_fft_z_c2r_multi<false, false>;
+    const auto along = m.wide ? k_fft_axis_multi<false, true> : k_fft_axis_multi<false, false>;
+    r2c<<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
+    if (m.big) k_fft_z_r2c_multi<true, false><<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
     for (int pass = 0; pass < 3; ++pass) {
         const int axis = pass == 1 ? 0 : 1, sign = pass == 2 ? +1 : -1, green = pass == 1;
-        k_fft_axis_multi<false><<<m.naxis_blocks, kFFTThreads, m.sma, stream>>>(m.boxes, m.map_axis, axis, sign,
-                                                                                green);
+        along<<<m.naxis_blocks, kFFTThreads, m.sma, stream>>>(m.boxes, m.map_axis, axis, sign, green);
         if (m.big)
-            k_fft_axis_multi<true><<<m.naxis_blocks, kFFTThreads, m.sma, stream>>>(m.boxes, m.map_axis, axis, sign,
+            k_fft_axis_multi<true, false><<<m.naxis_blocks, kFFTThreads, m.sma, stream>>>(m.boxes, m.map_axis, axis, sign,
                                                                                    green);
     }
-    k_fft_z_c2r_multi<false><<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
-    if (m.big) k_fft_z_c2r_multi<true><<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
+    c2r<<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
+    if (m.big) k_fft_z_c2r_multi<true, false><<<m.nz_blocks, kFFTThreads, m.smz, stream>>>(m.boxes, m.map_z);
     if (n) {
         if (m.fixed)
             k_interp_multi<true><<<(n + 255) / 256, 256, 0, stream>>>(pos, n, m.boxes, m.pbeg, m.nbox, acc);
@@ -1388,11 +1408,12 @@ cuco_status_t pm_plan_create(PMPlan *plan, int M, float boxsize, float asmth, fl
         return CUCO_ERR_UNSUPPORTED;
     }
     static const cudaError_t attr = [] {
-        cudaError_t e = cudaFuncSetAttribute(k_fft_z_r2c, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fft_z_c2r, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_fft_axis, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        cudaError_t e = cudaSuccess;
+        auto set = [&](auto kernel) {
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+        };
+        set(k_fft_z_r2c<false>), set(k_fft_z_c2r<false>), set(k_fft_axis<false>);
+        set(k_fft_z_r2c<true>), set(k_fft_z_c2r<true>), set(k_fft_axis<true>);
         return e;
     }();
     CUCO_TRY_CUDA(attr);
@@ -1447,13 +1468,17 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, const uint32_t *perm, u
         CUCO_TRY_CUDA(e);
     } else {
         const unsigned zblocks = (unsigned)((size_t)M * M / (2 * P));
-        k_fft_z_r2c<<<zblocks, kFFTThreads, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
+        const bool wide = wide_plan(plan.stages);
+        const auto r2c = wide ? k_fft_z_r2c<true> : k_fft_z_r2c<false>;
+        const auto along = wide ? k_fft_axis<true> : k_fft_axis<false>;
+        const auto c2r = wide ? k_fft_z_c2r<true> : k_fft_z_c2r<false>;
+        r2c<<<zblocks, kFFTThreads, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
                                                            plan.twiddle, M, plan.stages, P);
         dim3 ag((Mh + B - 1) / B, M);
-        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, -1, 0);
-        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 0, -1, 1);
-        k_fft_axis<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, +1, 0);
-        k_fft_z_c2r<<<zblocks, kFFTThreads, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, M, plan.stages, P);
+        along<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, -1, 0);
+        along<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 0, -1, 1);
+        along<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, +1, 0);
+        c2r<<<zblocks, kFFTThreads, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, M, plan.stages, P);
         CUCO_TRY_CUDA(cudaGetLastError());
     }
     plan.rho64_dirty = false;
