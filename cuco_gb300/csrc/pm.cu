@@ -1097,7 +1097,7 @@ __device__ __forceinline__ unsigned long long weight_u64(float w) {
 // adds its own weights directly.  Integer sums are associative, so the grid
 // is the same either way, bit for bit.  Called by every active lane of the
 // warp together.
-template <bool FIXED>
+template <bool FIXED, bool MANY>
 __device__ __forceinline__ void deposit_one(float4 p, unsigned long long *__restrict__ rho64, int M,
                                             float to_slab_fac) {
     int s[3][2];
@@ -1113,7 +1113,17 @@ __device__ __forceinline__ void deposit_one(float4 p, unsigned long long *__rest
                                weight_u64(m1 * (1.f - dy) * dz),        weight_u64(m1 * dy * dz)};
     const unsigned active = __activemask(), lane = threadIdx.x & 31;
     const unsigned cell = ((unsigned)sx * (unsigned)M + (unsigned)sy) * (unsigned)M + (unsigned)sz;
-    const unsigned peers = __match_any_sync(active, cell);
+    unsigned peers;
+    bool mixed = false;  // a warp whose lanes hold particles of two boxes
+    if (MANY) {
+        int same;
+        __match_all_sync(active, (unsigned long long)rho64, &same);
+        mixed = !same;
+    }
+    if (mixed)
+        peers = 1u << lane;  // (equal cells of different boxes are not the same cell)
+    else
+        peers = __match_any_sync(active, cell);
     bool lead = true;
     if (!__all_sync(active, peers == (1u << lane))) {
         // sum the group's weights into its lowest lane (every member runs the
@@ -1206,7 +1216,7 @@ template <bool FIXED>
 __global__ void k_deposit(const float4 *__restrict__ pos, uint32_t n, unsigned long long *__restrict__ rho64,
                           int M, float to_slab_fac) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) deposit_one<FIXED>(pos[i], rho64, M, to_slab_fac);
+    if (i < n) deposit_one<FIXED, false>(pos[i], rho64, M, to_slab_fac);
 }
 
 // perm (or null): where each result goes, for positions in cell order
@@ -1224,7 +1234,7 @@ __global__ void k_deposit_multi(const float4 *__restrict__ pos, uint32_t n, cons
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const PMBoxDesc &d = boxes[find_box(pbeg, nbox, i)];
-    deposit_one<FIXED>(pos[i], d.rho64, d.M, d.to_slab_fac);
+    deposit_one<FIXED, true>(pos[i], d.rho64, d.M, d.to_slab_fac);
 }
 
 template <bool FIXED>
