@@ -60,16 +60,23 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// The stages of a mesh's Stockham transform, largest radix first, five bits
-// each (0 ends): the fewest stages, of those the smallest radix sum.  Every
-// stage is one round trip through shared memory and one CTA barrier, which is
-// what these passes spend their time on: M = 200 takes 3 (8 5 5) instead of the
-// 4 of radices to 5, most meshes to 240 take 2.  Radices 18 and 24 make it 2
-// for 384 (24 16) and a few others, where 16 and less need 3: the five passes
-// at 384 1.08 -> 0.97 ms.  Their kernels hold 80 registers a thread instead of
-// 64, so only such meshes run them (0.4 % slower at 200 with them compiled in;
-// 200 as 20 10 was 2 % slower than 8 5 5).
-constexpr int kRadices[] = {24, 18, 16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+// The stages of a mesh's Stockham transform, five bits each (0 ends): the
+// fewest stages, of those the ones with the most factors of two in a single
+// radix, which goes first, of those the smallest radix sum.  Every stage is one
+// round trip through shared memory and one CTA barrier, which is what these
+// passes spend their time on: M = 200 takes 3 (8 5 5) instead of the 4 of
+// radices to 5, most meshes to 240 take 2.  Radices 18 and 24 make it 2 for 384
+// (16 24) and a few others, where 16 and less need 3: the five passes at 384
+// 1.08 -> 0.97 ms.  Their kernels hold 80 registers a thread instead of 64, so
+// only such meshes run them (0.4 % slower at 200 with them compiled in; 200 as
+// 20 10 was 2 % slower than 8 5 5).
+//
+// The factors of two go first for the rounding: the mesh of a hardly displaced
+// lattice is large harmonics of the lattice that cancel, and radices 4 and 2
+// take their sums before any twiddle.  Against 64 bits, over 20 such states of
+// 18^3 on 36^3, the largest error relative to that of 4 3 3 (and the mean):
+// 6 6 1.42 (1.03), 9 4 1.36 (1.05), 4 9 1.03 (0.99).
+constexpr int kRadices[] = {24, 18, 16, 15, 12, 10, 9, 8, 6, 5, 4, 3};  // (no even mesh to 1024 wants a 2)
 // Whether a plan has a radix above 16.
 __host__ __device__ __forceinline__ bool wide_plan(uint32_t plan) {
     for (; plan; plan >>= 5)
@@ -77,22 +84,38 @@ __host__ __device__ __forceinline__ bool wide_plan(uint32_t plan) {
     return false;
 }
 uint32_t stage_plan(int M) {
-    struct Best {
-        int stages = 99, sum = 0;
-        uint32_t plan = 0;
-    } best;
-    auto search = [&](auto &&self, int rem, int from, int stages, int sum, uint32_t plan) -> void {
+    constexpr int kMaxStages = 6;
+    struct Plan {
+        int stages = 0, twos = 0, sum = 0, radix[kMaxStages] = {};
+    } best, cur;
+    best.stages = kMaxStages + 1;
+    auto search = [&](auto &&self, int rem, int from) -> void {
         if (rem == 1) {
-            if (stages < best.stages || (stages == best.stages && sum < best.sum)) best = {stages, sum, plan};
+            if (cur.stages != best.stages ? cur.stages < best.stages
+                                          : (cur.twos != best.twos ? cur.twos > best.twos : cur.sum < best.sum))
+                best = cur;
             return;
         }
-        if (stages == 6) return;
-        for (int i = from; i < (int)(sizeof kRadices / sizeof kRadices[0]); ++i)
-            if (rem % kRadices[i] == 0)
-                self(self, rem / kRadices[i], i, stages + 1, sum + kRadices[i], plan | (uint32_t)kRadices[i] << (5 * stages));
+        if (cur.stages == kMaxStages) return;
+        for (int i = from; i < (int)(sizeof kRadices / sizeof kRadices[0]); ++i) {
+            const int R = kRadices[i];
+            if (rem % R) continue;
+            const Plan before = cur;
+            cur.radix[cur.stages++] = R;
+            cur.sum += R;
+            cur.twos = std::max(cur.twos, R & -R);
+            self(self, rem / R, i);
+            cur = before;
+        }
     };
-    search(search, M, 0, 0, 0, 0u);
-    return best.plan;
+    search(search, M, 0);
+    // the radix with the most factors of two first, the others largest first
+    int first = 0;
+    while (first < best.stages && (best.radix[first] & -best.radix[first]) != best.twos) ++first;
+    uint32_t plan = first < best.stages ? (uint32_t)best.radix[first] : 0u;
+    for (int k = 0, at = 5; k < best.stages; ++k)
+        if (k != first) plan |= (uint32_t)best.radix[k] << at, at += 5;
+    return plan;
 }
 
 // Division by a runtime d without a divide instruction: j / d is
@@ -255,7 +278,6 @@ __device__ float2 *fft_columns(float2 *x, float2 *y, const float2 *tw, int M, ui
         switch (r) {
 #define CUCO_STAGE(R) \
     case R: stockham_stage<R, S>(in, out, tw, M, Ns, bs, pitch); break
-            CUCO_STAGE(2);
             CUCO_STAGE(3);
             CUCO_STAGE(4);
             CUCO_STAGE(5);
