@@ -70,6 +70,34 @@ uint32_t bounds_violations_sort();
 uint32_t bounds_violations_pm();
 uint32_t bounds_violations_shortrange();
 
+// ------------------------------------------------------- chained launches
+
+// A kernel launched by launch_chained may start while the kernel before it on
+// the stream still runs, once every block of that one has called chain_next()
+// or ended: its launch and its constant tables' loads then cost nothing.  It
+// calls chain_wait(), in every block, before it touches anything another kernel
+// writes or reads; that returns when the kernel before it (and so, as that one
+// waited too, every kernel before) has completed.  Both do nothing in a plain
+// launch (`chain` false).
+__device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void chain_next() { cudaTriggerProgrammaticLaunchCompletion(); }
+
+template <typename... P, typename... A>
+cudaError_t launch_chained(bool chain, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                           A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = chain ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // -------------------------------------------------------------- sorting
 
 // Scratch a sort of n keys needs: alternate key/value buffers and the per-tile

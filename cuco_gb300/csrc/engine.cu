@@ -34,6 +34,7 @@ namespace {
 __global__ void k_drift_keys(float4 *__restrict__ pos, const float4 *__restrict__ vel,
                              double drift, float boxsize, int do_drift,
                              uint32_t *__restrict__ keys, uint32_t n, float gridfac, int G) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float4 p = pos[i];
@@ -74,6 +75,7 @@ __global__ void k_drift_keys(float4 *__restrict__ pos, const float4 *__restrict_
 __global__ void k_drift_keys_fixed(float4 *__restrict__ pos, const float4 *__restrict__ vel,
                                    float units_per_time, int do_drift, uint32_t *__restrict__ keys,
                                    uint32_t n, int G) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
@@ -243,9 +245,9 @@ cuco_status_t launch_drift_keys(float4 *pos, const float4 *vel, double drift, fl
                                 bool do_drift, uint32_t *keys, uint32_t n, float gridfac, int G,
                                 cudaStream_t stream) {
     if (!n) return CUCO_OK;
-    k_drift_keys<<<(n + 255) / 256, 256, 0, stream>>>(pos, vel, drift, boxsize, do_drift ? 1 : 0,
-                                                      keys, n, gridfac, G);
-    CUCO_TRY_CUDA(cudaGetLastError());
+    // (chained to the short range of the step before)
+    CUCO_TRY_CUDA(launch_chained(true, k_drift_keys, (n + 255) / 256, 256, 0, stream, pos, vel, drift, boxsize,
+                                 do_drift ? 1 : 0, keys, n, gridfac, G));
     return CUCO_OK;
 }
 
@@ -253,8 +255,8 @@ cuco_status_t launch_drift_keys_fixed(float4 *pos, const float4 *vel, double dri
                                       bool do_drift, uint32_t *keys, uint32_t n, int G, cudaStream_t stream) {
     if (!n) return CUCO_OK;
     const float upt = (float)(drift * 4294967296.0 / (double)boxsize);
-    k_drift_keys_fixed<<<(n + 255) / 256, 256, 0, stream>>>(pos, vel, upt, do_drift ? 1 : 0, keys, n, G);
-    CUCO_TRY_CUDA(cudaGetLastError());
+    CUCO_TRY_CUDA(launch_chained(true, k_drift_keys_fixed, (n + 255) / 256, 256, 0, stream, pos, vel, upt,
+                                 do_drift ? 1 : 0, keys, n, G));
     return CUCO_OK;
 }
 

@@ -517,6 +517,7 @@ __device__ __forceinline__ void fft_z_r2c_reg(unsigned long long *__restrict__ r
     float2 *x = sm, *tw_s = sm + FT::ROWS * pitch;
     const size_t r0 = (size_t)blk * 2 * P;
     load_twiddles(tw_s, tw, M);
+    chain_wait();
     // rows 2pr and 2pr+1 packed as one complex column, two points a thread
     // and load; every sum read is cleared for the next deposit
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
@@ -549,6 +550,7 @@ __device__ __forceinline__ void fft_z_r2c_reg(unsigned long long *__restrict__ r
     }
     __syncthreads();
     FT::template forward<-1>(x, tw_s, pitch, ilog2(P));
+    chain_next();
     // both rows of a pair from the same two transform values, consecutive k
     for (int e = threadIdx.x; e < P * (M / 2); e += blockDim.x) {
         const int pr = e / (M / 2), k = e & (M / 2 - 1);
@@ -575,6 +577,7 @@ __device__ __forceinline__ void fft_z_c2r_reg(const float2 *__restrict__ spec, f
     float2 *x = sm, *tw_s = sm + FT::ROWS * pitch;
     const size_t r0 = (size_t)blk * 2 * P;
     load_twiddles(tw_s, tw, M);
+    chain_wait();
     // row pair pr packed as one complex column a + i b (a, b the Hermitian
     // rows 2pr and 2pr+1, imaginary parts at k = 0 and M/2 dropped), placed
     // in the slot order the inverse transform starts from: a pair's values at
@@ -608,6 +611,7 @@ __device__ __forceinline__ void fft_z_c2r_reg(const float2 *__restrict__ spec, f
     }
     __syncthreads();
     FT::template inverse<+1>(x, tw_s, pitch, ilog2(P));
+    chain_next();
     // the pair's two real rows from one transform value
     for (int e = threadIdx.x; e < P * M; e += blockDim.x) {
         const int pr = e / M, m = e & (M - 1);
@@ -650,6 +654,7 @@ __device__ __forceinline__ void fft_axis_reg(float2 *__restrict__ spec, const fl
     // an inverse-only pass starts from the slot order
     const bool to_slots = sign > 0;
     load_twiddles(tw_s, tw, M);
+    chain_wait();
     for (int e0 = threadIdx.x; e0 < M * B; e0 += kLoadBatch * blockDim.x) {
         float2 v[kLoadBatch];
 #pragma unroll
@@ -697,6 +702,7 @@ __device__ __forceinline__ void fft_z_r2c(unsigned long long *__restrict__ rho64
     const size_t r0 = (size_t)blk * 2 * P;
     const FastDiv dH((uint32_t)half);
     load_twiddles(tw_s, tw, M);
+    chain_wait();
     const ulonglong2 zero = make_ulonglong2(0ull, 0ull);
     for (int e0 = threadIdx.x; e0 < P * half; e0 += kBatch * blockDim.x) {
         ulonglong2 a[kBatch], c[kBatch];
@@ -728,6 +734,7 @@ __device__ __forceinline__ void fft_z_r2c(unsigned long long *__restrict__ rho64
     }
     __syncthreads();
     float2 *res = fft_columns<-1, WIDE>(x, y, tw_s, M, plan, ilog2(P), pitch);
+    chain_next();
     for (int e = threadIdx.x; e < P * half; e += blockDim.x) {
         const int pr = (int)dH.div((uint32_t)e), k = e - pr * half;
         auto put = [&](int k) {
@@ -753,6 +760,7 @@ __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float
     const size_t r0 = (size_t)blk * 2 * P;
     const FastDiv dH((uint32_t)half), dM((uint32_t)M);
     load_twiddles(tw_s, tw, M);
+    chain_wait();
     for (int e0 = threadIdx.x; e0 < P * half; e0 += kLoadBatch * blockDim.x) {
         float2 a[kLoadBatch], b[kLoadBatch];
 #pragma unroll
@@ -783,6 +791,7 @@ __device__ __forceinline__ void fft_z_c2r(const float2 *__restrict__ spec, float
     }
     __syncthreads();
     float2 *res = fft_columns<+1, WIDE>(x, y, tw_s, M, plan, ilog2(P), pitch);
+    chain_next();
     for (int e = threadIdx.x; e < P * M; e += blockDim.x) {
         const int pr = (int)dM.div((uint32_t)e), m = e - pr * M;
         const float2 z = res[m * pitch + pr];
@@ -809,6 +818,7 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
     const size_t sm_stride = axis == 1 ? (size_t)spec_stride(M) : (size_t)M * spec_stride(M);
     const size_t base = (size_t)o * (axis == 1 ? M : 1) * spec_stride(M);
     load_twiddles(tw_s, tw, M);
+    chain_wait();
     for (int e0 = threadIdx.x; e0 < M * B; e0 += kLoadBatch * blockDim.x) {
         float2 v[kLoadBatch];
 #pragma unroll
@@ -846,6 +856,7 @@ __device__ __forceinline__ void fft_axis(float2 *__restrict__ spec, const float2
         float2 *other = res == x ? y : x;
         res = fft_columns<+1, WIDE>(res, other, tw_s, M, plan, bsh, pitch);
     }
+    chain_next();
     for (int e = threadIdx.x; e < M * B; e += blockDim.x) {
         const int m = e >> bsh, b = e & (B - 1);
         if (b < nb) spec[base + m * sm_stride + kz0 + b] = res[m * pitch + b];
@@ -895,6 +906,7 @@ __device__ __forceinline__ void fft_axis_reg_fixed(float2 *__restrict__ spec, co
     // an inverse-only pass starts from the slot order
     const bool to_slots = sign > 0;
     load_twiddles(tw_s, tw, M);
+    chain_wait();
 #pragma unroll
     for (int j0 = 0; j0 < per; j0 += kLoadBatch) {
         float2 v[kLoadBatch];
@@ -918,6 +930,7 @@ __device__ __forceinline__ void fft_axis_reg_fixed(float2 *__restrict__ spec, co
     } else {
         FT::template inverse<+1>(x, tw_s, B, bsh);
     }
+    chain_next();
     if (valid) {
 #pragma unroll 4
         for (int j = 0; j < per; ++j) {
@@ -963,7 +976,7 @@ __global__ void __launch_bounds__(kFFTThreads, M1 * M2 >= 512 ? 2 : 4)
 
 // The five transform passes of one box with the register transforms.
 template <int M1, int M2>
-cudaError_t fft_passes_reg(const PMPlan &plan, int P, cudaStream_t stream) {
+cuco_status_t fft_passes_reg(const PMPlan &plan, int P, bool chain, cudaStream_t stream) {
     constexpr int M = M1 * M2, Mh = M / 2 + 1, B = axis_batch(M);
     // the transform buffer and the twiddles
     constexpr int rows = RegFFT<M1, M2>::ROWS, zt = z_threads(M1, M2);
@@ -976,14 +989,18 @@ cudaError_t fft_passes_reg(const PMPlan &plan, int P, cudaStream_t stream) {
     }();
     (void)attr;
     const unsigned zblocks = (unsigned)((size_t)M * M / (2 * P));
-    k_fft_z_r2c_r<M1, M2><<<zblocks, zt, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
-                                                                 plan.twiddle, P);
+    CUCO_TRY_CUDA(launch_chained(chain, k_fft_z_r2c_r<M1, M2>, zblocks, zt, smz, stream, plan.rho64,
+                                 ldexpf(plan.mass, -32), plan.spec, plan.twiddle, P));
     dim3 ag((Mh + B - 1) / B, M);
-    k_fft_axis_r<M1, M2><<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, 1, -1, 0);
-    k_fft_axis_r<M1, M2><<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, 0, -1, 1);
-    k_fft_axis_r<M1, M2><<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, 1, +1, 0);
-    k_fft_z_c2r_r<M1, M2><<<zblocks, zt, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, P);
-    return cudaGetLastError();
+    CUCO_TRY_CUDA(launch_chained(chain, k_fft_axis_r<M1, M2>, ag, kFFTThreads, sma, stream, plan.spec, plan.twiddle,
+                                 plan.green1d, 1, -1, 0));
+    CUCO_TRY_CUDA(launch_chained(chain, k_fft_axis_r<M1, M2>, ag, kFFTThreads, sma, stream, plan.spec, plan.twiddle,
+                                 plan.green1d, 0, -1, 1));
+    CUCO_TRY_CUDA(launch_chained(chain, k_fft_axis_r<M1, M2>, ag, kFFTThreads, sma, stream, plan.spec, plan.twiddle,
+                                 plan.green1d, 1, +1, 0));
+    CUCO_TRY_CUDA(launch_chained(chain, k_fft_z_c2r_r<M1, M2>, zblocks, zt, smz, stream, plan.spec, plan.rho,
+                                 plan.twiddle, P));
+    return CUCO_OK;
 }
 
 // Many boxes in one launch: map[blockIdx.x] = (box, the box's own block
@@ -1263,6 +1280,7 @@ __device__ __forceinline__ float4 interp_one(float4 p, const float *__restrict__
 template <bool FIXED>
 __global__ void k_deposit(const float4 *__restrict__ pos, uint32_t n, unsigned long long *__restrict__ rho64,
                           int M, float to_slab_fac) {
+    chain_next();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) deposit_one<FIXED, false>(pos[i], rho64, M, to_slab_fac);
 }
@@ -1272,6 +1290,7 @@ template <bool FIXED>
 __global__ void k_interp(const float4 *__restrict__ pos, const uint32_t *__restrict__ perm, uint32_t n,
                          const float *__restrict__ phi, int M, float to_slab_fac, float fac,
                          float4 *__restrict__ acc) {
+    chain_wait();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) acc[perm ? perm[i] : i] = interp_one<FIXED>(pos[i], phi, M, to_slab_fac, fac);
 }
@@ -1489,6 +1508,15 @@ void pm_plan_destroy(PMPlan *plan) {
     plan->spec = nullptr;
 }
 
+// Meshes below this launch the PM's kernels after the deposit chained
+// (launch_chained): ten steps of 24^3 to 64^3 particles on twice the mesh take
+// 745 -> 590, 745 -> 605, 1060 -> 900, 1300 -> 1185 and 1930 -> 1800 us, 80^3
+// and 100^3 3655 -> 3455 and 6335 -> 6175; at 128^3 on 256^3 their launches
+// are nothing beside the kernels, and the blocks that wait take places from
+// the sort's (10.81 -> 10.83 ms).  A block lets the next kernel start when it
+// begins its stores: as it ended its loads, 100^3 clustered lost 3 %.
+constexpr int kChainMaxMesh = 256;
+
 cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, const uint32_t *perm, uint32_t n, float4 *acc,
                         cudaStream_t stream, cudaEvent_t *ev_deposit_done, cudaEvent_t *ev_fft_done,
                         int *launches) {
@@ -1501,6 +1529,7 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, const uint32_t *perm, u
     // The z r2c pass clears the sums it reads, so the grid is zero again when
     // the previous call enqueued its passes; otherwise (first call, or a call
     // that stopped at an error) it is cleared here.
+    const bool chain = M < kChainMaxMesh;
     if (plan.rho64_dirty)
         CUCO_TRY_CUDA(cudaMemsetAsync(plan.rho64, 0, sizeof(unsigned long long) * (size_t)M * M * M, stream));
     plan.rho64_dirty = true;
@@ -1513,39 +1542,45 @@ cuco_status_t pm_forces(PMPlan &plan, const float4 *pos, const uint32_t *perm, u
     CUCO_TRY_CUDA(cudaGetLastError());
     if (ev_deposit_done) CUCO_TRY_CUDA(cudaEventRecord(*ev_deposit_done, stream));
     if (reg_fft_ok(M, P) && reg_fft_ok(M, B)) {
-        cudaError_t e;
+        cuco_status_t s;
         switch (M) {
-            case 16: e = fft_passes_reg<4, 4>(plan, P, stream); break;
-            case 32: e = fft_passes_reg<4, 8>(plan, P, stream); break;
-            case 64: e = fft_passes_reg<8, 8>(plan, P, stream); break;
-            case 128: e = fft_passes_reg<8, 16>(plan, P, stream); break;
-            case 256: e = fft_passes_reg<16, 16>(plan, P, stream); break;
-            case 512: e = fft_passes_reg<16, 32>(plan, P, stream); break;
-            default: e = fft_passes_reg<32, 32>(plan, P, stream); break;
+            case 16: s = fft_passes_reg<4, 4>(plan, P, chain, stream); break;
+            case 32: s = fft_passes_reg<4, 8>(plan, P, chain, stream); break;
+            case 64: s = fft_passes_reg<8, 8>(plan, P, chain, stream); break;
+            case 128: s = fft_passes_reg<8, 16>(plan, P, chain, stream); break;
+            case 256: s = fft_passes_reg<16, 16>(plan, P, chain, stream); break;
+            case 512: s = fft_passes_reg<16, 32>(plan, P, chain, stream); break;
+            default: s = fft_passes_reg<32, 32>(plan, P, chain, stream); break;
         }
-        CUCO_TRY_CUDA(e);
+        CUCO_TRY(s);
     } else {
         const unsigned zblocks = (unsigned)((size_t)M * M / (2 * P));
         const bool wide = wide_plan(plan.stages);
         const auto r2c = wide ? k_fft_z_r2c<true> : k_fft_z_r2c<false>;
         const auto along = wide ? k_fft_axis<true> : k_fft_axis<false>;
         const auto c2r = wide ? k_fft_z_c2r<true> : k_fft_z_c2r<false>;
-        r2c<<<zblocks, kFFTThreads, smz, stream>>>(plan.rho64, ldexpf(plan.mass, -32), plan.spec,
-                                                           plan.twiddle, M, plan.stages, P);
+        CUCO_TRY_CUDA(launch_chained(chain, r2c, zblocks, kFFTThreads, smz, stream, plan.rho64, ldexpf(plan.mass,
+                                     -32), plan.spec, plan.twiddle, M, plan.stages, P));
         dim3 ag((Mh + B - 1) / B, M);
-        along<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, -1, 0);
-        along<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 0, -1, 1);
-        along<<<ag, kFFTThreads, sma, stream>>>(plan.spec, plan.twiddle, plan.green1d, M, plan.stages, B, 1, +1, 0);
-        c2r<<<zblocks, kFFTThreads, smz, stream>>>(plan.spec, plan.rho, plan.twiddle, M, plan.stages, P);
+        CUCO_TRY_CUDA(launch_chained(chain, along, ag, kFFTThreads, sma, stream, plan.spec, plan.twiddle,
+                                     plan.green1d, M, plan.stages, B, 1, -1, 0));
+        CUCO_TRY_CUDA(launch_chained(chain, along, ag, kFFTThreads, sma, stream, plan.spec, plan.twiddle,
+                                     plan.green1d, M, plan.stages, B, 0, -1, 1));
+        CUCO_TRY_CUDA(launch_chained(chain, along, ag, kFFTThreads, sma, stream, plan.spec, plan.twiddle,
+                                     plan.green1d, M, plan.stages, B, 1, +1, 0));
+        CUCO_TRY_CUDA(launch_chained(chain, c2r, zblocks, kFFTThreads, smz, stream, plan.spec, plan.rho,
+                                     plan.twiddle, M, plan.stages, P));
         CUCO_TRY_CUDA(cudaGetLastError());
     }
     plan.rho64_dirty = false;
     if (ev_fft_done) CUCO_TRY_CUDA(cudaEventRecord(*ev_fft_done, stream));
     if (n) {
         if (plan.fixed)
-            k_interp<true><<<(n + 255) / 256, 256, 0, stream>>>(pos, perm, n, plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc);
+            CUCO_TRY_CUDA(launch_chained(chain, k_interp<true>, (n + 255) / 256, 256, 0, stream, pos, perm, n,
+                                         plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc));
         else
-            k_interp<false><<<(n + 255) / 256, 256, 0, stream>>>(pos, perm, n, plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc);
+            CUCO_TRY_CUDA(launch_chained(chain, k_interp<false>, (n + 255) / 256, 256, 0, stream, pos, perm, n,
+                                         plan.rho, M, plan.to_slab_fac, plan.fd_fac, acc));
     }
     CUCO_TRY_CUDA(cudaGetLastError());
     if (launches) *launches += 5 + (n ? 2 : 0);  // five transform passes, deposit and interpolation

@@ -730,6 +730,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     __shared__ WarpMem s_warp[kWarps];
     __shared__ float s_tab[kTabPad];
     __shared__ char2 s_col[kMaxCols];
+    chain_next();  // (the next step's drift; its blocks start in the places this grid's leave)
     load_table(table_g, s_tab);
     for (int i = threadIdx.x; i < cs.ncols; i += kThreads) s_col[i] = make_char2(cs.dx[i], cs.dy[i]);
     __syncthreads();

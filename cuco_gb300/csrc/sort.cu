@@ -462,6 +462,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
             key[k] = kv.x, val[k] = kv.y;
         }
     }
+    chain_next();  // (the cell-order launch, which waits for the stores below)
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
         const uint32_t g = g0 + 32 * k;
@@ -677,6 +678,7 @@ __global__ void k_cell_subsort(const uint32_t *__restrict__ cell_off, const uint
                                const __grid_constant__ CellBox one, const CellBox *__restrict__ boxes, int nbox,
                                int fixed, uint32_t plan_blocks, const __grid_constant__ SRPlan plan,
                                const __grid_constant__ SRWork work) {
+    chain_wait();
     // the first blocks write the short range's work plan (a launch less)
     if (blockIdx.x < plan_blocks) {
         plan_box_segment(plan, blockIdx.x * blockDim.x + threadIdx.x, cell_off, 0u, 0u, work);
@@ -714,10 +716,9 @@ cuco_status_t launch_cell_subsort(const uint32_t *cell_off, const uint32_t *perm
     if (ncells == 0) return CUCO_OK;
     const uint64_t threads = 32ull * ((ncells + 32 / kSubLanes - 1) / (32 / kSubLanes));
     const uint32_t plan_blocks = plan ? (plan->nseg + 255) / 256 : 0u;
-    k_cell_subsort<<<plan_blocks + (unsigned)((threads + 255) / 256), 256, 0, stream>>>(
-        cell_off, perm, pos, sorted_pos, perm_s, slices, ncells, one, boxes, nbox, fixed ? 1 : 0, plan_blocks,
-        plan ? *plan : SRPlan{}, work ? *work : SRWork{});
-    CUCO_TRY_CUDA(cudaGetLastError());
+    CUCO_TRY_CUDA(launch_chained(!boxes, k_cell_subsort, plan_blocks + (unsigned)((threads + 255) / 256), 256, 0, stream,
+                                 cell_off, perm, pos, sorted_pos, perm_s, slices, ncells, one, boxes, nbox, fixed ? 1 : 0,
+                                 plan_blocks, plan ? *plan : SRPlan{}, work ? *work : SRWork{}));
     return CUCO_OK;
 }
 
