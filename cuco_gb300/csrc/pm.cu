@@ -1006,12 +1006,15 @@ cuco_status_t fft_passes_reg(const PMPlan &plan, int P, bool chain, cudaStream_t
 // Many boxes in one launch: map[blockIdx.x] = (box, the box's own block
 // index).  BIG: only the boxes with 32-point register transforms (meshes 512
 // and 1024), every other block returns; !BIG: every other box.
+// What bounds them is latency: at four CTAs an SM (64 registers, a few spilled)
+// instead of three (80) a step of 64 mixed boxes takes 6.15 instead of 6.31 ms,
+// of 16 boxes of 16^3 to 64^3 1.31 instead of 1.33.
 __device__ __forceinline__ bool big_box(const PMBoxDesc &d, int cols) {
     return d.M >= 512 && reg_fft_ok(d.M, cols);
 }
 
 template <bool BIG, bool WIDE>
-__global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
+__global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 4)
     k_fft_z_r2c_multi(const PMBoxDesc *__restrict__ boxes, const uint2 *__restrict__ map) {
     const uint2 m = map[blockIdx.x];
     const PMBoxDesc &d = boxes[m.x];
@@ -1035,7 +1038,7 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
 }
 
 template <bool BIG, bool WIDE>
-__global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
+__global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 4)
     k_fft_z_c2r_multi(const PMBoxDesc *__restrict__ boxes, const uint2 *__restrict__ map) {
     const uint2 m = map[blockIdx.x];
     const PMBoxDesc &d = boxes[m.x];
@@ -1059,7 +1062,7 @@ __global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
 }
 
 template <bool BIG, bool WIDE>
-__global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 3)
+__global__ void __launch_bounds__(kFFTThreads, BIG ? 2 : 4)
     k_fft_axis_multi(const PMBoxDesc *__restrict__ boxes, const uint2 *__restrict__ map, int axis, int sign,
                      int green) {
     const uint2 m = map[blockIdx.x];

@@ -1,5 +1,5 @@
-"""The PM on meshes whose transforms take radices 18 and 24, first, last, alone
-and twice: accelerations against the CPU oracle's PM, rms relative over all
+"""The PM on meshes whose transforms take radices 18 and 24, first and last:
+accelerations against the CPU oracle's PM, rms relative over all
 particles, 1e-4 as in the other parity tests; in an ensemble beside a mesh with
 small radices and a power of two, each box as it is alone, bit for bit; and 48,
 whose last stage is the smallest radix, 3."""
@@ -34,7 +34,7 @@ def forces(pos, cfg):
     return acc
 
 
-@pytest.mark.parametrize("M", [48, 216, 270, 288, 324, 360, 384])
+@pytest.mark.parametrize("M", [48, 216, 288])
 def test_one_box(port, M):
     pos, cfg, params = case(M)
     assert rms_rel(forces(pos, cfg), port.pm(pos, params, M, 4)) < 1e-4
