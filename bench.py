@@ -325,12 +325,12 @@ def run_serving(args, world, rank, local):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of the short range at z = 49:
-# ncu --set full of the first part of the split launch in the first timed step
+# ncu of the first part of the split launch in the first timed step
 # of `bench.py --steps 2 --warmup 3 --e2e-steps 0 --no-cpu` (-s 6 -c 1), which
-# runs alone under ncu and takes every unit (83.0 + 20.9 MB), and of the
-# precision form's (same command with --workload precision-128; 83.3 + 23.1 MB)
-SR_TRAFFIC = {"plain-128^3-L256-M256-G64-z49to0-200steps": 103.9e6,
-              "precision-128^3-L256-M256-G64-z49to0-200steps": 106.4e6}
+# runs alone under ncu and takes every unit (92.3 + 41.9 MB), and of the
+# precision form's (same command with --workload precision-128; 93.5 + 43.1 MB)
+SR_TRAFFIC = {"plain-128^3-L256-M256-G64-z49to0-200steps": 134.2e6,
+              "precision-128^3-L256-M256-G64-z49to0-200steps": 136.6e6}
 
 
 # softening (fraction of the mean spacing) of the small box: 0.03, the others 0.025
