@@ -5,7 +5,8 @@
 //                     gravlist_kernel.cu:92-118), fused
 //   sort_pairs        stable LSD radix sort of (key, index)
 //   reorder           cell offsets + gather of positions into cell order
-//   pm_forces         PM long-range force on the cell-ordered particles
+//   pm_forces         PM long-range force, beside the sort on a second stream
+//                     (a state in scattered order: after it, in cell order)
 //   shortrange        P3M short-range force; its epilogue scatters both forces
 //                     to original order and kicks the velocities
 // Particle state (pos, vel, forces) is kept in original particle order so that
@@ -438,7 +439,7 @@ cuco_status_t forces_after_keys(cuco_box *b, int pm, int pp, const KickArgs *kic
     // original order, needs nothing from the sort and runs beside it.  Where
     // that order scatters many particles over a large mesh it reads them in
     // cell order, after the sort: the deposit's atomics and the
-    // interpolation's 72 loads a particle then stay in a few sectors.  Random
+    // interpolation's 56 loads a particle then stay in a few sectors.  Random
     // order, PM alone, beside the sort against after it: 192^3 particles on
     // 384^3 4.37 -> 2.12 ms, 100^3 on 200^3 0.47 -> 0.41, 80^3 on 160^3 0.27
     // -> 0.26, but 64^3 on 128^3 0.137 -> 0.152; lattice order, early or

@@ -15,8 +15,9 @@
 // never for the step in flight.
 //
 // Autotuning.  A box's short-range cell grid G (cell_grid = 0) and its FFT
-// batching (columns per CTA) are chosen by timing candidates on a scratch box
-// of the same particle count and mesh with uniform positions; results are
+// batching (columns per CTA) are chosen by timing candidates: the grid on a
+// scratch box of the same particle count and mesh with uniform positions, the
+// batching on as many copies of the mesh as fill the GPU; results are
 // cached per (n, M, mode), since R = ceil(rcut / w) depends only on G / M.
 #include <algorithm>
 #include <cmath>
