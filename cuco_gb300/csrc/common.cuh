@@ -248,15 +248,16 @@ cuco_status_t launch_shortrange(const ShortRangeParams &p, const float4 *sorted_
 // Many boxes in one launch (the batched form).  A box's descriptor holds its
 // parameters and neighbour-column set; shortrange_desc_fill writes one (in
 // host memory, shortrange_desc_bytes() long) and returns the box's segment
-// count.  kicks[b] = (kick_pp, kick_pm) of box b.
+// count and the units its plan takes at most; the launch's `units` is their sum
+// over the boxes.  kicks[b] = (kick_pp, kick_pm) of box b.
 size_t shortrange_desc_bytes();
-cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32_t *segments);
+cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32_t *segments, uint32_t *units);
 // uniform_law_desc (host memory, or null): a descriptor whose pair law every
 // box shares (shortrange_descs_uniform_law said so); the launch then reads
 // the law from its parameters instead of each box's descriptor.
 bool shortrange_descs_uniform_law(const void *host_descs, int nbox);
 cuco_status_t launch_shortrange_multi(const void *descs, const double2 *kicks, const uint32_t *seg_base,
-                                      int nbox, uint32_t segments, uint32_t n, bool fixed,
+                                      int nbox, uint32_t segments, uint32_t units, uint32_t n, bool fixed,
                                       const float4 *sorted_pos, const uint32_t *perm, const uint32_t *cell_off,
                                       const float *table, float4 *acc_out, const KickArgs &kick,
                                       const SRWork &work, cudaStream_t stream, unsigned long long *pair_counter,

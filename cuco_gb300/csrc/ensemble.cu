@@ -322,7 +322,7 @@ struct cuco_ensemble {
     bool up_pending[2] = {false, false};
     int slot = 0;
     PMMulti pm{};
-    uint32_t segments = 0;
+    uint32_t segments = 0, units = 0;
     // box 0's short-range descriptor (host copy) when every box has its pair
     // law, so the launch reads the law from its parameters
     std::vector<char> sr_law;
@@ -387,7 +387,7 @@ cuco_status_t ensemble_pass(cuco_ensemble *e, int do_drift, bool kick) {
     k.vel = kick ? e->vel : nullptr;
     k.acc_pm_o = e->acc_pm;
     SRWork w{e->sr_units, (uint32_t)e->cap_units, e->sr_ctl};
-    CUCO_TRY(launch_shortrange_multi(e->d_sr, e->d_kicks, e->d_segbase, e->nbox, e->segments, e->n, e->fixed,
+    CUCO_TRY(launch_shortrange_multi(e->d_sr, e->d_kicks, e->d_segbase, e->nbox, e->segments, e->units, e->n, e->fixed,
                                      e->spos, perm_s, e->cell_off, e->table, e->acc_pp, k, w, e->stream,
                                      e->count_pairs ? e->pair_counter : nullptr,
                                      e->sr_law.empty() ? nullptr : e->sr_law.data()));
@@ -608,7 +608,7 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     std::vector<uint2> mapz, mapa;
     std::vector<float> green(gbase[nbox]);
     std::vector<float2> tw(tbase[nbox]);
-    size_t smz = 0, sma = 0;
+    size_t smz = 0, sma = 0, units = 0;
     for (int b = 0; b < nbox; ++b) {
         const cuco_config_t &c = cfg[b];
         const int M = c.pm_grid, Mh = M / 2 + 1;
@@ -623,14 +623,15 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
         for (uint32_t k = 0; k < na; ++k) mapa.push_back(make_uint2(b, k));
         smz = std::max(smz, pm_smem_z(M, P[b]));
         sma = std::max(sma, pm_smem_axis(M, B[b]));
-        uint32_t nseg = 0;
+        uint32_t nseg = 0, nunits = 0;
         if ((s = shortrange_desc_fill(sr_params(c, (uint32_t)c.n, (uint32_t)cbase[b], e->cell_sl),
-                                      srd.data() + b * shortrange_desc_bytes(), &nseg)))
+                                      srd.data() + b * shortrange_desc_bytes(), &nseg, &nunits)))
             return s;
         segbase[b + 1] = segbase[b] + nseg;
+        units += nunits;
     }
     if ((s = grow(e->d_mapz, e->cap_mapz, mapz.size(), st)) || (s = grow(e->d_mapa, e->cap_mapa, mapa.size(), st)) ||
-        (s = grow(e->sr_units, e->cap_units, (size_t)shortrange_unit_cap((uint32_t)n, segbase[nbox]), st)) ||
+        (s = grow(e->sr_units, e->cap_units, units, st)) ||
         (s = grow(e->sr_ctl, e->cap_ctl, kSRCtlWords, st)))
         return s;
     if (cudaStreamSynchronize(st) != cudaSuccess ||
@@ -662,6 +663,7 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     e->ncells = ncells;
     e->key_bits = kbits;
     e->segments = segbase[nbox];
+    e->units = (uint32_t)units;
     e->sr_law.clear();
     if (shortrange_descs_uniform_law(srd.data(), nbox))
         e->sr_law.assign(srd.begin(), srd.begin() + shortrange_desc_bytes());

@@ -112,6 +112,7 @@ struct ColumnSet {
 struct SRBoxDesc {
     ShortRangeParams p;
     ColumnSet cs;
+    uint32_t slice;  // unit_slice of the box's own particles
 };
 
 // One warp's shared memory: the source list (origin-relative), the runs of
@@ -752,16 +753,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 // entries); particles, cells (p.cell_base) and outputs are the concatenated
 // arrays of all boxes.
 __global__ void k_sr_plan_multi(const SRBoxDesc *__restrict__ boxes, const uint32_t *__restrict__ seg_base,
-                                int nbox, uint32_t nseg, const uint32_t *__restrict__ cell_off, uint32_t slice,
+                                int nbox, uint32_t nseg, const uint32_t *__restrict__ cell_off,
                                 const __grid_constant__ SRWork w) {
     const uint32_t gseg = blockIdx.x * blockDim.x + threadIdx.x;
-    SRPlan plan{1, 1, 0u, slice};
+    SRPlan plan{1, 1, 0u, (uint32_t)kUnitMax};
     uint32_t b = 0, seg = 0, base = 0;
     if (gseg < nseg) {
         b = find_box(seg_base, nbox, gseg);
         const SRBoxDesc &d = boxes[b];
         seg = gseg - seg_base[b];
-        plan = SRPlan{d.cs.S, d.p.grid, 0xffffffffu, slice};
+        plan = SRPlan{d.cs.S, d.p.grid, 0xffffffffu, d.slice};
         base = d.p.cell_base;
     }
     plan_box_segment(plan, seg, cell_off, base, b, w);
@@ -813,6 +814,9 @@ PersistentGrid persistent_grid(K kernel) {
 // Targets of a unit: kUnitMax, halved while the launch would have fewer than
 // two units for each of the GPU's resident warps (about 32 on each of ~150
 // SMs), down to kUnitMin: a box of 32^3 then still gives every warp a unit.
+// n is the box's own count, in a many-box launch too: the unit decides which
+// targets share a list, and so the order of the sums, and a box's forces must
+// not depend on the boxes beside it.
 uint32_t unit_slice(uint32_t n) {
     uint32_t s = kUnitMax;
     while (s > (uint32_t)kUnitMin && n / s < 2u * 4864u) s >>= 1;
@@ -967,13 +971,15 @@ cuco_status_t launch_shortrange(const ShortRangeParams &p_in, const float4 *sort
 
 size_t shortrange_desc_bytes() { return sizeof(SRBoxDesc); }
 
-cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32_t *segments) {
+cuco_status_t shortrange_desc_fill(const ShortRangeParams &p, void *desc, uint32_t *segments, uint32_t *units) {
     SRBoxDesc d{};
     d.p = p;
     finish_pair_law(d.p);
     CUCO_TRY(columns_of(p, &d.cs));
+    d.slice = unit_slice(p.n);
     memcpy(desc, &d, sizeof d);
     *segments = (uint32_t)p.grid * p.grid * (p.grid / d.cs.S);
+    *units = shortrange_unit_cap(p.n, *segments);
     return CUCO_OK;
 }
 
@@ -990,21 +996,20 @@ bool shortrange_descs_uniform_law(const void *host_descs, int nbox) {
 }
 
 cuco_status_t launch_shortrange_multi(const void *descs, const double2 *kicks, const uint32_t *seg_base,
-                                      int nbox, uint32_t segments, uint32_t n, bool fixed,
+                                      int nbox, uint32_t segments, uint32_t units, uint32_t n, bool fixed,
                                       const float4 *sorted_pos, const uint32_t *perm, const uint32_t *cell_off,
                                       const float *table, float4 *acc_out, const KickArgs &kick,
                                       const SRWork &work, cudaStream_t stream, unsigned long long *pair_counter,
                                       const void *uniform_law_desc) {
     if (!segments || !n) return CUCO_OK;
-    if (work.cap < shortrange_unit_cap(n, segments)) {
-        set_error("short range: work-plan scratch too small for the ensemble's segments");
+    if (work.cap < units) {
+        set_error("short range: work-plan scratch too small for the ensemble's units");
         return CUCO_ERR_INVALID;
     }
     const SRBoxDesc *d = static_cast<const SRBoxDesc *>(descs);
     const bool kick_on = kick.vel != nullptr;
-    const uint32_t slice = unit_slice(n);
     CUCO_TRY_CUDA(cudaMemsetAsync(work.ctl, 0, 3 * sizeof(uint32_t), stream));
-    k_sr_plan_multi<<<(segments + 255) / 256, 256, 0, stream>>>(d, seg_base, nbox, segments, cell_off, slice, work);
+    k_sr_plan_multi<<<(segments + 255) / 256, 256, 0, stream>>>(d, seg_base, nbox, segments, cell_off, work);
     // the shared law (any box's, all being equal) or, unused, box 0's shape
     ShortRangeParams law{};
     const bool uniform = uniform_law_desc != nullptr;

@@ -19,8 +19,9 @@ constexpr uint32_t kDense = 128;
 // a target does not change its result): the slices of a dense segment from the
 // front of the list, the others' from its back.  A unit's record holds
 // everything its warp needs to start (box < 2^24, cells < 2^10 per axis), so
-// that no unit repeats the divisions.  Every lane of the warp calls it
-// together (nt = 0: nothing).
+// that no unit repeats the divisions.  slice: the targets of a unit of this
+// segment's box, which may differ between the lanes.  Every lane of the warp
+// calls it together (nt = 0: nothing).
 __device__ __forceinline__ void plan_segment(uint32_t tb, uint32_t nt, uint32_t c0, uint32_t box, uint32_t ix,
                                              uint32_t iy, uint32_t iz, uint32_t slice, const SRWork &w) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -52,10 +53,10 @@ __device__ __forceinline__ void plan_segment(uint32_t tb, uint32_t nt, uint32_t 
     for (; any; any &= any - 1) {
         const int src = __ffs(any) - 1;
         const uint32_t cs = __shfl_sync(kAll, cd, src), os = __shfl_sync(kAll, od, src), ts = __shfl_sync(kAll, tb, src),
-                       ns = __shfl_sync(kAll, nt, src), c0s = __shfl_sync(kAll, c0, src),
+                       ns = __shfl_sync(kAll, nt, src), c0s = __shfl_sync(kAll, c0, src), ls = __shfl_sync(kAll, slice, src),
                        ats = __shfl_sync(kAll, at, src), bs = __shfl_sync(kAll, box, src);
         for (uint32_t k = lane; k < cs; k += 32)
-            w.units[CUCO_IDX(os + k, w.cap)] = make_uint4(ts + k * slice, min(slice, ns - k * slice) | bs << 8, c0s, ats);
+            w.units[CUCO_IDX(os + k, w.cap)] = make_uint4(ts + k * ls, min(ls, ns - k * ls) | bs << 8, c0s, ats);
     }
 }
 
