@@ -252,7 +252,7 @@ __device__ __forceinline__ void shortrange_unit(
     const int lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u, le_mask = lt_mask | (1u << lane);
     const int G = p.grid, nz = S + 2 * R;
-    const int ix = unit.w & 1023, iy = (unit.w >> 10) & 1023, iz0 = unit.w >> 20;
+    const int ix = unit.z & 0xffff, iy = unit.z >> 16, iz0 = unit.w;
     const uint32_t t_begin = unit.x, len = unit.y & 255u;
     const float L = p.boxsize, w = p.cellw, winv = 1.0f / w, fs = p.fscale;
     const bool ZS = p.slices != nullptr;  // sources in z-slice order within cells, with slice counts
