@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdio>
 #include <string>
 
@@ -69,6 +70,36 @@ static inline uint32_t bounds_violations_take() { return 0; }
 uint32_t bounds_violations_sort();
 uint32_t bounds_violations_pm();
 uint32_t bounds_violations_shortrange();
+
+// A kernel's dynamic shared-memory limit belongs to the device that is current
+// when it is raised.  run(set) calls `set` (which raises limits and returns a
+// cudaError_t) where it has not succeeded yet on the current device; a failure
+// is returned and not kept.
+class OncePerDevice {
+    static constexpr int kDevices = 64;  // (a device beyond them: each time)
+    std::atomic<bool> done_[kDevices] = {};
+
+  public:
+    template <typename F>
+    cudaError_t run(F set) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        const bool known = dev >= 0 && dev < kDevices;
+        if (known && done_[dev].load(std::memory_order_acquire)) return cudaSuccess;
+        e = set();
+        if (e != cudaSuccess)
+            cudaGetLastError();  // (reported by the value alone)
+        else if (known)
+            done_[dev].store(true, std::memory_order_release);
+        return e;
+    }
+};
+
+template <typename... P>
+cudaError_t raise_smem_limit(void (*kernel)(P...), size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 
 // ------------------------------------------------------- chained launches
 

@@ -44,6 +44,7 @@ namespace cuco {
 namespace {
 
 constexpr int kFFTThreads = 256;
+constexpr size_t kMaxSmem = 227 * 1024;  // shared memory a CTA can have
 constexpr int kLoadBatch = 8;  // global loads issued per thread before use
 
 // complex a + b, a - b: one packed instruction each (every element rounded as
@@ -981,13 +982,13 @@ cuco_status_t fft_passes_reg(const PMPlan &plan, int P, bool chain, cudaStream_t
     // the transform buffer and the twiddles
     constexpr int rows = RegFFT<M1, M2>::ROWS, zt = z_threads(M1, M2);
     const size_t smz = sizeof(float2) * ((size_t)rows * (P + 1) + M), sma = sizeof(float2) * ((size_t)rows * B + M);
-    static bool attr = [&] {
-        cudaFuncSetAttribute(k_fft_z_r2c_r<M1, M2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(k_fft_z_c2r_r<M1, M2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        cudaFuncSetAttribute(k_fft_axis_r<M1, M2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        return true;
-    }();
-    (void)attr;
+    static OncePerDevice limit;
+    CUCO_TRY_CUDA(limit.run([] {
+        cudaError_t e = raise_smem_limit(k_fft_z_r2c_r<M1, M2>, kMaxSmem);
+        if (e == cudaSuccess) e = raise_smem_limit(k_fft_z_c2r_r<M1, M2>, kMaxSmem);
+        if (e == cudaSuccess) e = raise_smem_limit(k_fft_axis_r<M1, M2>, kMaxSmem);
+        return e;
+    }));
     const unsigned zblocks = (unsigned)((size_t)M * M / (2 * P));
     CUCO_TRY_CUDA(launch_chained(chain, k_fft_z_r2c_r<M1, M2>, zblocks, zt, smz, stream, plan.rho64,
                                  ldexpf(plan.mass, -32), plan.spec, plan.twiddle, P));
@@ -1407,15 +1408,17 @@ size_t pm_smem_axis(int M, int B) { return sizeof(float2) * (2 * (size_t)M * B +
 
 cuco_status_t pm_forces_multi(const PMMulti &m, const float4 *pos, uint32_t n, float4 *acc,
                               cudaStream_t stream, int *launches) {
-    static bool attr = [] {
-        const int mx = 227 * 1024;
-        auto set = [&](auto kernel) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx); };
+    static OncePerDevice limit;
+    CUCO_TRY_CUDA(limit.run([] {
+        cudaError_t e = cudaSuccess;
+        auto set = [&](auto kernel) {
+            if (e == cudaSuccess) e = raise_smem_limit(kernel, kMaxSmem);
+        };
         set(k_fft_z_r2c_multi<true, false>), set(k_fft_z_c2r_multi<true, false>), set(k_fft_axis_multi<true, false>);
         set(k_fft_z_r2c_multi<false, false>), set(k_fft_z_c2r_multi<false, false>), set(k_fft_axis_multi<false, false>);
         set(k_fft_z_r2c_multi<false, true>), set(k_fft_z_c2r_multi<false, true>), set(k_fft_axis_multi<false, true>);
-        return true;
-    }();
-    (void)attr;
+        return e;
+    }));
     CUCO_TRY_CUDA(cudaMemsetAsync(m.rho64_all, 0, sizeof(unsigned long long) * m.rho_all_count, stream));
     if (n) {
         if (m.fixed)
@@ -1503,21 +1506,20 @@ cuco_status_t pm_plan_create(PMPlan *plan, int M, float boxsize, float asmth, fl
     const int P = fft_batch_z(M), B = fft_batch_axis(M);
     const size_t smz = sizeof(float2) * (2 * (size_t)M * (P + 1) + M);
     const size_t sma = sizeof(float2) * (2 * (size_t)M * B + M);
-    constexpr int kMaxSmem = 227 * 1024;
-    if (smz > (size_t)kMaxSmem || sma > (size_t)kMaxSmem) {
+    if (smz > kMaxSmem || sma > kMaxSmem) {
         set_error("PM: the transform of this mesh needs more shared memory than a CTA has");
         return CUCO_ERR_UNSUPPORTED;
     }
-    static const cudaError_t attr = [] {
+    static OncePerDevice limit;
+    CUCO_TRY_CUDA(limit.run([] {
         cudaError_t e = cudaSuccess;
         auto set = [&](auto kernel) {
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+            if (e == cudaSuccess) e = raise_smem_limit(kernel, kMaxSmem);
         };
         set(k_fft_z_r2c<false>), set(k_fft_z_c2r<false>), set(k_fft_axis<false>);
         set(k_fft_z_r2c<true>), set(k_fft_z_c2r<true>), set(k_fft_axis<true>);
         return e;
-    }();
-    CUCO_TRY_CUDA(attr);
+    }));
     return CUCO_OK;
 }
 

@@ -490,9 +490,8 @@ template <int ITEMS>
 cuco_status_t launch_sort_cluster(uint32_t *keys, uint32_t *vals, const uint32_t *vals_in, uint32_t n, int passes,
                                   int rb, uint32_t *cell_off, uint32_t ncells, uint32_t *plan_ctl,
                                   cudaStream_t stream) {
-    static const cudaError_t attr = cudaFuncSetAttribute(
-        k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterMem<ITEMS>));
-    CUCO_TRY_CUDA(attr);
+    static OncePerDevice limit;
+    CUCO_TRY_CUDA(limit.run([] { return raise_smem_limit(k_sort_cluster<ITEMS>, sizeof(ClusterMem<ITEMS>)); }));
     k_sort_cluster<ITEMS><<<kClusterCtas, kClusterThreads, sizeof(ClusterMem<ITEMS>), stream>>>(
         keys, vals, vals_in, n, passes, rb, cell_off, ncells, plan_ctl);
     CUCO_TRY_CUDA(cudaGetLastError());
