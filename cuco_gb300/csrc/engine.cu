@@ -757,9 +757,24 @@ cuco_status_t read_counts(cuco_box_t *b, bool pos, bool vel) {
     if (pos) b->scattered = 2 * (uint64_t)got[1] > 3 * (uint64_t)b->n;
     return CUCO_OK;
 }
+
+// Whether the box's kernels may work on a caller's device array where it lies:
+// memory of the box's own GPU, aligned as floats are.  Another GPU's memory
+// (which a kernel cannot reach without peer access), managed memory and odd
+// addresses go through the staging array, by copies that take them all.
+bool in_place(const cuco_box_t *b, const void *p) {
+    cudaPointerAttributes a{};
+    if ((uintptr_t)p % alignof(float)) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == b->cfg.device;
+}
 }  // namespace state_check
 
 using state_check::count_triplets;
+using state_check::in_place;
 using state_check::read_counts;
 
 extern "C" {
@@ -778,7 +793,7 @@ cuco_status_t cuco_box_set_state(cuco_box_t *b, const float *pos, const float *v
             CUCO_TRY(pack3to4(p, b->pos, b->n, b->stream));
         return v ? pack3to4(v, b->vel, b->n, b->stream) : CUCO_OK;
     };
-    if (on_device) {
+    if (on_device && in_place(b, pos) && (!vel || in_place(b, vel))) {
         // the caller's arrays are checked and read in place (no staging
         // copies: 512^3 set 6.9 -> 4.9 ms), and read to the end on return
         CUCO_TRY(count_triplets(b, pos, true, counts));
@@ -787,12 +802,13 @@ cuco_status_t cuco_box_set_state(cuco_box_t *b, const float *pos, const float *v
         CUCO_TRY(put(pos, vel));
         CUCO_TRY_CUDA(cudaStreamSynchronize(b->stream));
     } else {
-        CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, pos, bytes, cudaMemcpyHostToDevice, b->stream));
+        const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+        CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, pos, bytes, kind, b->stream));
         CUCO_TRY(count_triplets(b, b->stage3, true, counts));
         CUCO_TRY(read_counts(b, true, false));
         CUCO_TRY(put(b->stage3, nullptr));
         if (vel) {
-            CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, vel, bytes, cudaMemcpyHostToDevice, b->stream));
+            CUCO_TRY_CUDA(cudaMemcpyAsync(b->stage3, vel, bytes, kind, b->stream));
             CUCO_TRY(count_triplets(b, b->stage3, false, counts + 2));
             CUCO_TRY(read_counts(b, false, true));
             CUCO_TRY(put(nullptr, b->stage3));
@@ -809,16 +825,18 @@ cuco_status_t cuco_box_get_state(cuco_box_t *b, float *pos, float *vel, float *a
         return CUCO_ERR_INVALID;
     }
     const size_t bytes = sizeof(float) * 3 * b->n;
+    const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     float *dst[4] = {pos, vel, acc_pp, acc_pm};
     float4 *src[4] = {b->pos, b->vel, b->acc_pp, b->acc_pm};
     for (int k = 0; k < 4; ++k) {
         if (!dst[k]) continue;
-        float *out = on_device ? dst[k] : b->stage3;
+        const bool direct = on_device && in_place(b, dst[k]);
+        float *out = direct ? dst[k] : b->stage3;
         if (k == 0 && b->cfg.mode == CUCO_MODE_FIXED)
             CUCO_TRY(from_fixed(src[k], out, b->n, b->cfg.boxsize, b->stream));
         else
             CUCO_TRY(unpack4to3(src[k], out, b->n, b->stream));
-        if (!on_device) CUCO_TRY_CUDA(cudaMemcpyAsync(dst[k], out, bytes, cudaMemcpyDeviceToHost, b->stream));
+        if (!direct) CUCO_TRY_CUDA(cudaMemcpyAsync(dst[k], out, bytes, kind, b->stream));
     }
     return shortrange_check(b->work.ctl, b->stream);  // waits for the stream
 }
