@@ -124,7 +124,7 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
     KickArgs k{};
     // the work plan's scratch, grown on demand (like the reference's device
     // arrays, held until exit)
-    static SRWork w{};
+    static SRWork w{};  // (ctl[4]: blocks that the conversion has finished)
     static uint32_t *off = nullptr;  // cell offsets, then the conversion's scratch
     static size_t off_cap = 0;
     const size_t off_need = (size_t)numCells + 1 + offsets_scratch(numCells);
@@ -144,7 +144,7 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
         capi_check(cudaMalloc(&off, sizeof(uint32_t) * off_need), "cudaForceEvaluateShortrange");
         off_cap = off_need;
     }
-    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, off + numCells + 1, 0),
+    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, off + numCells + 1, w.ctl + 4, 0),
                 "cudaForceEvaluateShortrange");
     capi_status(launch_shortrange(p, (const float4 *)sortedPos, gridParticleIndex, off, s.table, (float4 *)gravAccel,
                                   k, w, false, 0),

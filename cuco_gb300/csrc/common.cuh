@@ -167,10 +167,10 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_
 
 // The reference's cell bounds (cell_end is read where cell_start is not
 // empty) -> the engine's offsets (ncells + 1).  scratch: offsets_scratch(ncells)
-// words.
+// words; finished: a word that is 0 and is 0 again afterwards.
 size_t offsets_scratch(uint32_t ncells);
 cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
-                                       uint32_t ncells, uint32_t *scratch, cudaStream_t stream);
+                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream);
 
 // A box's cell grid within a concatenated cell numbering (cells
 // cell_base .. cell_base + G^3 - 1).
@@ -243,7 +243,7 @@ struct SRWork {
     uint4 *units;
     uint32_t cap;
     uint32_t *ctl;  // kSRCtlWords: [0] dense slices listed, [1] next unit, [2] other units listed
-                    // (reset per launch), [3] timeout word (kept until read), [4], [5] spare
+                    // (reset per launch), [3] timeout word (kept until read), the rest spare
 };
 uint32_t shortrange_unit_cap(uint32_t n, uint64_t segments);
 // What a box's plan needs: cells a segment, the cell grid, segments, targets a

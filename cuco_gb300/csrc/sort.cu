@@ -807,89 +807,155 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_
 
 // ---- start/end -> offsets: off[c] is the largest end of the cells before c
 // (ends grow along the cell order), a running maximum over the cells in two
-// launches: each block's maximum, then every block its cells after the
-// maximum of the blocks before it.
+// launches: each block's maximum, which the last block to finish turns into
+// the maximum before each block; then every block its cells.  Bound by memory:
+// both bounds read twice.  (Every block of the second launch used to read the
+// maxima of all blocks before it, which is quadratic in the cells: a force on
+// 1000 particles in 512^3, 768^3 and 1024^3 cells took 1.90, 21.1 and 116 ms,
+// so 0.76, 2.14 and 4.88; on 64^3 cells 32^3 particles take 122 us either way.)
 namespace {
-constexpr uint32_t kOffItems = 4, kOffBlock = kSortThreads * kOffItems;  // cells per block
+// cells a thread: 4, or 16 from kOffWideCells cells (fewer blocks to scan)
+constexpr uint32_t kOffWideCells = 1u << 22;
 
-// this thread's kOffItems consecutive cells: the largest end of each
+// A warp takes 32 * ITEMS consecutive cells, a lane every 32nd of them (the
+// caller's arrays need no alignment beyond a word's): the end of each, 0 for an
+// empty one.
+template <uint32_t ITEMS>
+__device__ __forceinline__ uint32_t first_cell() {
+    return (blockIdx.x * kSortWarps + (threadIdx.x >> 5)) * (32 * ITEMS) + (threadIdx.x & 31);
+}
+template <uint32_t ITEMS>
 __device__ __forceinline__ void load_ends(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                                          uint32_t ncells, uint32_t (&v)[kOffItems]) {
-    const uint32_t c0 = blockIdx.x * kOffBlock + threadIdx.x * kOffItems;
-    uint32_t s[kOffItems], e[kOffItems];
+                                          uint32_t ncells, uint32_t (&v)[ITEMS]) {
+    const uint32_t c0 = first_cell<ITEMS>();
+    uint32_t s[ITEMS], e[ITEMS];
 #pragma unroll
-    for (uint32_t k = 0; k < kOffItems; ++k) {
-        s[k] = c0 + k < ncells ? start[c0 + k] : kEmptyCell;
-        e[k] = c0 + k < ncells ? end[c0 + k] : 0u;
+    for (uint32_t k = 0; k < ITEMS; ++k) {
+        s[k] = c0 + 32 * k < ncells ? start[c0 + 32 * k] : kEmptyCell;
+        e[k] = c0 + 32 * k < ncells ? end[c0 + 32 * k] : 0u;
     }
 #pragma unroll
-    for (uint32_t k = 0; k < kOffItems; ++k) v[k] = s[k] != kEmptyCell ? e[k] : 0u;
+    for (uint32_t k = 0; k < ITEMS; ++k) v[k] = s[k] != kEmptyCell ? e[k] : 0u;
 }
 
+// The largest v of the block's warps before this one (0 for the first), v
+// being the warp's own; *all: of the whole block.  Every thread calls it
+// together.
+__device__ __forceinline__ uint32_t warps_before(uint32_t v, uint32_t *all) {
+    __shared__ uint32_t s_warp[kSortWarps];
+    const uint32_t warp = threadIdx.x >> 5;
+    uint32_t before = 0;
+    __syncthreads();  // s_warp of a call before is read
+    if ((threadIdx.x & 31) == 0) s_warp[warp] = v;
+    __syncthreads();
+    *all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < (uint32_t)kSortWarps; ++w) {
+        const uint32_t x = s_warp[w];
+        before = max(before, w < warp ? x : 0u);
+        *all = max(*all, x);
+    }
+    return before;
+}
+
+// The running maximum of the lanes up to this one; *all: of the warp.
+__device__ __forceinline__ uint32_t warp_max_scan(uint32_t v, uint32_t *all) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (uint32_t off = 1; off < 32; off <<= 1) {
+        const uint32_t u = __shfl_up_sync(kFull, v, off);
+        if (lane >= off) v = max(v, u);
+    }
+    *all = __shfl_sync(kFull, v, 31);
+    return v;
+}
+
+// block_max[b] = the largest end before block b's cells.  *finished counts the
+// blocks that have written theirs; it is 0 between launches.
+template <uint32_t ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_block_end_max(const uint32_t *__restrict__ start,
                                                                 const uint32_t *__restrict__ end, uint32_t ncells,
-                                                                uint32_t *__restrict__ block_max) {
-    __shared__ uint32_t s_max[kSortWarps];
-    uint32_t v[kOffItems], m = 0;
+                                                                uint32_t *block_max, uint32_t *finished) {
+    __shared__ bool s_last;
+    uint32_t v[ITEMS], m = 0, all;
     load_ends(start, end, ncells, v);
 #pragma unroll
-    for (uint32_t k = 0; k < kOffItems; ++k) m = max(m, v[k]);
-    m = __reduce_max_sync(kFull, m);
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
-    __syncthreads();
+    for (uint32_t k = 0; k < ITEMS; ++k) m = max(m, v[k]);
+    warps_before(__reduce_max_sync(kFull, m), &all);
     if (threadIdx.x == 0) {
-        for (int w = 1; w < kSortWarps; ++w) m = max(m, s_max[w]);
-        block_max[blockIdx.x] = m;
+        __stcg(&block_max[blockIdx.x], all);
+        __threadfence();
+        s_last = atomicAdd(finished, 1u) == gridDim.x - 1;
     }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // the last block: the maximum before each block, 8 rounds' loads in flight
+    constexpr uint32_t kAhead = 8;
+    uint32_t carry = 0;
+    for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kAhead * kSortThreads) {
+        uint32_t x[kAhead];
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            const uint32_t b = b0 + k * kSortThreads + threadIdx.x;
+            x[k] = b < gridDim.x ? __ldcg(&block_max[b]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            const uint32_t b = b0 + k * kSortThreads + threadIdx.x;
+            uint32_t warp_all, round_all;
+            const uint32_t incl = warp_max_scan(x[k], &warp_all);
+            uint32_t before = __shfl_up_sync(kFull, incl, 1);
+            if ((threadIdx.x & 31) == 0) before = 0;
+            before = max(max(carry, before), warps_before(warp_all, &round_all));
+            if (b < gridDim.x) __stcg(&block_max[b], before);
+            carry = max(carry, round_all);
+        }
+    }
+    if (threadIdx.x == 0) *finished = 0;
 }
 
+template <uint32_t ITEMS>
 __global__ void __launch_bounds__(kSortThreads) k_start_end_offsets(const uint32_t *__restrict__ start,
                                                                     const uint32_t *__restrict__ end, uint32_t ncells,
                                                                     const uint32_t *__restrict__ block_max,
                                                                     uint32_t *__restrict__ cell_off) {
-    __shared__ uint32_t s_carry[kSortWarps], s_warp[kSortWarps];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t v[kOffItems];
+    uint32_t v[ITEMS], m = 0, all;
     load_ends(start, end, ncells, v);
-    uint32_t carry = 0;
-    for (uint32_t k = threadIdx.x; k < blockIdx.x; k += kSortThreads) carry = max(carry, block_max[k]);
-    carry = __reduce_max_sync(kFull, carry);
+    uint32_t carry = block_max[blockIdx.x];
 #pragma unroll
-    for (uint32_t k = 1; k < kOffItems; ++k) v[k] = max(v[k], v[k - 1]);
-    uint32_t incl = v[kOffItems - 1];
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t u = __shfl_up_sync(kFull, incl, off);
-        if (lane >= off) incl = max(incl, u);
-    }
-    uint32_t before = __shfl_up_sync(kFull, incl, 1);
-    if (lane == 0) before = 0;
-    if (lane == 31) s_warp[warp] = incl;
-    if (lane == 0) s_carry[warp] = carry;
-    __syncthreads();
-    for (uint32_t w = 0; w < (uint32_t)kSortWarps; ++w) {
-        before = max(before, s_carry[w]);
-        if (w < warp) before = max(before, s_warp[w]);
-    }
+    for (uint32_t k = 0; k < ITEMS; ++k) m = max(m, v[k]);
+    carry = max(carry, warps_before(__reduce_max_sync(kFull, m), &all));
     // cell c ends, and the next begins, at the largest end so far
-    const uint32_t c0 = blockIdx.x * kOffBlock + threadIdx.x * kOffItems;
+    const uint32_t c0 = first_cell<ITEMS>();
 #pragma unroll
-    for (uint32_t k = 0; k < kOffItems; ++k)
-        if (c0 + k < ncells) cell_off[c0 + k + 1] = max(before, v[k]);
+    for (uint32_t k = 0; k < ITEMS; ++k) {
+        const uint32_t off = max(carry, warp_max_scan(v[k], &all));
+        if (c0 + 32 * k < ncells) cell_off[c0 + 32 * k + 1] = off;
+        carry = max(carry, all);
+    }
     if (c0 == 0) cell_off[0] = 0;
+}
+
+template <uint32_t ITEMS>
+cuco_status_t start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
+                                uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream) {
+    constexpr uint32_t kCells = kSortThreads * ITEMS;
+    const unsigned blocks = ncells / kCells + (ncells % kCells != 0);
+    k_block_end_max<ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, finished);
+    k_start_end_offsets<ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, cell_off);
+    CUCO_TRY_CUDA(cudaGetLastError());
+    return CUCO_OK;
 }
 }  // namespace
 
-size_t offsets_scratch(uint32_t ncells) { return (ncells + kOffBlock - 1) / kOffBlock; }
+size_t offsets_scratch(uint32_t ncells) { return (size_t)ncells / (kSortThreads * 4) + 1; }
 
 cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
-                                       uint32_t ncells, uint32_t *scratch, cudaStream_t stream) {
-    const unsigned blocks = (unsigned)offsets_scratch(ncells);
-    if (!blocks) return CUCO_OK;
-    k_block_end_max<<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch);
-    k_start_end_offsets<<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, cell_off);
-    CUCO_TRY_CUDA(cudaGetLastError());
-    return CUCO_OK;
+                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream) {
+    if (!ncells) return CUCO_OK;
+    auto launch = ncells < kOffWideCells ? start_end_offsets<4> : start_end_offsets<16>;
+    return launch(cell_start, cell_end, cell_off, ncells, scratch, finished, stream);
 }
 
 uint32_t bounds_violations_sort() { return bounds_violations_take(); }

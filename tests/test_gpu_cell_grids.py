@@ -1,6 +1,7 @@
 """The reference-named short range (cudaForceEvaluateShortrange) on cell grids
 beyond 1024 an axis and on grids of many more cells than particles: forces
-against the CPU oracle, rms relative 1e-4 as in the other parity tests."""
+against the CPU oracle, rms relative 1e-4 as in the other parity tests, and a
+cost that grows with the cells, not with their square."""
 import ctypes
 
 import numpy as np
@@ -69,7 +70,7 @@ def clumps(n, G, seed):
     return pos
 
 
-@pytest.mark.parametrize("G", [300, 1024, 1025, 1032])
+@pytest.mark.parametrize("G", [20, 300, 1024, 1025, 1032])
 def test_forces(port, G):
     pos = clumps(4000, G, G)
     g = Gravlist(pos, G, G, 0.1 * L / G)
@@ -78,3 +79,31 @@ def test_forces(port, G):
     del g
     torch.cuda.empty_cache()
 
+
+def test_cost_grows_with_the_cells():
+    """768^3 cells, 1000 particles.  A call reads both bounds twice, writes the
+    offsets and reads them at the segments' ends: at most 24 bytes a cell.  A
+    copy of both bounds moves 16.  A work that is quadratic in the cells' blocks
+    of 1024 (390 GB of block results here) takes tens of such copies."""
+    g = Gravlist(clumps(1000, 768, 1), 768, 768, 0.1 * L / 768)
+    copies = [torch.empty_like(g.start), torch.empty_like(g.end)]
+
+    def best(f):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            f()
+            b.record()
+            torch.cuda.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    def copy():
+        copies[0].copy_(g.start)
+        copies[1].copy_(g.end)
+
+    force, moved = best(g.forces), best(copy)
+    print(f"force {force:.3f} ms, copy {moved:.3f} ms")
+    assert force < 6 * moved
