@@ -124,32 +124,63 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
     KickArgs k{};
     // the work plan's scratch, grown on demand (like the reference's device
     // arrays, held until exit)
-    static SRWork w{};  // (ctl[4]: blocks that the conversion has finished)
+    static SRWork w{};  // ctl[4]: blocks that the conversion has finished, ctl[5]: the bounds have gaps
     static uint32_t *off = nullptr;  // cell offsets, then the conversion's scratch
     static size_t off_cap = 0;
-    const size_t off_need = (size_t)numCells + 1 + offsets_scratch(numCells);
-    const uint32_t cap = shortrange_unit_cap(numParticles, numCells);
-    if (w.cap < cap) {
+    const char *const me = "cudaForceEvaluateShortrange";
+    auto reserve = [&](uint32_t n) {
+        const uint32_t cap = shortrange_unit_cap(n, numCells);
+        if (w.cap >= cap) return;
         cudaFree(w.units);
         cudaFree(w.ctl);
         w = SRWork{};
-        capi_check(cudaMalloc(&w.units, sizeof(uint4) * cap), "cudaForceEvaluateShortrange");
-        capi_check(cudaMalloc(&w.ctl, kSRCtlWords * sizeof(uint32_t)), "cudaForceEvaluateShortrange");
-        capi_check(cudaMemset(w.ctl, 0, kSRCtlWords * sizeof(uint32_t)), "cudaForceEvaluateShortrange");
+        capi_check(cudaMalloc(&w.units, sizeof(uint4) * cap), me);
+        capi_check(cudaMalloc(&w.ctl, kSRCtlWords * sizeof(uint32_t)), me);
+        capi_check(cudaMemset(w.ctl, 0, kSRCtlWords * sizeof(uint32_t)), me);
         w.cap = cap;
-    }
+    };
+    reserve(numParticles);
+    const size_t off_need = (size_t)numCells + 1 + offsets_scratch(numCells);
     if (off_cap < off_need) {
         cudaFree(off);
         off_cap = 0;
-        capi_check(cudaMalloc(&off, sizeof(uint32_t) * off_need), "cudaForceEvaluateShortrange");
+        capi_check(cudaMalloc(&off, sizeof(uint32_t) * off_need), me);
         off_cap = off_need;
     }
-    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, off + numCells + 1, w.ctl + 4, 0),
-                "cudaForceEvaluateShortrange");
+    uint32_t *const scratch = off + numCells + 1;
+    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, scratch, w.ctl + 4, w.ctl + 5, 0), me);
     capi_status(launch_shortrange(p, (const float4 *)sortedPos, gridParticleIndex, off, s.table, (float4 *)gravAccel,
-                                  k, w, false, 0),
-                "cudaForceEvaluateShortrange");
-    capi_status(shortrange_check(w.ctl, 0), "cudaForceEvaluateShortrange");
+                                  k, w, false, 0, nullptr, nullptr, nullptr, w.ctl + 5),
+                me);
+    uint32_t seen[3];  // the timeout word, ctl[4], ctl[5]
+    capi_check(cudaMemcpyAsync(seen, w.ctl + 3, sizeof seen, cudaMemcpyDeviceToHost, 0), me);
+    capi_check(cudaStreamSynchronize(0), me);
+    if (seen[2]) {
+        // Cells whose ranges leave particles out (or overlap): nothing has been
+        // evaluated yet.  The engine's offsets cannot say it; the cells' own
+        // particles are laid one after the other first.
+        static float4 *pos = nullptr;
+        static uint32_t *perm = nullptr;
+        static uint32_t held = 0;
+        capi_check(cudaMemsetAsync(w.ctl + 5, 0, sizeof(uint32_t), 0), me);
+        capi_status(launch_start_end_counts(cellStart, cellEnd, off, numCells, scratch, w.ctl + 4, 0), me);
+        capi_check(cudaMemcpyAsync(&p.n, off + numCells, sizeof(uint32_t), cudaMemcpyDeviceToHost, 0), me);
+        capi_check(cudaStreamSynchronize(0), me);
+        reserve(p.n);
+        if (held < p.n) {
+            cudaFree(pos);
+            cudaFree(perm);
+            held = 0;
+            capi_check(cudaMalloc(&pos, sizeof(float4) * p.n), me);
+            capi_check(cudaMalloc(&perm, sizeof(uint32_t) * p.n), me);
+            held = p.n;
+        }
+        capi_status(launch_gather_cells(cellStart, cellEnd, off, numCells, (const float4 *)sortedPos, gridParticleIndex,
+                                        pos, perm, 0),
+                    me);
+        capi_status(launch_shortrange(p, pos, perm, off, s.table, (float4 *)gravAccel, k, w, false, 0), me);
+    }
+    if (seen[0] || seen[2]) capi_status(shortrange_check(w.ctl, 0), me);
 }
 
 // what a caller's `counters` holds at least (the reference RadixSort's allocation)

@@ -166,11 +166,22 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_
                                      cudaStream_t stream, uint32_t *plan_ctl = nullptr);
 
 // The reference's cell bounds (cell_end is read where cell_start is not
-// empty) -> the engine's offsets (ncells + 1).  scratch: offsets_scratch(ncells)
-// words; finished: a word that is 0 and is 0 again afterwards.
+// empty) -> the engine's offsets (ncells + 1), where the cells' ranges follow
+// one another; *gap (0 before) is set where they do not.  scratch:
+// offsets_scratch(ncells) words; finished: a word that is 0 and is 0 again
+// afterwards.
 size_t offsets_scratch(uint32_t ncells);
 cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
-                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream);
+                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, uint32_t *gap,
+                                       cudaStream_t stream);
+
+// The same for ranges with gaps: the offsets that the cells' particles have
+// when they are laid one after the other, and that layout of them.
+cuco_status_t launch_start_end_counts(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
+                                      uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream);
+cuco_status_t launch_gather_cells(const uint32_t *cell_start, const uint32_t *cell_end, const uint32_t *cell_off,
+                                  uint32_t ncells, const float4 *pos, const uint32_t *perm, float4 *pos_out,
+                                  uint32_t *perm_out, cudaStream_t stream);
 
 // A box's cell grid within a concatenated cell numbering (cells
 // cell_base .. cell_base + G^3 - 1).
@@ -262,6 +273,8 @@ cuco_status_t shortrange_check(uint32_t *ctl, cudaStream_t stream);
 cuco_status_t shortrange_timeout_probe(uint32_t *ctl, long long limit_cycles, cudaStream_t stream);
 
 // planned: the work plan is in `work` already (launch_cell_subsort wrote it).
+// hold (not planned, or null): a word in device memory; where it is not 0 when
+// the plan is written, the plan stays empty and the launch does nothing.
 // pair_counter: when non-null, the launch adds its in-range pair count to it.
 // late_stream (with plan_done, an event of the caller's): the persistent grid
 // is split, one CTA per SM fewer on `stream` and the rest queued on
@@ -274,7 +287,7 @@ cuco_status_t launch_shortrange(const ShortRangeParams &p, const float4 *sorted_
                                 const uint32_t *perm, const uint32_t *cell_off, const float *table,
                                 float4 *acc_out, const KickArgs &kick, const SRWork &work, bool planned,
                                 cudaStream_t stream, unsigned long long *pair_counter = nullptr, cudaStream_t late_stream = nullptr,
-                                cudaEvent_t plan_done = nullptr);
+                                cudaEvent_t plan_done = nullptr, const uint32_t *hold = nullptr);
 
 // Many boxes in one launch (the batched form).  A box's descriptor holds its
 // parameters and neighbour-column set; shortrange_desc_fill writes one (in

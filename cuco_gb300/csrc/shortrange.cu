@@ -675,7 +675,8 @@ __device__ __forceinline__ void shortrange_unit(
 }
 
 __global__ void k_sr_plan(const __grid_constant__ SRPlan plan, const uint32_t *__restrict__ cell_off,
-                          const __grid_constant__ SRWork w) {
+                          const uint32_t *__restrict__ hold, const __grid_constant__ SRWork w) {
+    if (hold && *hold) return;
     plan_box_segment(plan, blockIdx.x * blockDim.x + threadIdx.x, cell_off, 0u, 0u, w);
 }
 
@@ -937,7 +938,8 @@ cuco_status_t shortrange_plan(const ShortRangeParams &p, SRPlan *plan) {
 cuco_status_t launch_shortrange(const ShortRangeParams &p_in, const float4 *sorted_pos, const uint32_t *perm,
                                 const uint32_t *cell_off, const float *table, float4 *acc_out, const KickArgs &kick,
                                 const SRWork &work, bool planned, cudaStream_t stream,
-                                unsigned long long *pair_counter, cudaStream_t late_stream, cudaEvent_t plan_done) {
+                                unsigned long long *pair_counter, cudaStream_t late_stream, cudaEvent_t plan_done,
+                                const uint32_t *hold) {
     ColumnSet cs;
     ShortRangeParams p = p_in;
     finish_pair_law(p);
@@ -952,7 +954,7 @@ cuco_status_t launch_shortrange(const ShortRangeParams &p_in, const float4 *sort
     const bool kick_on = kick.vel != nullptr;
     if (!planned) {
         CUCO_TRY_CUDA(cudaMemsetAsync(work.ctl, 0, 3 * sizeof(uint32_t), stream));
-        k_sr_plan<<<(plan.nseg + 255) / 256, 256, 0, stream>>>(plan, cell_off, work);
+        k_sr_plan<<<(plan.nseg + 255) / 256, 256, 0, stream>>>(plan, cell_off, hold, work);
     }
     if (late_stream) {
         if (!plan_done) {

@@ -805,10 +805,13 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_
     return CUCO_OK;
 }
 
-// ---- start/end -> offsets: off[c] is the largest end of the cells before c
-// (ends grow along the cell order), a running maximum over the cells in two
-// launches: each block's maximum, which the last block to finish turns into
-// the maximum before each block; then every block its cells.  Bound by memory:
+// ---- start/end -> offsets: where the cells' ranges follow one another without
+// gaps (as reorderDataAndFindCellStart leaves them), off[c] is the largest end
+// of the cells before c, a running maximum; a range that does not start there is
+// reported.  Where they do not, off[c] is the particles that the cells before c
+// hold, a running sum, for a copy of the particles in that order.  Either takes
+// two launches: each block's value, which the last block to finish turns into
+// the value before each block; then every block its cells.  Bound by memory:
 // both bounds read twice.  (Every block of the second launch used to read the
 // maxima of all blocks before it, which is quadratic in the cells: a force on
 // 1000 particles in 512^3, 768^3 and 1024^3 cells took 1.90, 21.1 and 116 ms,
@@ -817,30 +820,48 @@ namespace {
 // cells a thread: 4, or 16 from kOffWideCells cells (fewer blocks to scan)
 constexpr uint32_t kOffWideCells = 1u << 22;
 
+struct RunningEnd {
+    static __device__ __forceinline__ uint32_t of(uint32_t, uint32_t e) { return e; }
+    static __device__ __forceinline__ uint32_t join(uint32_t a, uint32_t b) { return max(a, b); }
+    static __device__ __forceinline__ uint32_t warp(uint32_t v) { return __reduce_max_sync(kFull, v); }
+};
+struct RunningCount {
+    static __device__ __forceinline__ uint32_t of(uint32_t s, uint32_t e) { return e > s ? e - s : 0u; }
+    static __device__ __forceinline__ uint32_t join(uint32_t a, uint32_t b) { return a + b; }
+    static __device__ __forceinline__ uint32_t warp(uint32_t v) { return __reduce_add_sync(kFull, v); }
+};
+
 // A warp takes 32 * ITEMS consecutive cells, a lane every 32nd of them (the
-// caller's arrays need no alignment beyond a word's): the end of each, 0 for an
-// empty one.
+// caller's arrays need no alignment beyond a word's): the value of each, 0 for
+// an empty one (s its start, kEmptyCell).
 template <uint32_t ITEMS>
 __device__ __forceinline__ uint32_t first_cell() {
     return (blockIdx.x * kSortWarps + (threadIdx.x >> 5)) * (32 * ITEMS) + (threadIdx.x & 31);
 }
-template <uint32_t ITEMS>
-__device__ __forceinline__ void load_ends(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                                          uint32_t ncells, uint32_t (&v)[ITEMS]) {
+template <typename Op, uint32_t ITEMS>
+__device__ __forceinline__ void load_cells(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+                                           uint32_t ncells, uint32_t (&s)[ITEMS], uint32_t (&v)[ITEMS]) {
     const uint32_t c0 = first_cell<ITEMS>();
-    uint32_t s[ITEMS], e[ITEMS];
+    uint32_t e[ITEMS];
 #pragma unroll
     for (uint32_t k = 0; k < ITEMS; ++k) {
         s[k] = c0 + 32 * k < ncells ? start[c0 + 32 * k] : kEmptyCell;
         e[k] = c0 + 32 * k < ncells ? end[c0 + 32 * k] : 0u;
     }
 #pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) v[k] = s[k] != kEmptyCell ? e[k] : 0u;
+    for (uint32_t k = 0; k < ITEMS; ++k) v[k] = s[k] != kEmptyCell ? Op::of(s[k], e[k]) : 0u;
+}
+template <typename Op, uint32_t ITEMS>
+__device__ __forceinline__ uint32_t joined(const uint32_t (&v)[ITEMS]) {
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < ITEMS; ++k) m = Op::join(m, v[k]);
+    return Op::warp(m);
 }
 
-// The largest v of the block's warps before this one (0 for the first), v
-// being the warp's own; *all: of the whole block.  Every thread calls it
-// together.
+// The joined v of the block's warps before this one (0 for the first), v being
+// the warp's own; *all: of the whole block.  Every thread calls it together.
+template <typename Op>
 __device__ __forceinline__ uint32_t warps_before(uint32_t v, uint32_t *all) {
     __shared__ uint32_t s_warp[kSortWarps];
     const uint32_t warp = threadIdx.x >> 5;
@@ -852,45 +873,45 @@ __device__ __forceinline__ uint32_t warps_before(uint32_t v, uint32_t *all) {
 #pragma unroll
     for (uint32_t w = 0; w < (uint32_t)kSortWarps; ++w) {
         const uint32_t x = s_warp[w];
-        before = max(before, w < warp ? x : 0u);
-        *all = max(*all, x);
+        before = Op::join(before, w < warp ? x : 0u);
+        *all = Op::join(*all, x);
     }
     return before;
 }
 
-// The running maximum of the lanes up to this one; *all: of the warp.
-__device__ __forceinline__ uint32_t warp_max_scan(uint32_t v, uint32_t *all) {
+// The joined v of the lanes before this one (0 for the first); *all: of the warp.
+template <typename Op>
+__device__ __forceinline__ uint32_t lanes_before(uint32_t v, uint32_t *all) {
     const uint32_t lane = threadIdx.x & 31;
 #pragma unroll
     for (uint32_t off = 1; off < 32; off <<= 1) {
         const uint32_t u = __shfl_up_sync(kFull, v, off);
-        if (lane >= off) v = max(v, u);
+        if (lane >= off) v = Op::join(v, u);
     }
     *all = __shfl_sync(kFull, v, 31);
-    return v;
+    const uint32_t before = __shfl_up_sync(kFull, v, 1);
+    return lane ? before : 0u;
 }
 
-// block_max[b] = the largest end before block b's cells.  *finished counts the
-// blocks that have written theirs; it is 0 between launches.
-template <uint32_t ITEMS>
-__global__ void __launch_bounds__(kSortThreads) k_block_end_max(const uint32_t *__restrict__ start,
-                                                                const uint32_t *__restrict__ end, uint32_t ncells,
-                                                                uint32_t *block_max, uint32_t *finished) {
+// before[b] = the value before block b's cells.  *finished counts the blocks
+// that have written theirs; it is 0 between launches.
+template <typename Op, uint32_t ITEMS>
+__global__ void __launch_bounds__(kSortThreads) k_block_values(const uint32_t *__restrict__ start,
+                                                               const uint32_t *__restrict__ end, uint32_t ncells,
+                                                               uint32_t *before, uint32_t *finished) {
     __shared__ bool s_last;
-    uint32_t v[ITEMS], m = 0, all;
-    load_ends(start, end, ncells, v);
-#pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) m = max(m, v[k]);
-    warps_before(__reduce_max_sync(kFull, m), &all);
+    uint32_t s[ITEMS], v[ITEMS], all;
+    load_cells<Op>(start, end, ncells, s, v);
+    warps_before<Op>(joined<Op>(v), &all);
     if (threadIdx.x == 0) {
-        __stcg(&block_max[blockIdx.x], all);
+        __stcg(&before[blockIdx.x], all);
         __threadfence();
         s_last = atomicAdd(finished, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    // the last block: the maximum before each block, 8 rounds' loads in flight
+    // the last block: the value before each block, 8 rounds' loads in flight
     constexpr uint32_t kAhead = 8;
     uint32_t carry = 0;
     for (uint32_t b0 = 0; b0 < gridDim.x; b0 += kAhead * kSortThreads) {
@@ -898,64 +919,100 @@ __global__ void __launch_bounds__(kSortThreads) k_block_end_max(const uint32_t *
 #pragma unroll
         for (uint32_t k = 0; k < kAhead; ++k) {
             const uint32_t b = b0 + k * kSortThreads + threadIdx.x;
-            x[k] = b < gridDim.x ? __ldcg(&block_max[b]) : 0u;
+            x[k] = b < gridDim.x ? __ldcg(&before[b]) : 0u;
         }
 #pragma unroll
         for (uint32_t k = 0; k < kAhead; ++k) {
             const uint32_t b = b0 + k * kSortThreads + threadIdx.x;
             uint32_t warp_all, round_all;
-            const uint32_t incl = warp_max_scan(x[k], &warp_all);
-            uint32_t before = __shfl_up_sync(kFull, incl, 1);
-            if ((threadIdx.x & 31) == 0) before = 0;
-            before = max(max(carry, before), warps_before(warp_all, &round_all));
-            if (b < gridDim.x) __stcg(&block_max[b], before);
-            carry = max(carry, round_all);
+            const uint32_t lanes = lanes_before<Op>(x[k], &warp_all);
+            const uint32_t at = Op::join(Op::join(carry, warps_before<Op>(warp_all, &round_all)), lanes);
+            if (b < gridDim.x) __stcg(&before[b], at);
+            carry = Op::join(carry, round_all);
         }
     }
     if (threadIdx.x == 0) *finished = 0;
 }
 
-template <uint32_t ITEMS>
-__global__ void __launch_bounds__(kSortThreads) k_start_end_offsets(const uint32_t *__restrict__ start,
-                                                                    const uint32_t *__restrict__ end, uint32_t ncells,
-                                                                    const uint32_t *__restrict__ block_max,
-                                                                    uint32_t *__restrict__ cell_off) {
-    uint32_t v[ITEMS], m = 0, all;
-    load_ends(start, end, ncells, v);
-    uint32_t carry = block_max[blockIdx.x];
-#pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) m = max(m, v[k]);
-    carry = max(carry, warps_before(__reduce_max_sync(kFull, m), &all));
-    // cell c ends, and the next begins, at the largest end so far
+// gap (or null): set where a cell's range does not start at its offset.
+template <typename Op, uint32_t ITEMS>
+__global__ void __launch_bounds__(kSortThreads) k_cell_offsets(const uint32_t *__restrict__ start,
+                                                               const uint32_t *__restrict__ end, uint32_t ncells,
+                                                               const uint32_t *__restrict__ block_before,
+                                                               uint32_t *__restrict__ cell_off, uint32_t *gap) {
+    uint32_t s[ITEMS], v[ITEMS], all;
+    load_cells<Op>(start, end, ncells, s, v);
+    uint32_t carry = Op::join(block_before[blockIdx.x], warps_before<Op>(joined<Op>(v), &all));
     const uint32_t c0 = first_cell<ITEMS>();
+    bool apart = false;
 #pragma unroll
     for (uint32_t k = 0; k < ITEMS; ++k) {
-        const uint32_t off = max(carry, warp_max_scan(v[k], &all));
-        if (c0 + 32 * k < ncells) cell_off[c0 + 32 * k + 1] = off;
-        carry = max(carry, all);
+        const uint32_t off = Op::join(carry, lanes_before<Op>(v[k], &all));
+        if (c0 + 32 * k < ncells) cell_off[c0 + 32 * k] = off;
+        apart |= s[k] != kEmptyCell && s[k] != off;
+        carry = Op::join(carry, all);
+        if (c0 + 32 * k == ncells - 1) cell_off[ncells] = Op::join(off, v[k]);
     }
-    if (c0 == 0) cell_off[0] = 0;
+    if (gap && __any_sync(kFull, apart) && (threadIdx.x & 31) == 0) atomicOr(gap, 1u);
 }
 
-template <uint32_t ITEMS>
-cuco_status_t start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
-                                uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream) {
+template <typename Op, uint32_t ITEMS>
+cuco_status_t cell_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off, uint32_t ncells,
+                           uint32_t *scratch, uint32_t *finished, uint32_t *gap, cudaStream_t stream) {
     constexpr uint32_t kCells = kSortThreads * ITEMS;
     const unsigned blocks = ncells / kCells + (ncells % kCells != 0);
-    k_block_end_max<ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, finished);
-    k_start_end_offsets<ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, cell_off);
+    k_block_values<Op, ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, finished);
+    k_cell_offsets<Op, ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, cell_off, gap);
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
+}
+
+// The particles of the cells' ranges, in cell order, to where cell_off says: a
+// warp takes 32 cells, and copies one cell after the other.
+__global__ void k_gather_cells(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+                               const uint32_t *__restrict__ cell_off, uint32_t ncells, const float4 *__restrict__ pos,
+                               const uint32_t *__restrict__ perm, float4 *__restrict__ pos_out,
+                               uint32_t *__restrict__ perm_out) {
+    const uint32_t lane = threadIdx.x & 31, c = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t s = c < ncells ? start[c] : kEmptyCell, e = s != kEmptyCell ? end[c] : 0u;
+    const uint32_t to = c < ncells ? cell_off[c] : 0u;
+    for (uint32_t rest = __ballot_sync(kFull, s != kEmptyCell && e > s); rest; rest &= rest - 1) {
+        const int src = __ffs(rest) - 1;
+        const uint32_t from = __shfl_sync(kFull, s, src), count = __shfl_sync(kFull, e, src) - from,
+                       at = __shfl_sync(kFull, to, src);
+        for (uint32_t k = lane; k < count; k += 32) {
+            pos_out[at + k] = pos[from + k];
+            perm_out[at + k] = perm[from + k];
+        }
+    }
 }
 }  // namespace
 
 size_t offsets_scratch(uint32_t ncells) { return (size_t)ncells / (kSortThreads * 4) + 1; }
 
 cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
-                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream) {
+                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, uint32_t *gap,
+                                       cudaStream_t stream) {
     if (!ncells) return CUCO_OK;
-    auto launch = ncells < kOffWideCells ? start_end_offsets<4> : start_end_offsets<16>;
-    return launch(cell_start, cell_end, cell_off, ncells, scratch, finished, stream);
+    auto launch = ncells < kOffWideCells ? cell_offsets<RunningEnd, 4> : cell_offsets<RunningEnd, 16>;
+    return launch(cell_start, cell_end, cell_off, ncells, scratch, finished, gap, stream);
+}
+
+cuco_status_t launch_start_end_counts(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
+                                      uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream) {
+    if (!ncells) return CUCO_OK;
+    auto launch = ncells < kOffWideCells ? cell_offsets<RunningCount, 4> : cell_offsets<RunningCount, 16>;
+    return launch(cell_start, cell_end, cell_off, ncells, scratch, finished, nullptr, stream);
+}
+
+cuco_status_t launch_gather_cells(const uint32_t *cell_start, const uint32_t *cell_end, const uint32_t *cell_off,
+                                  uint32_t ncells, const float4 *pos, const uint32_t *perm, float4 *pos_out,
+                                  uint32_t *perm_out, cudaStream_t stream) {
+    if (!ncells) return CUCO_OK;
+    k_gather_cells<<<ncells / 256 + (ncells % 256 != 0), 256, 0, stream>>>(cell_start, cell_end, cell_off, ncells, pos,
+                                                                         perm, pos_out, perm_out);
+    CUCO_TRY_CUDA(cudaGetLastError());
+    return CUCO_OK;
 }
 
 uint32_t bounds_violations_sort() { return bounds_violations_take(); }

@@ -78,7 +78,10 @@ void reorderDataAndFindCellStart(uint *cellStart, uint *cellEnd, float *sortedPo
 /* gravlist.cu:144-171 + gravlist_kernel.cu:20-88,162-234.  Short-range P3M
  * force on every sorted particle from all particles within rcut, with the
  * constants of setSimParam/setSoftParam; gravAccel[gridParticleIndex[i]] =
- * (ax, ay, az, 0).  numCells = G^3 of the grid the keys were made on. */
+ * (ax, ay, az, 0).  numCells = G^3 of the grid the keys were made on.  A
+ * particle that no cell's range [cellStart, cellEnd) holds is neither source
+ * nor target: its gravAccel is left as it was.  (Ranges that leave particles
+ * out cost a second conversion and a copy of the particles.) */
 void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridParticleIndex,
                                  uint *cellStart, uint *cellEnd, uint numParticles,
                                  uint numCells);
