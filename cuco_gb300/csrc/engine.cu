@@ -104,20 +104,36 @@ __global__ void k_to_fixed(const float *__restrict__ a, float4 *__restrict__ b, 
     b[i] = make_float4(__uint_as_float(c[0]), __uint_as_float(c[1]), __uint_as_float(c[2]), 0.f);
 }
 
-// fixed point -> float positions in [0, L].  The product u * L / 2^32 in two
-// float parts of u, the upper 24 bits fused with the rounded lower 8 bits'
-// part: one rounding to 24 bits of a sum that is off by 2^-40 of the result at
-// most (a double product, which this replaces, ran at the FP64 rate: 512^3
-// 2.14 ms, now bound by memory).
-__global__ void k_from_fixed(const float4 *__restrict__ b, float *__restrict__ a, uint32_t n, float length_per_unit) {
+// fixed point -> float positions in [0, L]: u * L / 2^32 rounded to double and
+// then to float, as the double product has it, by integers.  L is mant * 2^e
+// with a 24-bit mant, so u * mant is exact in 64 bits; it is rounded to 53 bits
+// (to nearest even) and converted, and the power of two only shifts it.  Bound
+// by memory: 256^3 particles read back in 104 us, 353 with the double product,
+// which runs at the FP64 rate, and 89 with a float product in two parts, which
+// rounds the low 8 bits' part first and is off by up to 2^-25 of a small u.  A
+// box so small that the float result may be subnormal takes the double product.
+__global__ void k_from_fixed(const float4 *__restrict__ b, float *__restrict__ a, uint32_t n, uint32_t mant,
+                             float scale, double length_per_unit) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 v = b[i];
     const uint32_t u[3] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z)};
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
-        a[3 * (size_t)i + d] = __fmaf_rn((float)(u[d] >> 8), 256.0f * length_per_unit,
-                                         __fmul_rn((float)(u[d] & 255u), length_per_unit));
+    for (int d = 0; d < 3; ++d) {
+        float x;
+        if (scale != 0.f) {
+            uint64_t p = (uint64_t)u[d] * mant;
+            const int drop = 11 - __clzll((long long)p);  // bits beyond 53: 3 at most
+            if (drop > 0) {
+                const uint64_t unit = 1ull << drop;
+                p = (p + (unit >> 1) - 1 + ((p >> drop) & 1)) & ~(unit - 1);
+            }
+            x = __fmul_rn(__ull2float_rn(p), scale);
+        } else {
+            x = (float)((double)u[d] * length_per_unit);
+        }
+        a[3 * (size_t)i + d] = x;
+    }
 }
 
 __global__ void k_scatter4(const float4 *__restrict__ src_sorted, const uint32_t *__restrict__ perm,
@@ -270,7 +286,11 @@ cuco_status_t to_fixed(const float *a, float4 *b, uint32_t n, float boxsize, cud
 
 cuco_status_t from_fixed(const float4 *b, float *a, uint32_t n, float boxsize, cudaStream_t stream) {
     if (!n) return CUCO_OK;
-    k_from_fixed<<<(n + 255) / 256, 256, 0, stream>>>(b, a, n, ldexpf(boxsize, -32));
+    int e;
+    const uint32_t mant = (uint32_t)ldexpf(frexpf(boxsize, &e), 24);  // boxsize = mant 2^(e - 24)
+    // (the smallest position is 2^(e - 33) at least: far from subnormal for e >= -64)
+    const float scale = e >= -64 ? ldexpf(1.f, e - 56) : 0.f;
+    k_from_fixed<<<(n + 255) / 256, 256, 0, stream>>>(b, a, n, mant, scale, (double)boxsize / 4294967296.0);
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
 }
