@@ -598,6 +598,7 @@ __device__ __forceinline__ void shortrange_unit(
             }
             // what is left of the list (less than one iteration) moves to its front
             if (more) {
+                __syncwarp();  // (the rare-case pairs have read the list)
                 const uint32_t rest = cnt - n_eval;
                 // (forward, 32 at a time: n_eval >= rest, so nothing is overwritten before it is read)
                 for (uint32_t k = lane; k < rest; k += 32) {
