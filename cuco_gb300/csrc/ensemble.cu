@@ -940,15 +940,17 @@ cuco_status_t cuco_ensemble_footprint(const cuco_config_t *boxes, int nbox, uint
     for (int k = 0; k < nbox; ++k) {
         const uint64_t n = (uint64_t)boxes[k].n, M = (uint64_t)boxes[k].pm_grid;
         ntot += n;
-        const uint64_t G = boxes[k].cell_grid > 0 ? (uint64_t)boxes[k].cell_grid : M / 2;  // the largest tuned grid
+        // (the largest tuned grid)
+        const uint64_t G = boxes[k].cell_grid > 0 ? (uint64_t)boxes[k].cell_grid : std::max<uint64_t>(M / 2, 8);
         b += n * (6 * sizeof(float4) + 4 * sizeof(uint32_t));    // state, sorted copies, keys
         b += 4 * (G * G * G + 1) + 16 * G * G * G;               // cell offsets, z-slice counts
+        b += sizeof(uint4) * (uint64_t)shortrange_unit_cap((uint32_t)n, G * G * G);  // the work plan's units
         b += 12 * M * M * M + 8 * pm_spec_points((int)M);        // deposit + real grid + half spectrum
         b += 12 * (M / 2 + 1) + 8 * M + 2048 + 16 * (M * M);    // tables, descriptors, CTA maps
         maxn = std::max(maxn, n);
     }
     b += 12 * maxn + 4 * (uint64_t)kNTab;
-    b += 2 * 4 * 256 * (ntot / 4096 + 1);  // the sort's digit histogram (digits of at most 8 bits)
+    b += 4 * (uint64_t)sort_hist_entries((uint32_t)std::min<uint64_t>(ntot, 0xffffffffu), 8, 8);  // the sort's digit histogram
     *bytes = b;
     return CUCO_OK;
 }
