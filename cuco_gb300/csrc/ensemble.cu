@@ -99,16 +99,6 @@ int key_bits(uint64_t ncells) {
     return b;
 }
 
-template <typename T>
-cuco_status_t dalloc(T **p, size_t count) {
-    cudaError_t e = cudaMalloc(p, sizeof(T) * (count ? count : 1));
-    if (e != cudaSuccess) {
-        set_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        return CUCO_ERR_NOMEM;
-    }
-    return CUCO_OK;
-}
-
 // Ensemble arrays come from the device's stream-ordered pool, which keeps
 // freed memory for reuse (release threshold raised once per device): a
 // serving loop rebuilds its ensemble whenever jobs join or leave, and must not
@@ -210,71 +200,83 @@ int tune_cell_grid(const cuco_config_t &c0, cudaStream_t stream) {
 // of the mesh as fill the GPU (2^24 points): alone, a small mesh is fastest
 // in batches so small that its CTAs' threads idle, which is what a full
 // ensemble then pays (the z passes of 16 boxes of 16^3 to 80^3: 357 us for
-// batches timed alone, 260 for these).
-void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, int *P_out, int *B_out) {
+// batches timed alone, 260 for these).  They work in the ensemble's own meshes
+// (`room` points, `spec_room` of the spectrum; scratch between steps), so that
+// tuning takes no memory beside what the ensemble holds: an ensemble of few
+// points tunes for few.  The maps and tables lie in rho, and the potential is
+// written over the deposit.
+void tune_fft(int M, float boxsize, float asmth, cudaStream_t stream, float *rho, unsigned long long *rho64,
+              float2 *spec, size_t room, size_t spec_room, int *P_out, int *B_out) {
     *P_out = pm_batch_z(M);
     *B_out = pm_batch_axis(M);
     const size_t Mh = M / 2 + 1, points = (size_t)M * M * M;
-    const int copies = (int)std::min<size_t>(std::max<size_t>(((size_t)1 << 24) / points, 1), 64);
-    float *rho = nullptr, *green = nullptr;
-    unsigned long long *rho64 = nullptr;
-    float2 *spec = nullptr, *tw = nullptr;
-    PMBoxDesc *dd = nullptr;
-    uint32_t *pbeg = nullptr;
-    uint2 *mz = nullptr, *ma = nullptr;
-    bool ok = dalloc(&rho, points * copies) == CUCO_OK && dalloc(&rho64, points * copies) == CUCO_OK &&
-              dalloc(&spec, pm_spec_points(M) * copies) == CUCO_OK &&
-              dalloc(&green, Mh) == CUCO_OK && dalloc(&tw, (size_t)M) == CUCO_OK &&
-              dalloc(&dd, (size_t)copies) == CUCO_OK && dalloc(&pbeg, (size_t)copies + 1) == CUCO_OK &&
-              dalloc(&mz, (size_t)M * M * copies) == CUCO_OK && dalloc(&ma, (size_t)M * Mh * copies) == CUCO_OK;
+    const size_t fit = std::min(room / points, spec_room / pm_spec_points(M));
+    const int copies = (int)std::min<size_t>({std::max<size_t>(((size_t)1 << 24) / points, 1), 64, fit});
+    if (copies < 1) return;
+    // in rho (4 M bytes a row, of which these take about 5): descriptors, z map,
+    // axis map, twiddles, Green's factors, particle bounds
+    char *at = reinterpret_cast<char *>(rho);
+    auto take = [&](auto **p, size_t count) {
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(at);
+        at += (sizeof(**p) * count + 15) / 16 * 16;
+    };
+    PMBoxDesc *dd;
+    uint2 *mz, *ma;
+    float2 *tw;
+    float *green;
+    uint32_t *pbeg;
+    take(&dd, (size_t)copies);
+    take(&mz, (size_t)M * M / 2 * copies);
+    take(&ma, (size_t)M * ((Mh + 3) / 4) * copies);
+    take(&tw, (size_t)M);
+    take(&green, Mh);
+    take(&pbeg, (size_t)copies + 1);
+    if (at > reinterpret_cast<char *>(rho) + sizeof(float) * points * copies) return;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
-    if (ok) {
-        std::vector<float> g(Mh);
-        std::vector<float2> t(M);
-        pm_tables(M, boxsize, asmth, g.data(), t.data());
-        cudaMemcpy(green, g.data(), sizeof(float) * Mh, cudaMemcpyHostToDevice);
-        cudaMemcpy(tw, t.data(), sizeof(float2) * M, cudaMemcpyHostToDevice);
-        cudaMemset(rho, 0, sizeof(float) * points * copies);
-        cudaMemset(pbeg, 0, sizeof(uint32_t) * (copies + 1));
-        cudaEventCreate(&e0);
-        cudaEventCreate(&e1);
-        float best = 1e30f;
-        for (int P : {1, 2, 4, 8, 16}) {
-            if (P > M / 2 || (M * M / 2) % P || pm_smem_z(M, P) > 200 * 1024) continue;
-            for (int B : {4, 8, 16}) {
-                if (pm_smem_axis(M, B) > 200 * 1024 || !pm_fft_batches_ok(M, P, B)) continue;
-                const uint32_t nz = (uint32_t)(M * M / (2 * P)), na = (uint32_t)((Mh + B - 1) / B) * M;
-                std::vector<PMBoxDesc> d;
-                std::vector<uint2> vz, va;
-                for (int k = 0; k < copies; ++k) {
-                    d.push_back(PMBoxDesc{M, P, B, pm_stage_plan(M), 1.f, 0.f, 0.f, rho + points * k,
-                                          rho64 + points * k, 1.f, spec + pm_spec_points(M) * k, green, tw});
-                    for (uint32_t i = 0; i < nz; ++i) vz.push_back(make_uint2(k, i));
-                    for (uint32_t i = 0; i < na; ++i) va.push_back(make_uint2(k, i));
-                }
-                cudaMemcpy(dd, d.data(), sizeof(PMBoxDesc) * d.size(), cudaMemcpyHostToDevice);
-                cudaMemcpy(mz, vz.data(), sizeof(uint2) * vz.size(), cudaMemcpyHostToDevice);
-                cudaMemcpy(ma, va.data(), sizeof(uint2) * va.size(), cudaMemcpyHostToDevice);
-                PMMulti m{copies, false, dd, pbeg, mz, ma, (uint32_t)vz.size(), (uint32_t)va.size(),
-                          pm_smem_z(M, P), pm_smem_axis(M, B), rho64, points * copies};
-                m.big = pm_big_fft(M, P, B);
-                m.wide = pm_wide_stages(pm_stage_plan(M));
-                if (pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr) != CUCO_OK) continue;  // warm-up
-                cudaEventRecord(e0, stream);
-                for (int r = 0; r < 3; ++r) pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr);
-                cudaEventRecord(e1, stream);
-                if (cudaEventSynchronize(e1) != cudaSuccess) continue;
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (ms < best) best = ms, *P_out = P, *B_out = B;
+    std::vector<float> g(Mh);
+    std::vector<float2> t(M);
+    pm_tables(M, boxsize, asmth, g.data(), t.data());
+    cudaStreamSynchronize(stream);  // (the copies below are not on the stream)
+    cudaMemcpy(green, g.data(), sizeof(float) * Mh, cudaMemcpyHostToDevice);
+    cudaMemcpy(tw, t.data(), sizeof(float2) * M, cudaMemcpyHostToDevice);
+    cudaMemset(pbeg, 0, sizeof(uint32_t) * (copies + 1));
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    float best = 1e30f;
+    for (int P : {1, 2, 4, 8, 16}) {
+        if (P > M / 2 || (M * M / 2) % P || pm_smem_z(M, P) > 200 * 1024) continue;
+        for (int B : {4, 8, 16}) {
+            if (pm_smem_axis(M, B) > 200 * 1024 || !pm_fft_batches_ok(M, P, B)) continue;
+            const uint32_t nz = (uint32_t)(M * M / (2 * P)), na = (uint32_t)((Mh + B - 1) / B) * M;
+            std::vector<PMBoxDesc> d;
+            std::vector<uint2> vz, va;
+            for (int k = 0; k < copies; ++k) {
+                d.push_back(PMBoxDesc{M, P, B, pm_stage_plan(M), 1.f, 0.f, 0.f,
+                                      reinterpret_cast<float *>(rho64 + points * k), rho64 + points * k, 1.f,
+                                      spec + pm_spec_points(M) * k, green, tw});
+                for (uint32_t i = 0; i < nz; ++i) vz.push_back(make_uint2(k, i));
+                for (uint32_t i = 0; i < na; ++i) va.push_back(make_uint2(k, i));
             }
+            cudaMemcpy(dd, d.data(), sizeof(PMBoxDesc) * d.size(), cudaMemcpyHostToDevice);
+            cudaMemcpy(mz, vz.data(), sizeof(uint2) * vz.size(), cudaMemcpyHostToDevice);
+            cudaMemcpy(ma, va.data(), sizeof(uint2) * va.size(), cudaMemcpyHostToDevice);
+            PMMulti m{copies, false, dd, pbeg, mz, ma, (uint32_t)vz.size(), (uint32_t)va.size(),
+                      pm_smem_z(M, P), pm_smem_axis(M, B), rho64, points * copies};
+            m.big = pm_big_fft(M, P, B);
+            m.wide = pm_wide_stages(pm_stage_plan(M));
+            if (pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr) != CUCO_OK) continue;  // warm-up
+            cudaEventRecord(e0, stream);
+            for (int r = 0; r < 3; ++r) pm_forces_multi(m, nullptr, 0, nullptr, stream, nullptr);
+            cudaEventRecord(e1, stream);
+            if (cudaEventSynchronize(e1) != cudaSuccess) continue;
+            float ms = 0.f;
+            cudaEventElapsedTime(&ms, e0, e1);
+            if (ms < best) best = ms, *P_out = P, *B_out = B;
         }
     }
     cudaGetLastError();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    cudaFree(rho), cudaFree(rho64), cudaFree(spec), cudaFree(green), cudaFree(tw), cudaFree(dd), cudaFree(pbeg), cudaFree(mz),
-        cudaFree(ma);
 }
 
 }  // namespace
@@ -472,33 +474,33 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     drop_graph(e);
     std::vector<cuco_config_t> cfg(boxes, boxes + nbox);
     std::vector<int> P(nbox), B(nbox);
-    // autotune: cell grid and FFT batching per (n, M, mode)
+    // autotune: cell grid and FFT batching per (n, M, mode); the grids first, on
+    // scratch boxes, then the batching, in the ensemble's meshes
+    using Key = std::tuple<int64_t, int, int>;
+    std::map<Key, Tuned> tuned;
+    std::vector<int> fresh;  // a box of each size that was not tuned before
     for (int b = 0; b < nbox; ++b) {
-        cuco_config_t &c = cfg[b];
-        const auto key = std::make_tuple(c.n, c.pm_grid, (int)c.mode);
-        Tuned t{};
-        bool cached;
+        const cuco_config_t &c = cfg[b];
+        const Key key(c.n, c.pm_grid, (int)c.mode);
+        if (tuned.count(key)) continue;
         {
             std::lock_guard<std::mutex> lk(g_tune_mu);
             auto it = g_tune_cache.find(key);
-            cached = it != g_tune_cache.end();
-            if (cached) t = it->second;
-        }
-        if (!cached) {
-            t.cell_grid = tune_cell_grid(c, st);
-            tune_fft(c.pm_grid, c.boxsize, c.asmth, st, &t.P, &t.B);
-            std::lock_guard<std::mutex> lk(g_tune_mu);
-            g_tune_cache[key] = t;
-        }
-        if (c.cell_grid <= 0) {
-            if (t.cell_grid <= 0) {
-                set_error("ensemble: no admissible cell grid for a box");
-                return CUCO_ERR_UNSUPPORTED;
+            if (it != g_tune_cache.end()) {
+                tuned[key] = it->second;
+                continue;
             }
-            c.cell_grid = t.cell_grid;
         }
-        P[b] = t.P;
-        B[b] = t.B;
+        tuned[key].cell_grid = tune_cell_grid(c, st);
+        fresh.push_back(b);
+    }
+    for (cuco_config_t &c : cfg) {
+        if (c.cell_grid > 0) continue;
+        c.cell_grid = tuned[Key(c.n, c.pm_grid, (int)c.mode)].cell_grid;
+        if (c.cell_grid <= 0) {
+            set_error("ensemble: no admissible cell grid for a box");
+            return CUCO_ERR_UNSUPPORTED;
+        }
     }
     // sizes and offsets
     std::vector<uint32_t> pbeg(nbox + 1, 0);
@@ -519,6 +521,22 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     if (cbase[nbox] >= 0xffffffffull || (uint64_t)pbeg[nbox] > 0xfffffff0ull) {
         set_error("ensemble: more than 2^32 cells or particles in total");
         return CUCO_ERR_UNSUPPORTED;
+    }
+    CUCO_TRY(grow(e->rho, e->cap_mesh, mbase[nbox], st));
+    CUCO_TRY(grow(e->rho64, e->cap_mesh64, mbase[nbox], st));
+    CUCO_TRY(grow(e->spec, e->cap_spec, sbase[nbox], st));
+    for (int b : fresh) {
+        const cuco_config_t &c = cfg[b];
+        const Key key(c.n, c.pm_grid, (int)c.mode);
+        Tuned &t = tuned[key];
+        tune_fft(c.pm_grid, c.boxsize, c.asmth, st, e->rho, e->rho64, e->spec, mbase[nbox], sbase[nbox], &t.P, &t.B);
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        g_tune_cache[key] = t;
+    }
+    for (int b = 0; b < nbox; ++b) {
+        const Tuned &t = tuned[Key(cfg[b].n, cfg[b].pm_grid, (int)cfg[b].mode)];
+        P[b] = t.P;
+        B[b] = t.B;
     }
     const size_t n = pbeg[nbox];
     const uint64_t ncells = cbase[nbox];
@@ -585,8 +603,6 @@ cuco_status_t ensemble_layout(cuco_ensemble *e, const cuco_config_t *boxes, int 
     const size_t nbc = (size_t)nbox + 1;
     if ((s = grow(e->hist, e->cap_hist, sort_hist_entries((uint32_t)n, kbits, 8), st)) ||
         (s = grow(e->cell_off, e->cap_cells, ncells + 1, st)) || (s = grow(e->cell_sl, e->cap_cellsl, ncells, st)) || (s = grow(e->stage3, e->cap_stage3, 3 * maxn, st)) ||
-        (s = grow(e->rho, e->cap_mesh, mbase[nbox], st)) ||
-        (s = grow(e->rho64, e->cap_mesh64, mbase[nbox], st)) || (s = grow(e->spec, e->cap_spec, sbase[nbox], st)) ||
         (s = grow(e->green, e->cap_green, gbase[nbox], st)) || (s = grow(e->tw, e->cap_tw, tbase[nbox], st)) ||
         (s = grow(e->table, e->cap_table, (size_t)kNTab, st)) || (s = grow(e->d_pbeg, e->cap_pbeg, nbc, st)) ||
         (s = grow(e->d_segbase, e->cap_segbase, nbc, st)) || (s = grow(e->d_drift, e->cap_drift, nbc, st)) ||
