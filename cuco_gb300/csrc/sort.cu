@@ -821,7 +821,7 @@ namespace {
 constexpr uint32_t kOffWideCells = 1u << 22;
 
 struct RunningEnd {
-    static __device__ __forceinline__ uint32_t of(uint32_t, uint32_t e) { return e; }
+    static __device__ __forceinline__ uint32_t of(uint32_t s, uint32_t e) { return e > s ? e : 0u; }
     static __device__ __forceinline__ uint32_t join(uint32_t a, uint32_t b) { return max(a, b); }
     static __device__ __forceinline__ uint32_t warp(uint32_t v) { return __reduce_max_sync(kFull, v); }
 };
@@ -833,7 +833,8 @@ struct RunningCount {
 
 // A warp takes 32 * ITEMS consecutive cells, a lane every 32nd of them (the
 // caller's arrays need no alignment beyond a word's): the value of each, 0 for
-// an empty one (s its start, kEmptyCell).
+// one that is empty (kEmptyCell for a start, or an end not above it); s its
+// start.
 template <uint32_t ITEMS>
 __device__ __forceinline__ uint32_t first_cell() {
     return (blockIdx.x * kSortWarps + (threadIdx.x >> 5)) * (32 * ITEMS) + (threadIdx.x & 31);
@@ -949,7 +950,7 @@ __global__ void __launch_bounds__(kSortThreads) k_cell_offsets(const uint32_t *_
     for (uint32_t k = 0; k < ITEMS; ++k) {
         const uint32_t off = Op::join(carry, lanes_before<Op>(v[k], &all));
         if (c0 + 32 * k < ncells) cell_off[c0 + 32 * k] = off;
-        apart |= s[k] != kEmptyCell && s[k] != off;
+        apart |= v[k] != 0 && s[k] != off;
         carry = Op::join(carry, all);
         if (c0 + 32 * k == ncells - 1) cell_off[ncells] = Op::join(off, v[k]);
     }

@@ -1,6 +1,7 @@
 """Bounds given to cudaForceEvaluateShortrange that leave particles out: cells
-marked empty (0xffffffff) whose particles are still in the sorted array, single
-cells and whole columns of them, at both ends and in between.  The particles of
+marked empty (0xffffffff, or an end not above the start) whose particles are
+still in the sorted array, single cells and whole columns of them, at both ends
+and in between.  The particles of
 the other cells get the forces of a box that holds only them (against the CPU
 oracle, rms relative 1e-4), the others are neither sources nor targets: their
 accelerations are left as they were."""
@@ -16,8 +17,9 @@ pytestmark = pytest.mark.gpu
 G = 32
 
 
+@pytest.mark.parametrize("mark", [0xFFFFFFFF, 5])
 @pytest.mark.parametrize("masked", ["column", "cells", "first", "last", "none"])
-def test_masked_cells(port, masked):
+def test_masked_cells(port, masked, mark):
     rng = np.random.default_rng(11)
     n = 20000
     pos = rng.uniform(0, L, size=(n, 3)).astype(np.float32)
@@ -25,7 +27,9 @@ def test_masked_cells(port, masked):
     cells = torch.arange(g.ncell, device="cuda:0")
     keep = {"column": (cells // G) % 7 != 3, "cells": cells % 5 != 2, "first": cells >= 9 * G + 5,
             "last": cells < g.ncell - 6 * G - 11, "none": cells >= 0}[masked]
-    g.start[~keep] = -1
+    g.start[~keep] = np.uint32(mark).astype(np.int32).item()
+    if mark == 5:
+        g.end[~keep] = 5
     covered = keep[g.keys.long()].cpu().numpy()  # in sorted order
     at = g.perm.cpu().numpy()[covered]
     g.acc[:] = 7.0
