@@ -1343,7 +1343,7 @@ __global__ void k_interp_multi(const float4 *__restrict__ pos, uint32_t n, const
 int fft_batch_z(int M) {
     int P = 4096 / M;
     if (P > 16) P = 16;
-    if (P > M / 2) P = M / 2;  // k_fft_z_c2r stages 2P rows of M/2+1 in an M*(P+1) buffer
+    if (P > M / 2) P = M / 2;
     if (P < 1) P = 1;
     P = 1 << ilog2(P);
     // P pairs per CTA must divide the M*M/2 row pairs

@@ -222,7 +222,7 @@ __device__ __forceinline__ bool bar_wait_bounded(uint64_t *bar, uint32_t parity,
 // copies that are never issued, waits at most `limit` cycles, and reports
 // through the short range's timeout word.  No copy is in flight when it gives
 // up.  (The short range itself waits on nothing.)
-__global__ void k_staging_timeout_probe(uint32_t *__restrict__ err, long long limit) {
+__global__ void k_timeout_probe(uint32_t *__restrict__ err, long long limit) {
     if (threadIdx.x == 0) bar_init(&g_probe_bar);
     __syncthreads();
     if (threadIdx.x == 0) bar_arrive_expect(&g_probe_bar, 16u);
@@ -836,7 +836,7 @@ bool build_columns(const ShortRangeParams &p, ColumnSet *cs) {
     // segment length: a power of two dividing G, with the S + 2R z-cells of a
     // column at most G (so a column's z range wraps at most once)
     int S = kMaxSeg;
-    // fixed point also needs every staged source within G/2 cells of the
+    // fixed point also needs every source within G/2 cells of the
     // segment corner (the int32 difference is the periodic image)
     auto bad = [&](int s) { return p.grid % s || p.grid < s + 2 * R || (p.fixed && 2 * (s + R) >= p.grid); };
     while (S > 1 && bad(S)) S >>= 1;
@@ -886,7 +886,7 @@ uint32_t shortrange_unit_cap(uint32_t n, uint64_t segments) {
 }
 
 cuco_status_t shortrange_timeout_probe(uint32_t *ctl, long long limit_cycles, cudaStream_t stream) {
-    k_staging_timeout_probe<<<1, kThreads, 0, stream>>>(ctl + 3, limit_cycles);
+    k_timeout_probe<<<1, kThreads, 0, stream>>>(ctl + 3, limit_cycles);
     CUCO_TRY_CUDA(cudaGetLastError());
     return shortrange_check(ctl, stream);
 }
@@ -897,7 +897,7 @@ cuco_status_t shortrange_check(uint32_t *ctl, cudaStream_t stream) {
     CUCO_TRY_CUDA(cudaStreamSynchronize(stream));
     if (flag) {
         CUCO_TRY_CUDA(cudaMemsetAsync(ctl + 3, 0, sizeof(uint32_t), stream));
-        set_error("short range: a bulk-copy wait into shared memory gave up after ~1 s; forces are invalid");
+        set_error("short range: a bounded wait gave up; forces are invalid");
         return CUCO_ERR_TIMEOUT;
     }
     return CUCO_OK;
