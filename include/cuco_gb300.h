@@ -236,7 +236,9 @@ cuco_status_t cuco_box_create(const cuco_config_t *cfg, cuco_box_t **box);
 cuco_status_t cuco_box_destroy(cuco_box_t *box);
 
 /* State in original particle order, n x 3 floats each.  `on_device` selects
- * whether the pointers are device (1) or host (0) memory.  vel is the
+ * whether the pointers are device (1) or host (0) memory.  Device arrays of the
+ * box's own GPU are read and written in place (aligned as floats), others
+ * through the box's staging array, by copies.  vel is the
  * integrator's variable a^2 dx/dt (the reference's P[].Vel after init.c:30). */
 cuco_status_t cuco_box_set_state(cuco_box_t *box, const float *pos, const float *vel,
                                  int on_device);
