@@ -124,7 +124,8 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
     KickArgs k{};
     // the work plan's scratch, grown on demand (like the reference's device
     // arrays, held until exit)
-    static SRWork w{};  // ctl[4]: blocks that the conversion has finished, ctl[5]: the bounds have gaps
+    static SRWork w{};  // ctl[3] has kGap too where the bounds have gaps, ctl[4]: blocks that the conversion has finished
+    constexpr uint32_t kGap = 2;
     static uint32_t *off = nullptr;  // cell offsets, then the conversion's scratch
     static size_t off_cap = 0;
     const char *const me = "cudaForceEvaluateShortrange";
@@ -148,21 +149,21 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
         off_cap = off_need;
     }
     uint32_t *const scratch = off + numCells + 1;
-    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, scratch, w.ctl + 4, w.ctl + 5, 0), me);
+    capi_status(launch_start_end_offsets(cellStart, cellEnd, off, numCells, scratch, w.ctl + 4, w.ctl + 3, kGap, 0), me);
     capi_status(launch_shortrange(p, (const float4 *)sortedPos, gridParticleIndex, off, s.table, (float4 *)gravAccel,
-                                  k, w, false, 0, nullptr, nullptr, nullptr, w.ctl + 5),
+                                  k, w, false, 0, nullptr, nullptr, nullptr, w.ctl + 3),
                 me);
-    uint32_t seen[3];  // the timeout word, ctl[4], ctl[5]
-    capi_check(cudaMemcpyAsync(seen, w.ctl + 3, sizeof seen, cudaMemcpyDeviceToHost, 0), me);
+    uint32_t seen = 0;
+    capi_check(cudaMemcpyAsync(&seen, w.ctl + 3, sizeof seen, cudaMemcpyDeviceToHost, 0), me);
     capi_check(cudaStreamSynchronize(0), me);
-    if (seen[2]) {
+    if (seen & kGap) {
         // Cells whose ranges leave particles out (or overlap): nothing has been
         // evaluated yet.  The engine's offsets cannot say it; the cells' own
         // particles are laid one after the other first.
         static float4 *pos = nullptr;
         static uint32_t *perm = nullptr;
         static uint32_t held = 0;
-        capi_check(cudaMemsetAsync(w.ctl + 5, 0, sizeof(uint32_t), 0), me);
+        capi_check(cudaMemsetAsync(w.ctl + 3, 0, sizeof(uint32_t), 0), me);
         capi_status(launch_start_end_counts(cellStart, cellEnd, off, numCells, scratch, w.ctl + 4, 0), me);
         capi_check(cudaMemcpyAsync(&p.n, off + numCells, sizeof(uint32_t), cudaMemcpyDeviceToHost, 0), me);
         capi_check(cudaStreamSynchronize(0), me);
@@ -180,7 +181,7 @@ void cudaForceEvaluateShortrange(float *gravAccel, float *sortedPos, uint *gridP
                     me);
         capi_status(launch_shortrange(p, pos, perm, off, s.table, (float4 *)gravAccel, k, w, false, 0), me);
     }
-    if (seen[0] || seen[2]) capi_status(shortrange_check(w.ctl, 0), me);
+    if (seen) capi_status(shortrange_check(w.ctl, 0), me);
 }
 
 // what a caller's `counters` holds at least (the reference RadixSort's allocation)

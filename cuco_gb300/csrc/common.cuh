@@ -167,13 +167,13 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_
 
 // The reference's cell bounds (cell_end is read where cell_start is not
 // empty) -> the engine's offsets (ncells + 1), where the cells' ranges follow
-// one another; *gap (0 before) is set where they do not.  scratch:
+// one another; gap_bit is set in *gap where they do not.  scratch:
 // offsets_scratch(ncells) words; finished: a word that is 0 and is 0 again
 // afterwards.
 size_t offsets_scratch(uint32_t ncells);
 cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
                                        uint32_t ncells, uint32_t *scratch, uint32_t *finished, uint32_t *gap,
-                                       cudaStream_t stream);
+                                       uint32_t gap_bit, cudaStream_t stream);
 
 // The same for ranges with gaps: the offsets that the cells' particles have
 // when they are laid one after the other, and that layout of them.

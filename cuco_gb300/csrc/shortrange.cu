@@ -677,8 +677,7 @@ __device__ __forceinline__ void shortrange_unit(
 
 __global__ void k_sr_plan(const __grid_constant__ SRPlan plan, const uint32_t *__restrict__ cell_off,
                           const uint32_t *__restrict__ hold, const __grid_constant__ SRWork w) {
-    if (hold && *hold) return;
-    plan_box_segment(plan, blockIdx.x * blockDim.x + threadIdx.x, cell_off, 0u, 0u, w);
+    plan_box_segment(plan, blockIdx.x * blockDim.x + threadIdx.x, cell_off, 0u, 0u, w, hold);
 }
 
 // The next unit for a warp: the dense slices first (the longest work).  Takes

@@ -62,13 +62,16 @@ __device__ __forceinline__ void plan_segment(uint32_t tb, uint32_t nt, uint32_t 
 }
 
 // Segment `seg` of a box of G^3 cells (segments are numbered in cell order).
+// hold (or null): where it is not 0, nothing is planned.
 __device__ __forceinline__ void plan_box_segment(const SRPlan &plan, uint32_t seg, const uint32_t *__restrict__ cell_off,
-                                                 uint32_t cell_base, uint32_t box, const SRWork &w) {
+                                                 uint32_t cell_base, uint32_t box, const SRWork &w,
+                                                 const uint32_t *__restrict__ hold = nullptr) {
     uint32_t tb = 0, nt = 0, ix = 0, iy = 0, iz = 0;
     if (seg < plan.nseg) {
         const uint32_t c0 = cell_base + seg * (uint32_t)plan.S;
         tb = cell_off[c0];
         nt = cell_off[c0 + plan.S] - tb;
+        if (hold && *hold) nt = 0;
         const uint32_t segs = plan.G / plan.S, row = seg / segs;
         iz = (seg - row * segs) * plan.S;
         ix = row / plan.G;

@@ -810,15 +810,18 @@ cuco_status_t launch_reorder_offsets(uint32_t *cell_off, const uint32_t *sorted_
 // of the cells before c, a running maximum; a range that does not start there is
 // reported.  Where they do not, off[c] is the particles that the cells before c
 // hold, a running sum, for a copy of the particles in that order.  Either takes
-// two launches: each block's value, which the last block to finish turns into
-// the value before each block; then every block its cells.  Bound by memory:
-// both bounds read twice.  (Every block of the second launch used to read the
-// maxima of all blocks before it, which is quadratic in the cells: a force on
-// 1000 particles in 512^3, 768^3 and 1024^3 cells took 1.90, 21.1 and 116 ms,
-// so 0.76, 2.14 and 4.88; on 64^3 cells 32^3 particles take 122 us either way.)
+// two launches: each block's value, then every block its cells after the values
+// of the blocks before it.  Up to kDirectBlocks blocks, each reads those values
+// itself; beyond, which would be quadratic in the cells, the last block of the
+// first launch to finish turns them into running values (at few blocks that
+// costs 5 us of latency).  Bound by memory: both bounds read twice.  A force on
+// 1000 particles in 512^3, 768^3 and 1024^3 cells: 1.81, 21.0 and 116 ms with
+// every block reading all values before it, 0.54, 1.66 and 3.86 so; on 32^3
+// particles in 64^3 and 256^3 cells 0.108 and 0.206 ms, 0.108 and 0.195.
 namespace {
-// cells a thread: 4, or 16 from kOffWideCells cells (fewer blocks to scan)
-constexpr uint32_t kOffWideCells = 1u << 22;
+constexpr unsigned kDirectBlocks = 4096;
+// 4 cells a thread; 16 from kOffWideCells cells
+constexpr uint32_t kOffWideCells = 1u << 20;
 
 struct RunningEnd {
     static __device__ __forceinline__ uint32_t of(uint32_t s, uint32_t e) { return e > s ? e : 0u; }
@@ -831,32 +834,49 @@ struct RunningCount {
     static __device__ __forceinline__ uint32_t warp(uint32_t v) { return __reduce_add_sync(kFull, v); }
 };
 
-// A warp takes 32 * ITEMS consecutive cells, a lane every 32nd of them (the
-// caller's arrays need no alignment beyond a word's): the value of each, 0 for
-// one that is empty (kEmptyCell for a start, or an end not above it); s its
-// start.
-template <uint32_t ITEMS>
+// The caller's bounds; wide: both on 16 bytes.
+struct CellBounds {
+    const uint32_t *start, *end;
+    uint32_t ncells;
+    bool wide;
+};
+
+// Cells c .. c + 3 of an array, `past` beyond the last.
+__device__ __forceinline__ uint4 load_four(const uint32_t *__restrict__ p, uint32_t c, const CellBounds &b, uint32_t past) {
+    if (b.wide && c + 3 < b.ncells) return *reinterpret_cast<const uint4 *>(p + c);
+    return make_uint4(c < b.ncells ? p[c] : past, c + 1 < b.ncells ? p[c + 1] : past, c + 2 < b.ncells ? p[c + 2] : past,
+                      c + 3 < b.ncells ? p[c + 3] : past);
+}
+
+// A warp takes ROUNDS times 128 consecutive cells, a lane four neighbours of
+// each: their starts and values, 0 for a cell that is empty (kEmptyCell for a
+// start, or an end not above it).
+template <uint32_t ROUNDS>
 __device__ __forceinline__ uint32_t first_cell() {
-    return (blockIdx.x * kSortWarps + (threadIdx.x >> 5)) * (32 * ITEMS) + (threadIdx.x & 31);
+    return (blockIdx.x * kSortWarps + (threadIdx.x >> 5)) * (128 * ROUNDS) + (threadIdx.x & 31) * 4;
 }
-template <typename Op, uint32_t ITEMS>
-__device__ __forceinline__ void load_cells(const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-                                           uint32_t ncells, uint32_t (&s)[ITEMS], uint32_t (&v)[ITEMS]) {
-    const uint32_t c0 = first_cell<ITEMS>();
-    uint32_t e[ITEMS];
+template <typename Op, uint32_t ROUNDS>
+__device__ __forceinline__ void load_cells(const CellBounds &b, uint4 (&s)[ROUNDS], uint4 (&v)[ROUNDS]) {
+    const uint32_t c0 = first_cell<ROUNDS>();
 #pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) {
-        s[k] = c0 + 32 * k < ncells ? start[c0 + 32 * k] : kEmptyCell;
-        e[k] = c0 + 32 * k < ncells ? end[c0 + 32 * k] : 0u;
+    for (uint32_t k = 0; k < ROUNDS; ++k) {
+        s[k] = load_four(b.start, c0 + 128 * k, b, kEmptyCell);
+        v[k] = load_four(b.end, c0 + 128 * k, b, 0u);
     }
+    auto value = [](uint32_t st, uint32_t e) { return st != kEmptyCell ? Op::of(st, e) : 0u; };
 #pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) v[k] = s[k] != kEmptyCell ? Op::of(s[k], e[k]) : 0u;
+    for (uint32_t k = 0; k < ROUNDS; ++k)
+        v[k] = make_uint4(value(s[k].x, v[k].x), value(s[k].y, v[k].y), value(s[k].z, v[k].z), value(s[k].w, v[k].w));
 }
-template <typename Op, uint32_t ITEMS>
-__device__ __forceinline__ uint32_t joined(const uint32_t (&v)[ITEMS]) {
+template <typename Op>
+__device__ __forceinline__ uint32_t joined(const uint4 &v) {
+    return Op::join(Op::join(v.x, v.y), Op::join(v.z, v.w));
+}
+template <typename Op, uint32_t ROUNDS>
+__device__ __forceinline__ uint32_t warp_joined(const uint4 (&v)[ROUNDS]) {
     uint32_t m = 0;
 #pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) m = Op::join(m, v[k]);
+    for (uint32_t k = 0; k < ROUNDS; ++k) m = Op::join(m, joined<Op>(v[k]));
     return Op::warp(m);
 }
 
@@ -894,21 +914,24 @@ __device__ __forceinline__ uint32_t lanes_before(uint32_t v, uint32_t *all) {
     return lane ? before : 0u;
 }
 
-// before[b] = the value before block b's cells.  *finished counts the blocks
-// that have written theirs; it is 0 between launches.
-template <typename Op, uint32_t ITEMS>
-__global__ void __launch_bounds__(kSortThreads) k_block_values(const uint32_t *__restrict__ start,
-                                                               const uint32_t *__restrict__ end, uint32_t ncells,
-                                                               uint32_t *before, uint32_t *finished) {
+// values[b] = block b's value; with `finished`, which counts the blocks that
+// have written theirs and is 0 between launches, the value before block b.
+template <typename Op, uint32_t ROUNDS>
+__global__ void __launch_bounds__(kSortThreads)
+    k_block_values(const __grid_constant__ CellBounds bounds, uint32_t *values, uint32_t *finished) {
     __shared__ bool s_last;
-    uint32_t s[ITEMS], v[ITEMS], all;
-    load_cells<Op>(start, end, ncells, s, v);
-    warps_before<Op>(joined<Op>(v), &all);
+    uint4 s[ROUNDS], v[ROUNDS];
+    uint32_t all;
+    load_cells<Op>(bounds, s, v);
+    warps_before<Op>(warp_joined<Op>(v), &all);
     if (threadIdx.x == 0) {
-        __stcg(&before[blockIdx.x], all);
-        __threadfence();
-        s_last = atomicAdd(finished, 1u) == gridDim.x - 1;
+        __stcg(&values[blockIdx.x], all);
+        if (finished) {
+            __threadfence();
+            s_last = atomicAdd(finished, 1u) == gridDim.x - 1;
+        }
     }
+    if (!finished) return;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
@@ -920,7 +943,7 @@ __global__ void __launch_bounds__(kSortThreads) k_block_values(const uint32_t *_
 #pragma unroll
         for (uint32_t k = 0; k < kAhead; ++k) {
             const uint32_t b = b0 + k * kSortThreads + threadIdx.x;
-            x[k] = b < gridDim.x ? __ldcg(&before[b]) : 0u;
+            x[k] = b < gridDim.x ? __ldcg(&values[b]) : 0u;
         }
 #pragma unroll
         for (uint32_t k = 0; k < kAhead; ++k) {
@@ -928,44 +951,72 @@ __global__ void __launch_bounds__(kSortThreads) k_block_values(const uint32_t *_
             uint32_t warp_all, round_all;
             const uint32_t lanes = lanes_before<Op>(x[k], &warp_all);
             const uint32_t at = Op::join(Op::join(carry, warps_before<Op>(warp_all, &round_all)), lanes);
-            if (b < gridDim.x) __stcg(&before[b], at);
+            if (b < gridDim.x) __stcg(&values[b], at);
             carry = Op::join(carry, round_all);
         }
     }
     if (threadIdx.x == 0) *finished = 0;
 }
 
-// gap (or null): set where a cell's range does not start at its offset.
-template <typename Op, uint32_t ITEMS>
-__global__ void __launch_bounds__(kSortThreads) k_cell_offsets(const uint32_t *__restrict__ start,
-                                                               const uint32_t *__restrict__ end, uint32_t ncells,
-                                                               const uint32_t *__restrict__ block_before,
-                                                               uint32_t *__restrict__ cell_off, uint32_t *gap) {
-    uint32_t s[ITEMS], v[ITEMS], all;
-    load_cells<Op>(start, end, ncells, s, v);
-    uint32_t carry = Op::join(block_before[blockIdx.x], warps_before<Op>(joined<Op>(v), &all));
-    const uint32_t c0 = first_cell<ITEMS>();
+// running: values[b] is the value before block b, else block b's own.  gap (or
+// null): gap_bit is set where a cell's range does not start at its offset.
+// cell_off lies on 16 bytes.
+template <typename Op, uint32_t ROUNDS>
+__global__ void __launch_bounds__(kSortThreads)
+    k_cell_offsets(const __grid_constant__ CellBounds bounds, const uint32_t *__restrict__ values, bool running,
+                   uint32_t *__restrict__ cell_off, uint32_t *gap, uint32_t gap_bit) {
+    uint4 s[ROUNDS], v[ROUNDS];
+    uint32_t all, carry = 0;
+    load_cells<Op>(bounds, s, v);
+    if (running) {
+        carry = values[blockIdx.x];
+    } else {
+#pragma unroll 4
+        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kSortThreads) carry = Op::join(carry, values[b]);
+        warps_before<Op>(Op::warp(carry), &all);
+        carry = all;
+    }
+    carry = Op::join(carry, warps_before<Op>(warp_joined<Op>(v), &all));
+    const uint32_t c0 = first_cell<ROUNDS>();
     bool apart = false;
 #pragma unroll
-    for (uint32_t k = 0; k < ITEMS; ++k) {
-        const uint32_t off = Op::join(carry, lanes_before<Op>(v[k], &all));
-        if (c0 + 32 * k < ncells) cell_off[c0 + 32 * k] = off;
-        apart |= v[k] != 0 && s[k] != off;
+    for (uint32_t k = 0; k < ROUNDS; ++k) {
+        const uint32_t c = c0 + 128 * k;
+        uint4 o;
+        o.x = Op::join(carry, lanes_before<Op>(joined<Op>(v[k]), &all));
+        o.y = Op::join(o.x, v[k].x);
+        o.z = Op::join(o.y, v[k].y);
+        o.w = Op::join(o.z, v[k].z);
+        if (c + 3 < bounds.ncells) {
+            *reinterpret_cast<uint4 *>(cell_off + c) = o;
+        } else {
+            if (c < bounds.ncells) cell_off[c] = o.x;
+            if (c + 1 < bounds.ncells) cell_off[c + 1] = o.y;
+            if (c + 2 < bounds.ncells) cell_off[c + 2] = o.z;
+        }
+        apart |= (v[k].x && s[k].x != o.x) || (v[k].y && s[k].y != o.y) || (v[k].z && s[k].z != o.z) ||
+                 (v[k].w && s[k].w != o.w);
+        // (cells past the last have no value: theirs is the offset of the end)
+        if (c <= bounds.ncells - 1 && bounds.ncells - 1 <= c + 3) cell_off[bounds.ncells] = Op::join(o.w, v[k].w);
         carry = Op::join(carry, all);
-        if (c0 + 32 * k == ncells - 1) cell_off[ncells] = Op::join(off, v[k]);
     }
-    if (gap && __any_sync(kFull, apart) && (threadIdx.x & 31) == 0) atomicOr(gap, 1u);
+    if (gap && __any_sync(kFull, apart) && (threadIdx.x & 31) == 0) atomicOr(gap, gap_bit);
 }
 
-template <typename Op, uint32_t ITEMS>
-cuco_status_t cell_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off, uint32_t ncells,
-                           uint32_t *scratch, uint32_t *finished, uint32_t *gap, cudaStream_t stream) {
-    constexpr uint32_t kCells = kSortThreads * ITEMS;
-    const unsigned blocks = ncells / kCells + (ncells % kCells != 0);
-    k_block_values<Op, ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, finished);
-    k_cell_offsets<Op, ITEMS><<<blocks, kSortThreads, 0, stream>>>(cell_start, cell_end, ncells, scratch, cell_off, gap);
+template <typename Op, uint32_t ROUNDS>
+cuco_status_t cell_offsets(const CellBounds &bounds, uint32_t *cell_off, uint32_t *scratch, uint32_t *finished,
+                           uint32_t *gap, uint32_t gap_bit, cudaStream_t stream) {
+    constexpr uint32_t kCells = kSortThreads * 4 * ROUNDS;
+    const unsigned blocks = bounds.ncells / kCells + (bounds.ncells % kCells != 0);
+    const bool running = blocks > kDirectBlocks;
+    k_block_values<Op, ROUNDS><<<blocks, kSortThreads, 0, stream>>>(bounds, scratch, running ? finished : nullptr);
+    k_cell_offsets<Op, ROUNDS><<<blocks, kSortThreads, 0, stream>>>(bounds, scratch, running, cell_off, gap, gap_bit);
     CUCO_TRY_CUDA(cudaGetLastError());
     return CUCO_OK;
+}
+
+CellBounds cell_bounds(const uint32_t *start, const uint32_t *end, uint32_t ncells) {
+    return {start, end, ncells, ((uintptr_t)start | (uintptr_t)end) % sizeof(uint4) == 0};
 }
 
 // The particles of the cells' ranges, in cell order, to where cell_off says: a
@@ -993,17 +1044,17 @@ size_t offsets_scratch(uint32_t ncells) { return (size_t)ncells / (kSortThreads 
 
 cuco_status_t launch_start_end_offsets(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
                                        uint32_t ncells, uint32_t *scratch, uint32_t *finished, uint32_t *gap,
-                                       cudaStream_t stream) {
+                                       uint32_t gap_bit, cudaStream_t stream) {
     if (!ncells) return CUCO_OK;
-    auto launch = ncells < kOffWideCells ? cell_offsets<RunningEnd, 4> : cell_offsets<RunningEnd, 16>;
-    return launch(cell_start, cell_end, cell_off, ncells, scratch, finished, gap, stream);
+    auto launch = ncells < kOffWideCells ? cell_offsets<RunningEnd, 1> : cell_offsets<RunningEnd, 4>;
+    return launch(cell_bounds(cell_start, cell_end, ncells), cell_off, scratch, finished, gap, gap_bit, stream);
 }
 
 cuco_status_t launch_start_end_counts(const uint32_t *cell_start, const uint32_t *cell_end, uint32_t *cell_off,
                                       uint32_t ncells, uint32_t *scratch, uint32_t *finished, cudaStream_t stream) {
     if (!ncells) return CUCO_OK;
-    auto launch = ncells < kOffWideCells ? cell_offsets<RunningCount, 4> : cell_offsets<RunningCount, 16>;
-    return launch(cell_start, cell_end, cell_off, ncells, scratch, finished, nullptr, stream);
+    auto launch = ncells < kOffWideCells ? cell_offsets<RunningCount, 1> : cell_offsets<RunningCount, 4>;
+    return launch(cell_bounds(cell_start, cell_end, ncells), cell_off, scratch, finished, nullptr, 0u, stream);
 }
 
 cuco_status_t launch_gather_cells(const uint32_t *cell_start, const uint32_t *cell_end, const uint32_t *cell_off,

@@ -38,3 +38,21 @@ def test_masked_cells(port, masked, mark):
     left = np.ones(n, dtype=bool)
     left[at] = False
     assert (got[left] == 7.0).all()
+
+
+@pytest.mark.parametrize("shift", [1, 2])
+def test_bounds_at_any_word(port, shift):
+    """Bounds that do not lie on 16 bytes, contiguous and with cells left out."""
+    rng = np.random.default_rng(shift)
+    pos = rng.uniform(0, L, size=(9000, 3)).astype(np.float32)
+    for G, left_out in ((21, False), (21, True), (110, False), (110, True)):
+        g = Gravlist(pos, G, G, 0.02 * L / G)
+        if left_out:
+            g.start[::3] = -1
+        want = g.forces()
+        held = [torch.empty(g.ncell + shift, dtype=torch.int32, device="cuda:0") for _ in range(2)]
+        for h, a in zip(held, (g.start, g.end)):
+            h[shift:] = a
+        g.start, g.end = held[0][shift:], held[1][shift:]
+        g.acc[:] = 0
+        assert np.array_equal(g.forces(), want)

@@ -70,7 +70,7 @@ def clumps(n, G, seed):
     return pos
 
 
-@pytest.mark.parametrize("G", [20, 300, 1024, 1025, 1032])
+@pytest.mark.parametrize("G", [20, 150, 300, 1024, 1025, 1032])
 def test_forces(port, G):
     pos = clumps(4000, G, G)
     g = Gravlist(pos, G, G, 0.1 * L / G)
